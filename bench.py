@@ -56,7 +56,8 @@ FJORD2048_FLOPS_PER_CELL_STEP = 804.0
 # them until a new capture replaces the numbers and the hash.
 COUNTER_SOURCES = ("landslidehysea_gb300/csrc/lsh_core.cu", "landslidehysea_gb300/csrc/lsh_kernels.cuh",
                    "landslidehysea_gb300/csrc/lsh_passes.cuh", "landslidehysea_gb300/csrc/lsh_scheme.cuh",
-                   "landslidehysea_gb300/csrc/lsh_fpmath.h", "landslidehysea_gb300/csrc/lsh_setup.h",
+                   "landslidehysea_gb300/csrc/lsh_fpmath.h", "landslidehysea_gb300/csrc/lsh_ieee.h",
+                   "landslidehysea_gb300/csrc/lsh_setup.h",
                    "landslidehysea_gb300/build.py", "landslidehysea_gb300/scenarios.py")
 COUNTERS_SOURCE_HASH = "032c79f00d393a67"
 # FP64-pipe thread instructions per cell-update of one step (6.060e8 per step

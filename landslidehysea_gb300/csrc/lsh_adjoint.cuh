@@ -41,22 +41,22 @@ LSH_HD double times_sgn1(double x, double s) { return lshm::neg_if(x, lt0(s)); }
 
 // d vfac / dh
 LSH_HD double vfac_d(double h, double eps_h) {
-    if (gt_pos(h, eps_h)) { const double v = 1.0 / h; return -(v * v); }
+    if (gt_pos(h, eps_h)) { const double v = rcp_call(h); return -(v * v); }
     const double h2 = h * h, m2 = eps_h * eps_h;
     const double q = fmad(h2, h2, m2 * m2);
-    const double s = sqrt(q);
+    const double s = root_call(q);
     // d/dh [sqrt2 h q^-1/2] = sqrt2 q^-1/2 (1 - 2 h^4 / q)
-    return (kSqrt2 / s) * (1.0 - (2.0 * (h2 * h2)) / q);
+    return div_call(kSqrt2, s) * (1.0 - div_call(2.0 * (h2 * h2), q));
 }
 
 // d (h cbrt h) / dh = (4/3) cbrt h; 0 at h = 0
 LSH_HD double pow43_d(double h) {
     if (!gt0(h)) return 0.0;
     const double c = lshm::cbrt_pos(h);
-    return c + c / 3.0;
+    return c + div_call(c, 3.0);
 }
 
-LSH_HD double sqrt_bar(double s, double sb) { return gt0(s) ? sb / (2.0 * s) : 0.0; }
+LSH_HD double sqrt_bar(double s, double sb) { return gt0(s) ? div_call(sb, 2.0 * s) : 0.0; }
 
 // The compare-and-swap network of sort_eig on values, carrying the labels
 // of the unsorted entries: after the call D[k] = entry perm[k].
@@ -89,14 +89,14 @@ LSH_HD void eig_adj(double h1, double h2, double u1, double u2, double q, const 
     const double F = useFk ? Fknown : vfac(h, c.eps_h);
     const double u = direct ? u1 : q * F;
     const bool useSh = !lt0(sqrt_h);
-    const double cg = useSh ? c.sqrt_g * sqrt_h : sqrt(c.g * h);
+    const double cg = useSh ? c.sqrt_g * sqrt_h : root_call(c.g * h);
     double uu = 0.0, ci = 0.0, d = 0.0, aux = 0.0, P = 0.0;
     if (L2) {
         uu = fmad(u1, h2, u2 * h1) * F;
         d = u1 - u2;
         aux = fmad(-((d * d) * F), c.inv_gp, 1.0);
         P = (((c.gp * h1) * h2) * F);
-        ci = sqrt(P * abs_bits(aux));
+        ci = root_call(P * abs_bits(aux));
     }
     double e[4] = {u - cg, uu - ci, uu + ci, u + cg};
     int perm[4] = {0, 1, 2, 3};
@@ -140,7 +140,7 @@ LSH_HD void eig_adj(double h1, double h2, double u1, double u2, double q, const 
         h1b += nb * u2;
     }
     if (useSh) sqrt_hb += cgb * c.sqrt_g;
-    else if (gt0(cg)) hb += (cgb * c.g) / (2.0 * cg);
+    else if (gt0(cg)) hb += div_call(cgb * c.g, 2.0 * cg);
     if (direct) {
         u1b += ub;
     } else {
@@ -201,16 +201,16 @@ LSH_HD void edge_flux_adj(const EdgeIn& e, double dt, const Consts& c, const Edg
 
     const double fA1 = vfac(Ah1, eps), fB1 = vfac(Bh1, eps);
     const double fA2 = L2 ? vfac(Ah2, eps) : 0.0, fB2 = L2 ? vfac(Bh2, eps) : 0.0;
-    const double sa1 = sqrt(Ah1), sb1 = sqrt(Bh1);
+    const double sa1 = root_call(Ah1), sb1 = root_call(Bh1);
     const double num1 = fmad(sa1, fA1 * Aq1, sb1 * (fB1 * Bq1));
     const double den1 = sa1 + sb1 + kEps;
-    const double u1ij = num1 / den1;
+    const double u1ij = div_call(num1, den1);
     double sa2 = 0.0, sb2 = 0.0, num2 = 0.0, den2 = 1.0, u2ij = 0.0;
     if (L2) {
-        sa2 = sqrt(Ah2); sb2 = sqrt(Bh2);
+        sa2 = root_call(Ah2); sb2 = root_call(Bh2);
         num2 = fmad(sa2, fA2 * Aq2, sb2 * (fB2 * Bq2));
         den2 = sa2 + sb2 + kEps;
-        u2ij = num2 / den2;
+        u2ij = div_call(num2, den2);
     }
     const bool oneA = !L2 || is_zero(Ah2), oneB = !L2 || is_zero(Bh2);
 
@@ -259,7 +259,7 @@ LSH_HD void edge_flux_adj(const EdgeIn& e, double dt, const Consts& c, const Edg
         if (L2 && !lt_pos(h1ij, eps) && !lt_pos(h2ij, eps)) {
             branch = 0;
             d12 = aut1 - aut2; d13 = aut1 - aut3; d23 = aut2 - aut3;
-            inv = 1.0 / ((d12 * d13) * d23);
+            inv = rcp_call((d12 * d13) * d23);
             aa = (fabs(aut1) * d23) * inv;
             bb = -((fabs(aut2) * d13) * inv);
             cc = (fabs(aut3) * d12) * inv;
@@ -268,7 +268,7 @@ LSH_HD void edge_flux_adj(const EdgeIn& e, double dt, const Consts& c, const Edg
             a2 = aa + bb + cc;
         } else {
             branch = 1;
-            inv = 1.0 / (aut3 - aut1);
+            inv = rcp_call(aut3 - aut1);
             a0 = fmad(aut3, fabs(aut1), -(aut1 * fabs(aut3))) * inv;
             a1 = (fabs(aut3) - fabs(aut1)) * inv;
         }
@@ -357,10 +357,10 @@ LSH_HD void edge_flux_adj(const EdgeIn& e, double dt, const Consts& c, const Edg
         if (useB[layer]) denB[layer] = fmad(factor, P[k], kEps);
         lim[layer] = (useA[layer] && lt(ha, dt * denA[layer])) || (useB[layer] && lt(hb, dt * denB[layer]));
         if (lim[layer]) {
-            if (useA[layer]) dta[layer] = ha / denA[layer];
-            if (useB[layer]) dtbv[layer] = hb / denB[layer];
+            if (useA[layer]) dta[layer] = div_call(ha, denA[layer]);
+            if (useB[layer]) dtbv[layer] = div_call(hb, denB[layer]);
             dtl[layer] = tmin(dta[layer], dtbv[layer]);
-            alpha[layer] = dtl[layer] / (dt + kEps);
+            alpha[layer] = div_call(dtl[layer], dt + kEps);
         }
     }
 
@@ -384,16 +384,16 @@ LSH_HD void edge_flux_adj(const EdgeIn& e, double dt, const Consts& c, const Edg
             mb[q] = mb[q] * alpha[layer];
             pb[q] = pb[q] * alpha[layer];
         }
-        const double dtlb = alb / (dt + kEps);
-        dtb += -alb * (alpha[layer] / (dt + kEps));
+        const double dtlb = div_call(alb, dt + kEps);
+        dtb += -alb * div_call(alpha[layer], dt + kEps);
         // tmin(dta, dtb) = (dtb < dta) ? dtb : dta
         if (lt(dtbv[layer], dta[layer])) {
             // dtb = hp1 area1 / (beta P + eps)
-            hp1b[layer] += dtlb * (e.area1 / denB[layer]);
-            pb[k] += (-dtlb * (dtbv[layer] / denB[layer])) * factor;
+            hp1b[layer] += dtlb * div_call(e.area1, denB[layer]);
+            pb[k] += (-dtlb * div_call(dtbv[layer], denB[layer])) * factor;
         } else if (useA[layer]) {
-            hp0b[layer] += dtlb * (e.area0 / denA[layer]);
-            mb[k] += (-dtlb * (dta[layer] / denA[layer])) * factor;
+            hp0b[layer] += dtlb * div_call(e.area0, denA[layer]);
+            mb[k] += (-dtlb * div_call(dta[layer], denA[layer])) * factor;
         }
     }
     // hp = b acc + hc, b = dt / area
@@ -591,8 +591,8 @@ LSH_HD void edge_flux_adj(const EdgeIn& e, double dt, const Consts& c, const Edg
     if (gt0(P0)) { Ah1b -= deta1b; if (L2) Ah2b -= deta1b; }
     // Roe-type velocities
     {
-        const double num1b = u1b / den1;
-        const double den1b = -u1b * (u1ij / den1);
+        const double num1b = div_call(u1b, den1);
+        const double den1b = -u1b * div_call(u1ij, den1);
         sa1b += num1b * uA1 + den1b;
         fA1b += num1b * (sa1 * Aq1);
         Aq1b += num1b * (sa1 * fA1);
@@ -601,8 +601,8 @@ LSH_HD void edge_flux_adj(const EdgeIn& e, double dt, const Consts& c, const Edg
         Bq1b += num1b * (sb1 * fB1);
     }
     if (L2) {
-        const double num2b = u2b / den2;
-        const double den2b = -u2b * (u2ij / den2);
+        const double num2b = div_call(u2b, den2);
+        const double den2b = -u2b * div_call(u2ij, den2);
         sa2b += num2b * uA2 + den2b;
         fA2b += num2b * (sa2 * Aq2);
         Aq2b += num2b * (sa2 * fA2);
@@ -635,16 +635,16 @@ LSH_HD void edge_initial_wave_adj(const Face& A, const Face& B, double len, cons
     const double eps = c.eps_h;
     const double h1ij = 0.5 * (A.h1 + B.h1);
     const double fA1 = vfac(A.h1, eps), fB1 = vfac(B.h1, eps);
-    const double sa1 = sqrt(A.h1), sb1 = sqrt(B.h1);
+    const double sa1 = root_call(A.h1), sb1 = root_call(B.h1);
     const double uA1 = fA1 * A.qn1, uB1 = fB1 * B.qn1;
     const double num1 = fmad(sa1, uA1, sb1 * uB1), den1 = sa1 + sb1 + kEps;
-    const double u1ij = num1 / den1;
+    const double u1ij = div_call(num1, den1);
     const double h2ij = 0.5 * (A.h2 + B.h2);
     const double fA2 = vfac(A.h2, eps), fB2 = vfac(B.h2, eps);
-    const double sa2 = sqrt(A.h2), sb2 = sqrt(B.h2);
+    const double sa2 = root_call(A.h2), sb2 = root_call(B.h2);
     const double uA2 = fA2 * A.qn2, uB2 = fB2 * B.qn2;
     const double num2 = fmad(sa2, uA2, sb2 * uB2), den2 = sa2 + sb2 + kEps;
-    const double u2ij = num2 / den2;
+    const double u2ij = div_call(num2, den2);
     const double q = fmad(h1ij, u1ij, h2ij * u2ij);
     const V4 D = eig<true>(h1ij, h2ij, u1ij, u2ij, q, c);
     const double lm0 = tmax(D.x, D.w);
@@ -664,8 +664,8 @@ LSH_HD void edge_initial_wave_adj(const Face& A, const Face& B, double len, cons
     eig_adj<true>(h1ij, h2ij, u1ij, u2ij, q, c, -1.0, -1.0, Db, h1ijb, h2ijb, u1b, u2b, qb, fk, sh, cb);
     h1ijb += qb * u1ij; u1b += qb * h1ij;
     h2ijb += qb * u2ij; u2b += qb * h2ij;
-    const double num1b = u1b / den1, den1b = -u1b * (u1ij / den1);
-    const double num2b = u2b / den2, den2b = -u2b * (u2ij / den2);
+    const double num1b = div_call(u1b, den1), den1b = -u1b * div_call(u1ij, den1);
+    const double num2b = div_call(u2b, den2), den2b = -u2b * div_call(u2ij, den2);
     const double sa1b = num1b * uA1 + den1b, sb1b = num1b * uB1 + den1b;
     const double sa2b = num2b * uA2 + den2b, sb2b = num2b * uB2 + den2b;
     const double uA1b = num1b * sa1, uB1b = num1b * sb1, uA2b = num2b * sa2, uB2b = num2b * sb2;
@@ -684,7 +684,7 @@ LSH_HD void edge_initial_wave_adj(const Face& A, const Face& B, double len, cons
 LSH_HD void bottom_friction_adj(double h, double un, double gm, double dt, double eps, const double win[2],
                                 double wbar[2], double& hb, double& unb, double& gmb, double& dtb) {
     const double Y = pow43(h) + kEps, X = (dt * gm) * un;
-    const double inv = Y / (Y + X);
+    const double inv = div_call(Y, Y + X);
     double invb = 0.0;
     if (gt_pos(h, eps)) {
         invb = wbar[0] * win[0] + wbar[1] * win[1];
@@ -704,8 +704,8 @@ LSH_HD void bottom_friction_adj(double h, double un, double gm, double dt, doubl
         hb += fb * vfac_d(h, eps);
     }
     const double YX = Y + X;
-    const double Yb = invb * (X / (YX * YX));
-    const double Xb = -invb * (Y / (YX * YX));
+    const double Yb = invb * div_call(X, YX * YX);
+    const double Xb = -invb * div_call(Y, YX * YX);
     hb += Yb * pow43_d(h);
     dtb += Xb * (gm * un);
     gmb += Xb * (dt * un);
@@ -759,7 +759,7 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
         dd[layer] = fmad(x2s[layer], x2s[layer], kEps);
         if (lt_pos(dt, dd[layer] * 0x1.fp-55)) continue;  // dd >= EPSILON: the bound is positive
         damp[layer] = true;
-        auxs[layer] = exp_neg(dt * (1.0 / dd[layer]));
+        auxs[layer] = exp_neg(dt * rcp_call(dd[layer]));
         wd[k + 1] = wd[k + 1] * auxs[layer];
         wd[k + 2] = wd[k + 2] * auxs[layer];
     }
@@ -775,10 +775,10 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
         vf[layer] = vfac(h, eps);
         vux[layer] = vf[layer] * wv[k + 1];
         vuy[layer] = vf[layer] * wv[k + 2];
-        vu[layer] = sqrt(fmad(vux[layer], vux[layer], vuy[layer] * vuy[layer]));
+        vu[layer] = root_call(fmad(vux[layer], vux[layer], vuy[layer] * vuy[layer]));
         if (gt_pos(vu[layer], vmax)) {
             cap[layer] = true;
-            vs[layer] = vmax / vu[layer];
+            vs[layer] = div_call(vmax, vu[layer]);
             wv[k + 1] = (vux[layer] * vs[layer]) * h;
             wv[k + 2] = (vuy[layer] * vs[layer]) * h;
         }
@@ -786,12 +786,12 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
     // dis_implicita (its clamps are no-ops after filtro's)
     const double h1 = wv[0], h2 = single ? 0.0 : wv[3];
     const double uo1x = fo1 * wo[1], uo1y = fo1 * wo[2];
-    const double u1o = sqrt(fmad(uo1x, uo1x, uo1y * uo1y));
+    const double u1o = root_call(fmad(uo1x, uo1x, uo1y * uo1y));
     const double fo2 = vfac(wo[3], eps);
     const double uo2x = fo2 * wo[4], uo2y = fo2 * wo[5];
     const double ddx = uo1x - uo2x, ddy = uo1y - uo2y;
-    const double du = sqrt(fmad(ddx, ddx, ddy * ddy));
-    const double u2o = sqrt(fmad(uo2x, uo2x, uo2y * uo2y));
+    const double du = root_call(fmad(ddx, ddx, ddy * ddy));
+    const double u2o = root_call(fmad(uo2x, uo2x, uo2y * uo2y));
     const bool blkA = !single && gt0(h1) && gt0(h2);
     const bool blkB = gt0(h1) && lt_pos(h2, eps);
     const bool blkC = !single && gt0(h2) && lt_pos(h1, eps);
@@ -807,15 +807,15 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
         hmod = fmad(c.r, h1, h2);
         mm = gt_pos(hmod, c.eps_1r) ? hmod : c.eps_1r;
         hm2 = hmod * hmod; m2 = mm * mm;
-        Sq = sqrt(fmad(hm2, hm2, m2 * m2));
-        hh = hmod / Sq;
+        Sq = root_call(fmad(hm2, hm2, m2 * m2));
+        hh = div_call(hmod, Sq);
         k12 = ((dt * kSqrt2) * hh) * (c.mfc * du);
         c1 = k12 * h2;
         c2 = (k12 * c.r) * h1;
         P3 = pow43(h2) + kEps;
-        c3 = ((dt * c.g_mfs2) * u2o) / P3;
+        c3 = div_call((dt * c.g_mfs2) * u2o, P3);
         e1 = 1.0 + c1; e2 = 1.0 + c2 + c3;
-        det = 1.0 / fmad(e1, e2, -(c1 * c2));
+        det = rcp_call(fmad(e1, e2, -(c1 * c2)));
         n1x = fmad(u1x, e2, c1 * u2x); n2x = fmad(u2x, e1, c2 * u1x);
         n1y = fmad(u1y, e2, c1 * u2y); n2y = fmad(u2y, e1, c2 * u1y);
         wa[1] = (h1 * n1x) * det;
@@ -827,7 +827,7 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
     for (int k = 0; k < 6; ++k) wbk[k] = wa[k];
     if (blkB) {
         const double Y = pow43(h1) + kEps, X = (dt * c.g_mf02) * u1o;
-        const double inv = Y / (Y + X);
+        const double inv = div_call(Y, Y + X);
         if (gt_pos(h1, eps)) { wbk[1] = wa[1] * inv; wbk[2] = wa[2] * inv; }
         else { wbk[1] = (h1 * (f1 * wa[1])) * inv; wbk[2] = (h1 * (f1 * wa[2])) * inv; }
     }
@@ -835,7 +835,7 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
     for (int k = 0; k < 6; ++k) wcc[k] = wbk[k];
     if (blkC) {
         const double Y = pow43(h2) + kEps, X = (dt * c.g_mfs2) * u2o;
-        const double inv = Y / (Y + X);
+        const double inv = div_call(Y, Y + X);
         if (gt_pos(h2, eps)) { wcc[4] = wbk[4] * inv; wcc[5] = wbk[5] * inv; }
         else { wcc[4] = (h2 * (f2 * wbk[4])) * inv; wcc[5] = (h2 * (f2 * wbk[5])) * inv; }
     }
@@ -853,17 +853,17 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
         const double ex = exp_neg(a * a);
         const double fsc = 1.0 - c.r * (1.0 - ex);
         const double sc = (((fsc * c.mu) * c.g) * hc2) * dt;
-        const double nq = sqrt(fmad(wcc[4], wcc[4], wcc[5] * wcc[5]));
+        const double nq = root_call(fmad(wcc[4], wcc[4], wcc[5] * wcc[5]));
         const bool act = !lt_pos(nq + sc, kEps) && !lt(nq, sc);
-        const double aux = act ? nq / (nq + sc) : 0.0;
+        const double aux = act ? div_call(nq, nq + sc) : 0.0;
         const double auxb = g[4] * wcc[4] + g[5] * wcc[5];
         g[4] = g[4] * aux;
         g[5] = g[5] * aux;
         if (act) {
             const double s2 = (nq + sc) * (nq + sc);
-            const double nqb = auxb * (sc / s2);
-            const double scb = -auxb * (nq / s2);
-            if (gt0(nq)) { g[4] += nqb * (wcc[4] / nq); g[5] += nqb * (wcc[5] / nq); }
+            const double nqb = auxb * div_call(sc, s2);
+            const double scb = -auxb * div_call(nq, s2);
+            if (gt0(nq)) { g[4] += nqb * div_call(wcc[4], nq); g[5] += nqb * div_call(wcc[5], nq); }
             const double fscb = scb * (((c.mu * c.g) * hc2) * dt);
             cb.mu += scb * (((fsc * c.g) * hc2) * dt);
             g[3] += scb * (((fsc * c.mu) * c.g) * dt);
@@ -911,8 +911,8 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
         c2b += e2b;
         const double c3b = e2b;
         const double nn = (dt * c.g_mfs2) * u2o;
-        const double nnb = c3b / P3;
-        const double P3b = -c3b * (c3 / P3);
+        const double nnb = div_call(c3b, P3);
+        const double P3b = -c3b * div_call(c3, P3);
         dtb += nnb * (c.g_mfs2 * u2o);
         cb.g_mfs2 += nnb * (dt * u2o);
         u2ob += nnb * (dt * c.g_mfs2);
@@ -925,8 +925,8 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
         dtb += k12b * ((kSqrt2 * hh) * (c.mfc * du));
         const double hhb = k12b * ((dt * kSqrt2) * (c.mfc * du));
         const double dub = k12b * ((dt * kSqrt2) * hh) * c.mfc;
-        double hmodb = hhb / Sq;
-        const double Sqb = -hhb * (hh / Sq);
+        double hmodb = div_call(hhb, Sq);
+        const double Sqb = -hhb * div_call(hh, Sq);
         const double Qb = sqrt_bar(Sq, Sqb);
         const double hm2b = Qb * (2.0 * hm2), m2b = Qb * (2.0 * m2);
         hmodb += hm2b * (2.0 * hmod);
@@ -937,7 +937,7 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
         h1b += hmodb * c.r;
         h2b += hmodb;
         if (gt0(du)) {
-            const double dxb = dub * (ddx / du), dyb = dub * (ddy / du);
+            const double dxb = dub * div_call(ddx, du), dyb = dub * div_call(ddy, du);
             uo1xb += dxb; uo2xb -= dxb;
             uo1yb += dyb; uo2yb -= dyb;
         }
@@ -950,8 +950,8 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
         h2b += f2b * vfac_d(h2, eps);
     }
     // old speeds
-    if (gt0(u1o)) { uo1xb += u1ob * (uo1x / u1o); uo1yb += u1ob * (uo1y / u1o); }
-    if (!single && gt0(u2o)) { uo2xb += u2ob * (uo2x / u2o); uo2yb += u2ob * (uo2y / u2o); }
+    if (gt0(u1o)) { uo1xb += u1ob * div_call(uo1x, u1o); uo1yb += u1ob * div_call(uo1y, u1o); }
+    if (!single && gt0(u2o)) { uo2xb += u2ob * div_call(uo2x, u2o); uo2yb += u2ob * div_call(uo2y, u2o); }
     const double fo1b = uo1xb * wo[1] + uo1yb * wo[2];
     wob[1] += uo1xb * fo1;
     wob[2] += uo1yb * fo1;
@@ -974,8 +974,8 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
         const double sb = oxb * (vux[layer] * h) + oyb * (vuy[layer] * h);
         double hb = oxb * (vux[layer] * vs[layer]) + oyb * (vuy[layer] * vs[layer]);
         const double vmax = layer ? c.vmax2 : c.vmax1;
-        const double ub = -sb * (vmax / (vu[layer] * vu[layer]));
-        if (gt0(vu[layer])) { uxb += ub * (vux[layer] / vu[layer]); uyb += ub * (vuy[layer] / vu[layer]); }
+        const double ub = -sb * div_call(vmax, vu[layer] * vu[layer]);
+        if (gt0(vu[layer])) { uxb += ub * div_call(vux[layer], vu[layer]); uyb += ub * div_call(vuy[layer], vu[layer]); }
         const double fb = uxb * wd[k + 1] + uyb * wd[k + 2];
         g[k + 1] = uxb * vf[layer];
         g[k + 2] = uyb * vf[layer];
@@ -989,7 +989,7 @@ LSH_HD void volume_update_adj(const double wo[6], const double acc[7], double in
         const double auxb = g[k + 1] * wc[k + 1] + g[k + 2] * wc[k + 2];
         g[k + 1] = g[k + 1] * auxs[layer];
         g[k + 2] = g[k + 2] * auxs[layer];
-        const double invd = 1.0 / dd[layer];
+        const double invd = rcp_call(dd[layer]);
         const double zb = -auxb * auxs[layer];
         dtb += zb * invd;
         const double db = -(zb * dt) * (invd * invd);

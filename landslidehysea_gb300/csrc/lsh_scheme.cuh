@@ -23,12 +23,12 @@
 #include <cstdint>
 
 #include "lsh_fpmath.h"
+#include "lsh_ieee.h"
 
 namespace lsh {
 
 #if !defined(__CUDA_ARCH__)
 using std::fabs;
-using std::sqrt;
 #endif
 
 constexpr double kEps = 1.1920928955078125e-07;  // FLT_EPSILON (Constantes.hxx:13)
@@ -85,6 +85,13 @@ using lshm::lt;
 using lshm::lt0;
 using lshm::lt_pos;
 using lshm::okey;
+// IEEE division, reciprocal and square root on the integer pipe (lsh_ieee.h)
+using lshm::div;
+using lshm::div_call;
+using lshm::rcp;
+using lshm::rcp_call;
+using lshm::root;
+using lshm::root_call;
 
 LSH_HD double tmin(double a, double b) { return lt(b, a) ? b : a; }
 LSH_HD double tmax(double a, double b) { return lt(a, b) ? b : a; }
@@ -94,9 +101,9 @@ LSH_HD double exp_neg(double x) { return lshm::exp_neg(x); }
 
 // sqrt(2) h / sqrt(h^4 + max(h, eps_h)^4); exactly 1/h for h > eps_h
 LSH_HD double vfac(double h, double eps_h) {
-    if (gt_pos(h, eps_h)) return 1.0 / h;
+    if (gt_pos(h, eps_h)) return rcp(h);
     const double h2 = h * h, m2 = eps_h * eps_h;
-    return (kSqrt2 * h) / sqrt(fmad(h2, h2, m2 * m2));
+    return div(kSqrt2 * h, root(fmad(h2, h2, m2 * m2)));
 }
 
 LSH_HD double pow43(double h) { return h * lshm::cbrt_pos(h); }
@@ -155,13 +162,13 @@ LSH_HD V4 eig(double h1, double h2, double u1, double u2, double q, const Consts
     if (L2 || !direct) F = (!L2 && !lt0(Fknown)) ? Fknown : vfac(h, c.eps_h);
     const double u = direct ? u1 : q * F;
     // sqrt_h >= 0: sqrt(h1) is known and h2 == 0, so sqrt(g h) = sqrt(g) sqrt(h1)
-    const double cg = !lt0(sqrt_h) ? c.sqrt_g * sqrt_h : sqrt(c.g * h);
+    const double cg = !lt0(sqrt_h) ? c.sqrt_g * sqrt_h : root(c.g * h);
     double uu = 0.0, ci = 0.0;
     if (L2) {
         uu = fmad(u1, h2, u2 * h1) * F;
         const double d = u1 - u2;
         const double aux = fmad(-((d * d) * F), c.inv_gp, 1.0);
-        ci = sqrt((((c.gp * h1) * h2) * F) * abs_bits(aux));
+        ci = root((((c.gp * h1) * h2) * F) * abs_bits(aux));
     }
     V4 D{u - cg, uu - ci, uu + ci, u + cg};
     sort_eig(D, c.eig_sort);
@@ -174,17 +181,17 @@ LSH_HD double friction_mu(double h1, double u1, double h2, double u2, const Cons
     const double a = (10.0 * h1) * c.inv_eps;
     const double rr = 1.0 - c.r * (1.0 - exp_neg(a * a));
     const double gp = c.g * rr;
-    const double fr1 = ((u1 * u1) * vfac(h1, c.eps_h)) / gp;
-    const double fr2 = ((u2 * u2) * vfac(h2, c.eps_h)) / gp;
-    const double fr = sqrt(fmad((1.0 - rr) * fr1, fr2, fr1 + fr2));
+    const double fr1 = div((u1 * u1) * vfac(h1, c.eps_h), gp);
+    const double fr2 = div((u2 * u2) * vfac(h2, c.eps_h), gp);
+    const double fr = root(fmad((1.0 - rr) * fr1, fr2, fr1 + fr2));
     const double beta = 0.136, L2c = 8.0e-4, chi = 1.0e-3;
-    const double mustop = c.tan1 + (c.tan2 - c.tan1) / (1.0 + h2 / L2c);
-    const double mustart = c.tan3 + (c.tan4 - c.tan3) / (1.0 + h2 / L2c);
+    const double mustop = c.tan1 + div(c.tan2 - c.tan1, 1.0 + div(h2, L2c));
+    const double mustart = c.tan3 + div(c.tan4 - c.tan3, 1.0 + div(h2, L2c));
     double muf;
-    if (gt_pos(fr, beta)) muf = c.tan1 + (c.tan2 - c.tan1) / (1.0 + beta * h2 / (fr * L2c));
-    else if (abs_lt(fr, kEps)) muf = c.tan3 + (c.tan4 - c.tan3) / (1.0 + h2 / L2c);
-    else muf = fmad(lshm::pow_pos(fr / beta, chi), mustop - mustart, mustart);
-    return (muf * c.L) / c.H;
+    if (gt_pos(fr, beta)) muf = c.tan1 + div(c.tan2 - c.tan1, 1.0 + div(beta * h2, fr * L2c));
+    else if (abs_lt(fr, kEps)) muf = c.tan3 + div(c.tan4 - c.tan3, 1.0 + div(h2, L2c));
+    else muf = fmad(lshm::pow_pos(div(fr, beta), chi), mustop - mustart, mustart);
+    return div(muf * c.L, c.H);
 }
 
 LSH_HD double fsc_of(double h1, const Consts& c) {
@@ -252,12 +259,12 @@ LSH_HD void edge_flux(const EdgeIn& e, double dt, const Consts& c, EdgeOut& o, c
 
     const double fA1 = vfac(Ah1, eps), fB1 = vfac(Bh1, eps);
     const double fA2 = L2 ? vfac(Ah2, eps) : 0.0, fB2 = L2 ? vfac(Bh2, eps) : 0.0;
-    const double sa1 = sqrt(Ah1), sb1 = sqrt(Bh1);
-    const double u1ij = fmad(sa1, fA1 * Aq1, sb1 * (fB1 * Bq1)) / (sa1 + sb1 + kEps);
+    const double sa1 = root(Ah1), sb1 = root(Bh1);
+    const double u1ij = div(fmad(sa1, fA1 * Aq1, sb1 * (fB1 * Bq1)), sa1 + sb1 + kEps);
     double u2ij = 0.0;
     if (L2) {
-        const double sa2 = sqrt(Ah2), sb2 = sqrt(Bh2);
-        u2ij = fmad(sa2, fA2 * Aq2, sb2 * (fB2 * Bq2)) / (sa2 + sb2 + kEps);
+        const double sa2 = root(Ah2), sb2 = root(Bh2);
+        u2ij = div(fmad(sa2, fA2 * Aq2, sb2 * (fB2 * Bq2)), sa2 + sb2 + kEps);
     }
     // a face's celerity sqrt(g h) is sqrt(g) sqrt(h1) when its granular layer is empty
     const bool oneA = !L2 || is_zero(Ah2), oneB = !L2 || is_zero(Bh2);
@@ -293,7 +300,7 @@ LSH_HD void edge_flux(const EdgeIn& e, double dt, const Consts& c, EdgeOut& o, c
     if (!abs_lt(aut1 - aut3, kEps) && !abs_lt(aut1 - aut2, kEps) && !abs_lt(aut2 - aut3, kEps)) {
         if (L2 && !lt_pos(h1ij, eps) && !lt_pos(h2ij, eps)) {
             const double d12 = aut1 - aut2, d13 = aut1 - aut3, d23 = aut2 - aut3;
-            const double inv = 1.0 / ((d12 * d13) * d23);
+            const double inv = rcp((d12 * d13) * d23);
             const double a = (abs_bits(aut1) * d23) * inv;
             const double b = -((abs_bits(aut2) * d13) * inv);
             const double cc = (abs_bits(aut3) * d12) * inv;
@@ -301,7 +308,7 @@ LSH_HD void edge_flux(const EdgeIn& e, double dt, const Consts& c, EdgeOut& o, c
             a1 = -fmad(a, aut2 + aut3, fmad(b, aut1 + aut3, cc * (aut1 + aut2)));
             a2 = a + b + cc;
         } else {
-            const double inv = 1.0 / (aut3 - aut1);
+            const double inv = rcp(aut3 - aut1);
             a0 = fmad(aut3, abs_bits(aut1), -(aut1 * abs_bits(aut3))) * inv;
             a1 = (abs_bits(aut3) - abs_bits(aut1)) * inv;
         }
@@ -383,9 +390,9 @@ LSH_HD void edge_flux(const EdgeIn& e, double dt, const Consts& c, EdgeOut& o, c
         const double da = oa ? fmad(factor, M[k], kEps) : 1.0, db = ob ? fmad(factor, P[k], kEps) : 1.0;
         const bool lim = (oa && lt(ha, dt * da)) || (ob && lt(hb, dt * db));
         if (lim) {
-            const double dta = oa ? ha / da : kBig, dtb = ob ? hb / db : kBig;
+            const double dta = oa ? div(ha, da) : kBig, dtb = ob ? div(hb, db) : kBig;
             const double dtl = tmin(dta, dtb);
-            const double alpha = dtl / (dt + kEps);
+            const double alpha = div(dtl, dt + kEps);
 #pragma unroll
             for (int q = 0; q < 3; ++q) { M[k + q] = alpha * M[k + q]; P[k + q] = alpha * P[k + q]; }
         }
@@ -412,12 +419,12 @@ LSH_HD double edge_initial_wave(const Face& A, const Face& B, double len, const 
     const double eps = c.eps_h;
     const double h1ij = 0.5 * (A.h1 + B.h1);
     const double fA1 = vfac(A.h1, eps), fB1 = vfac(B.h1, eps);
-    double sa = sqrt(A.h1), sb = sqrt(B.h1);
-    const double u1ij = fmad(sa, fA1 * A.qn1, sb * (fB1 * B.qn1)) / (sa + sb + kEps);
+    double sa = root(A.h1), sb = root(B.h1);
+    const double u1ij = div(fmad(sa, fA1 * A.qn1, sb * (fB1 * B.qn1)), sa + sb + kEps);
     const double h2ij = 0.5 * (A.h2 + B.h2);
     const double fA2 = vfac(A.h2, eps), fB2 = vfac(B.h2, eps);
-    sa = sqrt(A.h2); sb = sqrt(B.h2);
-    const double u2ij = fmad(sa, fA2 * A.qn2, sb * (fB2 * B.qn2)) / (sa + sb + kEps);
+    sa = root(A.h2); sb = root(B.h2);
+    const double u2ij = div(fmad(sa, fA2 * A.qn2, sb * (fB2 * B.qn2)), sa + sb + kEps);
     const V4 D = eig<true>(h1ij, h2ij, u1ij, u2ij, fmad(h1ij, u1ij, h2ij * u2ij), c);
     double lmax = tmax(D.x, D.w);
     const double b = tmax(abs_bits(u1ij), abs_bits(u2ij));
@@ -441,7 +448,7 @@ LSH_HD void filtro(double w[6], double dt, const Consts& c) {
         // exp(-dt/d) is exactly 1 once dt/d < 2^-54: skip the division below a
         // bound that holds with ample margin over the roundings
         if (lt_pos(dt, d * 0x1.fp-55)) continue;  // d >= EPSILON: the bound is positive
-        const double aux = exp_neg(dt * (1.0 / d));
+        const double aux = exp_neg(dt * rcp(d));
         w[k + 1] = w[k + 1] * aux;
         w[k + 2] = w[k + 2] * aux;
     }
@@ -453,9 +460,9 @@ LSH_HD void filtro(double w[6], double dt, const Consts& c) {
             const double h = w[k];
             const double f = vfac(h, c.eps_h);
             double ux = f * w[k + 1], uy = f * w[k + 2];
-            const double u = sqrt(fmad(ux, ux, uy * uy));
+            const double u = root(fmad(ux, ux, uy * uy));
             if (gt_pos(u, vmax)) {
-                const double s = vmax / u;
+                const double s = div(vmax, u);
                 ux = ux * s; uy = uy * s;
                 w[k + 1] = ux * h; w[k + 2] = uy * h;
             }
@@ -474,13 +481,13 @@ LSH_HD void dis_implicita(const double wo[6], double w[6], double dt, const Cons
     const double eps = c.eps_h;
     const double h1 = w[0], h2 = L2 ? w[3] : 0.0;
     const double uo1x = fo1 * wo[1], uo1y = fo1 * wo[2];
-    const double u1 = sqrt(fmad(uo1x, uo1x, uo1y * uo1y));
+    const double u1 = root(fmad(uo1x, uo1x, uo1y * uo1y));
     if (!L2) {
         // bottom friction h u / (1 + c1), 1/(1 + X/Y) = Y/(Y + X); above
         // eps_h, h u is q itself
         if (gt0(h1)) {
             const double Y = pow43(h1) + kEps, X = (dt * c.g_mf02) * u1;
-            const double inv = Y / (Y + X);
+            const double inv = div(Y, Y + X);
             if (gt_pos(h1, eps)) { w[1] = w[1] * inv; w[2] = w[2] * inv; }
             else {
                 const double f1 = vfac(h1, eps);
@@ -497,19 +504,19 @@ LSH_HD void dis_implicita(const double wo[6], double w[6], double dt, const Cons
     const double fo2 = vfac(wo[3], eps);
     const double uo2x = fo2 * wo[4], uo2y = fo2 * wo[5];
     const double dx = uo1x - uo2x, dy = uo1y - uo2y;
-    const double du = sqrt(fmad(dx, dx, dy * dy));
-    const double u2 = sqrt(fmad(uo2x, uo2x, uo2y * uo2y));
+    const double du = root(fmad(dx, dx, dy * dy));
+    const double u2 = root(fmad(uo2x, uo2x, uo2y * uo2y));
     if (gt0(h1) && gt0(h2)) {
         const double hmod = fmad(c.r, h1, h2);
         const double m = gt_pos(hmod, c.eps_1r) ? hmod : c.eps_1r;
         const double hm2 = hmod * hmod, m2 = m * m;
-        const double hh = hmod / sqrt(fmad(hm2, hm2, m2 * m2));
+        const double hh = div(hmod, root(fmad(hm2, hm2, m2 * m2)));
         const double k12 = ((dt * kSqrt2) * hh) * (c.mfc * du);
         const double c1 = k12 * h2;
         const double c2 = (k12 * c.r) * h1;
-        const double c3 = ((dt * c.g_mfs2) * u2) / (pow43(h2) + kEps);
+        const double c3 = div((dt * c.g_mfs2) * u2, pow43(h2) + kEps);
         const double e1 = 1.0 + c1, e2 = 1.0 + c2 + c3;
-        const double det = 1.0 / fmad(e1, e2, -(c1 * c2));
+        const double det = rcp(fmad(e1, e2, -(c1 * c2)));
         w[1] = (h1 * fmad(u1x, e2, c1 * u2x)) * det;
         w[4] = (h2 * fmad(u2x, e1, c2 * u1x)) * det;
         w[2] = (h1 * fmad(u1y, e2, c1 * u2y)) * det;
@@ -517,13 +524,13 @@ LSH_HD void dis_implicita(const double wo[6], double w[6], double dt, const Cons
     }
     if (gt0(h1) && lt_pos(h2, eps)) {
         const double Y = pow43(h1) + kEps, X = (dt * c.g_mf02) * u1;
-        const double inv = Y / (Y + X);
+        const double inv = div(Y, Y + X);
         if (gt_pos(h1, eps)) { w[1] = w[1] * inv; w[2] = w[2] * inv; }
         else { w[1] = (h1 * (f1 * w[1])) * inv; w[2] = (h1 * (f1 * w[2])) * inv; }
     }
     if (gt0(h2) && lt_pos(h1, eps)) {
         const double Y = pow43(h2) + kEps, X = (dt * c.g_mfs2) * u2;
-        const double inv = Y / (Y + X);
+        const double inv = div(Y, Y + X);
         if (gt_pos(h2, eps)) { w[4] = w[4] * inv; w[5] = w[5] * inv; }
         else { w[4] = (h2 * (f2 * w[4])) * inv; w[5] = (h2 * (f2 * w[5])) * inv; }
     }
@@ -538,14 +545,14 @@ LSH_HD void coulomb(double w[6], double dt, const Consts& c) {
     }
     double mu = c.mu;
     if (c.law != 0) {
-        const double u1 = sqrt(fmad(w[1], w[1], w[2] * w[2])) * vfac(w[0], c.eps_h);
-        const double u2 = sqrt(fmad(w[4], w[4], w[5] * w[5])) * vfac(w[3], c.eps_h);
+        const double u1 = root(fmad(w[1], w[1], w[2] * w[2])) * vfac(w[0], c.eps_h);
+        const double u2 = root(fmad(w[4], w[4], w[5] * w[5])) * vfac(w[3], c.eps_h);
         mu = friction_mu(w[0], u1, w[3], u2, c);
     }
     const double sc = ((((fsc_of(w[0], c) * mu) * c.g) * w[3]) * dt);
-    const double normq = sqrt(fmad(w[4], w[4], w[5] * w[5]));
+    const double normq = root(fmad(w[4], w[4], w[5] * w[5]));
     double aux = 0.0;
-    if (!lt_pos(normq + sc, kEps) && !lt(normq, sc)) aux = normq / (normq + sc);
+    if (!lt_pos(normq + sc, kEps) && !lt(normq, sc)) aux = div(normq, normq + sc);
     w[4] = w[4] * aux;
     w[5] = w[5] * aux;
 }
