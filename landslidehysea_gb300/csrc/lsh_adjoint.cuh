@@ -58,6 +58,58 @@ LSH_HD double pow43_d(double h) {
 
 LSH_HD double sqrt_bar(double s, double sb) { return gt0(s) ? div_call(sb, 2.0 * s) : 0.0; }
 
+// Compare-and-swap sequence of Arista_kernel.cu:193-234 (with its (2,1)
+// compare) or, with `full`, the same sequence made a true sort.
+// The compares run on ordered keys (okey), which travel with the values.
+LSH_HD void cswap(double& a, double& b, int64_t& ka, int64_t& kb) {
+    if (ka > kb) {
+        const double t = a; a = b; b = t;
+        const int64_t k = ka; ka = kb; kb = k;
+    }
+}
+LSH_HD void sort_eig(V4& D, int full) {
+    int64_t kx = okey(D.x), ky = okey(D.y), kz = okey(D.z), kw = okey(D.w);
+    cswap(D.x, D.y, kx, ky);
+    cswap(D.x, D.z, kx, kz);
+    cswap(D.x, D.w, kx, kw);
+    cswap(D.y, D.z, ky, kz);
+    cswap(D.y, D.w, ky, kw);
+    if (full) cswap(D.y, D.z, ky, kz);
+    else cswap(D.z, D.y, kz, ky);
+    cswap(D.z, D.w, kz, kw);
+}
+
+// aproximarAutovalores1D (Arista_kernel.cu:152-237), all four values in order
+// (the adjoint has to know where each one went).  L2 == false: the
+// granular layer is absent (h2 = 0, u2 = 0), so the internal pair is exactly
+// zero and its square root is skipped.
+template <bool L2>
+LSH_HD V4 eig(double h1, double h2, double u1, double u2, double q, const Consts& c,
+                                  double Fknown = -1.0, double sqrt_h = -1.0, bool mean_u = false) {
+    const double h = L2 ? h1 + h2 : h1;
+    // mean_u (the edge average, q = h1 u1 + h2 u2): with no granular layer and
+    // h > eps_h, u = q vfac(h) = (h1 u1) / h1 is u1 itself -- an exact
+    // restatement the CPU oracle makes too; the single-layer edge then skips
+    // the division
+    const bool direct = mean_u && is_zero(h2) && gt_pos(h, c.eps_h);
+    double F = 0.0;
+    // single layer: vfac(h1 + 0) is vfac(h1), which the caller may already hold
+    if (L2 || !direct) F = (!L2 && !lt0(Fknown)) ? Fknown : vfac(h, c.eps_h);
+    const double u = direct ? u1 : q * F;
+    // sqrt_h >= 0: sqrt(h1) is known and h2 == 0, so sqrt(g h) = sqrt(g) sqrt(h1)
+    const double cg = !lt0(sqrt_h) ? c.sqrt_g * sqrt_h : root_call(c.g * h);
+    double uu = 0.0, ci = 0.0;
+    if (L2) {
+        uu = fmad(u1, h2, u2 * h1) * F;
+        const double d = u1 - u2;
+        const double aux = fmad(-((d * d) * F), c.inv_gp, 1.0);
+        ci = root_call((((c.gp * h1) * h2) * F) * abs_bits(aux));
+    }
+    V4 D{u - cg, uu - ci, uu + ci, u + cg};
+    sort_eig(D, c.eig_sort);
+    return D;
+}
+
 // The compare-and-swap network of sort_eig on values, carrying the labels
 // of the unsorted entries: after the call D[k] = entry perm[k].
 LSH_HD void sort_eig_perm(double D[4], int perm[4], int full) {

@@ -106,6 +106,46 @@ LSH_HD double vfac(double h, double eps_h) {
     return div(kSqrt2 * h, root(fmad(h2, h2, m2 * m2)));
 }
 
+// x / 2 and 2 x on the exponent field (integer pipe), the FP64 multiply only
+// where the result or x is not a normal number or zero
+LSH_HD double half(double x) {
+    uint32_t lo, hi;
+    lshm::halves(x, lo, hi);
+    if (((hi >> 20) & 0x7ffu) - 2u < 2045u) return lshm::from_halves(lo, hi - 0x00100000u);
+    if (((hi << 1) | lo) == 0u) return x;
+    return 0.5 * x;
+}
+LSH_HD double twice(double x) {
+    uint32_t lo, hi;
+    lshm::halves(x, lo, hi);
+    if (((hi >> 20) & 0x7ffu) - 1u < 2045u) return lshm::from_halves(lo, hi + 0x00100000u);
+    if (((hi << 1) | lo) == 0u) return x;
+    return 2.0 * x;
+}
+
+// 0 + x and 0 - x on the integer pipe: x and -x, with +0 for either zero (NaN
+// takes the FP64 operation: its sign steers the limiter's integer compares)
+LSH_HD double plus0(double x) {
+    uint32_t lo, hi;
+    lshm::halves(x, lo, hi);
+    return lshm::from_halves(lo, (lo == 0u && hi == 0x80000000u) ? 0u : hi);
+}
+LSH_HD double minus0(double x) {
+    uint32_t lo, hi;
+    lshm::halves(x, lo, hi);
+    if ((hi & 0x7ff00000u) == 0x7ff00000u) return 0.0 - x;
+    return lshm::from_halves(lo, (((hi << 1) | lo) == 0u) ? 0u : (hi ^ 0x80000000u));
+}
+
+// log2 x of a positive normal x in units of 2^-20, low by at most 0.0861
+// (the significand taken as its own logarithm): the high word, rebased
+LSH_HD int32_t log2_low(double x) {
+    uint32_t lo, hi;
+    lshm::halves(x, lo, hi);
+    return (int32_t)(hi & 0x7fffffffu) - 0x3ff00000;
+}
+constexpr int32_t kLog2One = 1 << 20;
+
 LSH_HD double pow43(double h) { return h * lshm::cbrt_pos(h); }
 
 LSH_HD int sgn(double x) { return abs_lt(x, kEps) ? 0 : (gt0(x) ? 1 : -1); }
@@ -124,32 +164,44 @@ LSH_HD bool is_bad(double x) {
     return (hi & 0x7ff00000u) == 0x7ff00000u;
 }
 
-// Compare-and-swap sequence of Arista_kernel.cu:193-234 (with its (2,1)
-// compare) or, with `full`, the same sequence made a true sort.
-// The compares run on ordered keys (okey), which travel with the values.
-LSH_HD void cswap(double& a, double& b, int64_t& ka, int64_t& kb) {
-    if (ka > kb) {
-        const double t = a; a = b; b = t;
-        const int64_t k = ka; ka = kb; kb = k;
+// Bounds of the four eigenvalue estimates as the compare-and-swap sequence of
+// Arista_kernel.cu:193-234 leaves them (with its (2,1) compare, or with `full`
+// the same sequence made a true sort): its first and last value and the
+// larger magnitude of the two between.  The estimates are a = u - c, b = u' -
+// c', c = u' + c', d = u + c with a <= d and b <= c (rounding is monotone), so
+// of its seven compares three can swap:
+//   first (a, b); then the larger of those against d, which is above d only
+//   when b is.  Last: the (2,1) form leaves max(b, d) and between it
+//   {c, d or max(a, b)}; the true sort max(c, d), with {max(a, b), min(c, d)}.
+struct EigBounds { double lo, hi, mid; };
+LSH_HD EigBounds eig_bounds(double a, double b, double c, double d, int full) {
+    EigBounds e;
+    const bool ab = lt(b, a);
+    e.lo = ab ? b : a;
+    const double top = ab ? a : b;
+    double m1, m2;
+    if (full) {
+        const bool cd = lt(d, c);
+        e.hi = cd ? c : d;
+        m1 = top;
+        m2 = cd ? d : c;
+    } else {
+        const bool bd = lt(d, b);
+        e.hi = bd ? b : d;
+        m1 = bd ? d : top;
+        m2 = c;
     }
-}
-LSH_HD void sort_eig(V4& D, int full) {
-    int64_t kx = okey(D.x), ky = okey(D.y), kz = okey(D.z), kw = okey(D.w);
-    cswap(D.x, D.y, kx, ky);
-    cswap(D.x, D.z, kx, kz);
-    cswap(D.x, D.w, kx, kw);
-    cswap(D.y, D.z, ky, kz);
-    cswap(D.y, D.w, ky, kw);
-    if (full) cswap(D.y, D.z, ky, kz);
-    else cswap(D.z, D.y, kz, ky);
-    cswap(D.z, D.w, kz, kw);
+    m1 = abs_bits(m1);
+    m2 = abs_bits(m2);
+    e.mid = lt_pos(m1, m2) ? m2 : m1;
+    return e;
 }
 
 // aproximarAutovalores1D (Arista_kernel.cu:152-237).  L2 == false: the
 // granular layer is absent (h2 = 0, u2 = 0), so the internal pair is exactly
 // zero and its square root is skipped.
 template <bool L2>
-LSH_HD V4 eig(double h1, double h2, double u1, double u2, double q, const Consts& c,
+LSH_HD EigBounds eig_edge(double h1, double h2, double u1, double u2, double q, const Consts& c,
                                   double Fknown = -1.0, double sqrt_h = -1.0, bool mean_u = false) {
     const double h = L2 ? h1 + h2 : h1;
     // mean_u (the edge average, q = h1 u1 + h2 u2): with no granular layer and
@@ -163,16 +215,18 @@ LSH_HD V4 eig(double h1, double h2, double u1, double u2, double q, const Consts
     const double u = direct ? u1 : q * F;
     // sqrt_h >= 0: sqrt(h1) is known and h2 == 0, so sqrt(g h) = sqrt(g) sqrt(h1)
     const double cg = !lt0(sqrt_h) ? c.sqrt_g * sqrt_h : root(c.g * h);
-    double uu = 0.0, ci = 0.0;
-    if (L2) {
-        uu = fmad(u1, h2, u2 * h1) * F;
-        const double d = u1 - u2;
-        const double aux = fmad(-((d * d) * F), c.inv_gp, 1.0);
-        ci = root((((c.gp * h1) * h2) * F) * abs_bits(aux));
+    const double a = u - cg, d = u + cg;
+    if (!L2) {
+        // the internal pair is 0, 0: both sorts leave min(a, 0), max(d, 0) and
+        // between them 0 and the external value on the other side of 0, if any
+        const bool up = gt0(a), down = lt0(d);
+        return EigBounds{up ? 0.0 : a, down ? 0.0 : d, up ? a : (down ? abs_bits(d) : 0.0)};
     }
-    V4 D{u - cg, uu - ci, uu + ci, u + cg};
-    sort_eig(D, c.eig_sort);
-    return D;
+    const double uu = fmad(u1, h2, u2 * h1) * F;
+    const double du = u1 - u2;
+    const double aux = fmad(-((du * du) * F), c.inv_gp, 1.0);
+    const double ci = root((((c.gp * h1) * h2) * F) * abs_bits(aux));
+    return eig_bounds(a, uu - ci, uu + ci, d, c.eig_sort);
 }
 
 // defTerminoFriccion (Arista_kernel.cu:11-58)
@@ -195,6 +249,9 @@ LSH_HD double friction_mu(double h1, double u1, double h2, double u2, const Cons
 }
 
 LSH_HD double fsc_of(double h1, const Consts& c) {
+    // above 4 eps_h the exponent's argument is beyond 746 (40^2) and
+    // exp_neg gives 0, so this is 1 - r (1 - 0) = 1 - r
+    if (log2_low(h1) - log2_low(c.eps_h) > 3 * kLog2One && gt0(h1)) return 1.0 - c.r;
     const double a = (10.0 * h1) * c.inv_eps;
     return 1.0 - c.r * (1.0 - exp_neg(a * a));
 }
@@ -226,45 +283,61 @@ struct EdgeInPos {
     LSH_HD double acch(int side, int layer) const { return side ? e.acc1h[layer] : e.acc0h[layer]; }
 };
 
-// procesarArista (Arista_kernel.cu:324-645), the depths already known to be
-// wet (the caller skips dry edges, :397).  L2 == false: both faces have no
-// granular layer (h2 = qn2 = 0); every layer-1 value is then the same as in
-// the general path and every layer-2 output is zero, so that work is skipped.
-// `pos` supplies the positivity limiter's inputs (cell areas, cell depths and
-// the partial accumulators of the cells' depths; EdgeInPos reads them from
-// `e`): a caller may load them only where the limiter needs them, so they do
-// not stay live through the flux computation.
-template <bool L2, class Pos>
-LSH_HD void edge_flux(const EdgeIn& e, double dt, const Consts& c, EdgeOut& o, const Pos& pos) {
-    const double eps = c.eps_h;
-    double Aq1 = e.A.qn1, Aq2 = L2 ? e.A.qn2 : 0.0, Bq1 = e.B.qn1, Bq2 = L2 ? e.B.qn2 : 0.0;
-    const double Ah1 = e.A.h1, Bh1 = e.B.h1;
-    const double Ah2 = L2 ? e.A.h2 : 0.0, Bh2 = L2 ? e.B.h2 : 0.0;
-    const double H0 = e.A.H, H1 = e.B.H;
-    const double h1ij = 0.5 * (Ah1 + Bh1);
-    const double h2ij = L2 ? 0.5 * (Ah2 + Bh2) : 0.0;
+// The flux of one edge before the positivity limiter, in the normal frame and
+// times the edge length: m (mass, normal and tangential momentum of each
+// layer, for cell 0) and p (mass and normal momentum, for cell 1; its
+// tangential momentum is -m[3 l + 2]), and the wave term.
+struct EdgeRaw { double m[6], p[4], wave; };
 
-    // tratamientoSecoMojado (Arista_kernel.cu:301-321)
+// procesarArista (Arista_kernel.cu:324-645) up to the limiter, the depths
+// already known to be wet (the caller skips dry edges, :397).  L2 == false:
+// both faces have no granular layer (h2 = qn2 = 0); every layer-1 value is
+// then the same as in the general path and every layer-2 output is zero, so
+// that work is skipped.
+//
+// The FP64 unit bounds this (16 cycles per instruction and SM, 55 cycles of
+// latency), so what gives the same bits off it runs on the integer pipe:
+// divisions and roots (lsh_ieee.h), halvings, sums with zero, compares, the
+// eigenvalue bounds' order (eig_bounds), and the differences of eigenvalues
+// with an aut2 of zero.
+template <bool L2>
+LSH_HD void edge_raw(const Face& A, const Face& B, double len, double dt, const Consts& c, EdgeRaw& o) {
+    const double eps = c.eps_h;
+    double Aq1 = A.qn1, Aq2 = L2 ? A.qn2 : 0.0, Bq1 = B.qn1, Bq2 = L2 ? B.qn2 : 0.0;
+    const double Ah1 = A.h1, Bh1 = B.h1;
+    const double Ah2 = L2 ? A.h2 : 0.0, Bh2 = L2 ? B.h2 : 0.0;
+    const double H0 = A.H, H1 = B.H;
+    const double h1ij = half(Ah1 + Bh1);
+    const double h2ij = L2 ? half(Ah2 + Bh2) : 0.0;
+
+    // tratamientoSecoMojado (Arista_kernel.cu:301-321): the conditions on
+    // layer 1 need its depth below eps_h on one side (or a negative h2)
     if (L2) {
         if (lt_pos(Ah2, eps) && lt(H0, H1 - Bh2)) Bq2 = 0.0;
         if (lt_pos(Bh2, eps) && lt(H1, H0 - Ah2)) Aq2 = 0.0;
-        if (lt_pos(Ah1, eps) && lt(H0 - Ah2, H1 - Bh1 - Bh2)) Bq1 = 0.0;
-        if (lt_pos(Bh1, eps) && lt(H1 - Bh2, H0 - Ah1 - Ah2)) Aq1 = 0.0;
-        if (lt_pos(Ah2 + Ah1, eps) && lt(H0, H1 - Bh1 - Bh2)) { Bq1 = 0.0; Bq2 = 0.0; }
-        if (lt_pos(Bh2 + Bh1, eps) && lt(H1, H0 - Ah1 - Ah2)) { Aq1 = 0.0; Aq2 = 0.0; }
-    } else {
+        if (lt_pos(Ah1, eps) || lt_pos(Bh1, eps) || lt0(Ah2) || lt0(Bh2)) {
+            if (lt_pos(Ah1, eps) && lt(H0 - Ah2, H1 - Bh1 - Bh2)) Bq1 = 0.0;
+            if (lt_pos(Bh1, eps) && lt(H1 - Bh2, H0 - Ah1 - Ah2)) Aq1 = 0.0;
+            if (lt_pos(Ah2 + Ah1, eps) && lt(H0, H1 - Bh1 - Bh2)) { Bq1 = 0.0; Bq2 = 0.0; }
+            if (lt_pos(Bh2 + Bh1, eps) && lt(H1, H0 - Ah1 - Ah2)) { Aq1 = 0.0; Aq2 = 0.0; }
+        }
+    } else if (lt_pos(Ah1, eps) || lt_pos(Bh1, eps)) {
         if (lt_pos(Ah1, eps) && lt(H0, H1 - Bh1)) Bq1 = 0.0;
         if (lt_pos(Bh1, eps) && lt(H1, H0 - Ah1)) Aq1 = 0.0;
     }
 
     const double fA1 = vfac(Ah1, eps), fB1 = vfac(Bh1, eps);
-    const double fA2 = L2 ? vfac(Ah2, eps) : 0.0, fB2 = L2 ? vfac(Bh2, eps) : 0.0;
     const double sa1 = root(Ah1), sb1 = root(Bh1);
-    const double u1ij = div(fmad(sa1, fA1 * Aq1, sb1 * (fB1 * Bq1)), sa1 + sb1 + kEps);
-    double u2ij = 0.0;
+    const double uA1 = fA1 * Aq1, uB1 = fB1 * Bq1;
+    const double u1ij = div(fmad(sa1, uA1, sb1 * uB1), sa1 + sb1 + kEps);
+    double u2ij = 0.0, uA2 = 0.0, uB2 = 0.0, fA2 = 0.0, fB2 = 0.0;
     if (L2) {
+        fA2 = vfac(Ah2, eps);
+        fB2 = vfac(Bh2, eps);
         const double sa2 = root(Ah2), sb2 = root(Bh2);
-        u2ij = div(fmad(sa2, fA2 * Aq2, sb2 * (fB2 * Bq2)), sa2 + sb2 + kEps);
+        uA2 = fA2 * Aq2;
+        uB2 = fB2 * Bq2;
+        u2ij = div(fmad(sa2, uA2, sb2 * uB2), sa2 + sb2 + kEps);
     }
     // a face's celerity sqrt(g h) is sqrt(g) sqrt(h1) when its granular layer is empty
     const bool oneA = !L2 || is_zero(Ah2), oneB = !L2 || is_zero(Bh2);
@@ -273,140 +346,173 @@ LSH_HD void edge_flux(const EdgeIn& e, double dt, const Consts& c, EdgeOut& o, c
     const double deta1 = L2 ? max0(Bh1 + Bh2 - H1 + Hm) - max0(Ah1 + Ah2 - H0 + Hm)
                             : max0(Bh1 - H1 + Hm) - max0(Ah1 - H0 + Hm);
     const double deta2 = L2 ? max0(Bh2 - H1 + Hm) - max0(Ah2 - H0 + Hm) : 0.0;
-    const double gh1 = c.g * h1ij, gh2 = c.g * h2ij;
-    const V4 tp{0.0, gh1 * deta1, 0.0, L2 ? gh2 * fmad(c.omr, deta2, c.r * deta1) : 0.0};
+    const double gh1 = c.g * h1ij, gh2 = L2 ? c.g * h2ij : 0.0;
+    const double p1 = gh1 * deta1;                                            // pressure terms
+    const double p2 = L2 ? gh2 * fmad(c.omr, deta2, c.r * deta1) : 0.0;
 
     bool coul = false;
-    V4 tp2 = tp;
+    double p2c = p2;
     if (L2) {
         const double mu = friction_mu(h1ij, u1ij, h2ij, u2ij, c);
         const double sc = ((fsc_of(h1ij, c) * mu) * c.g) * h2ij;
         coul = lt(abs_bits(h2ij * u2ij), (c.peso * sc) * dt);
-        if (coul) tp2.w = (gh2 * c.r) * deta1;
+        if (coul) p2c = (gh2 * c.r) * deta1;
     }
 
-    const V4 D = eig<L2>(h1ij, h2ij, u1ij, u2ij, L2 ? fmad(h1ij, u1ij, h2ij * u2ij) : h1ij * u1ij, c, -1.0, -1.0, true);
-    const V4 E0 = eig<L2>(Ah1, Ah2, fA1 * Aq1, fA2 * Aq2, L2 ? Aq1 + Aq2 : Aq1, c, fA1, oneA ? sa1 : -1.0);
-    const V4 E1 = eig<L2>(Bh1, Bh2, fB1 * Bq1, fB2 * Bq2, L2 ? Bq1 + Bq2 : Bq1, c, fB1, oneB ? sb1 : -1.0);
-    const double aut1 = tmin(D.x, tmin(E0.x, E1.x));
-    const double aut3 = tmax(D.w, tmax(E0.w, E1.w));
-    double lmax = tmax(abs_bits(aut3), abs_bits(aut1));
+    const EigBounds D = eig_edge<L2>(h1ij, h2ij, u1ij, u2ij, L2 ? fmad(h1ij, u1ij, h2ij * u2ij) : h1ij * u1ij, c, -1.0, -1.0, true);
+    const EigBounds E0 = eig_edge<L2>(Ah1, Ah2, uA1, uA2, L2 ? Aq1 + Aq2 : Aq1, c, fA1, oneA ? sa1 : -1.0);
+    const EigBounds E1 = eig_edge<L2>(Bh1, Bh2, uB1, uB2, L2 ? Bq1 + Bq2 : Bq1, c, fB1, oneB ? sb1 : -1.0);
+    const double aut1 = tmin(D.lo, tmin(E0.lo, E1.lo));
+    const double aut3 = tmax(D.hi, tmax(E0.hi, E1.hi));
+    const double b1 = abs_bits(aut1), b3 = abs_bits(aut3);
+    double lmax = tmax(b3, b1);
     const double umax = L2 ? tmax(abs_bits(u1ij), abs_bits(u2ij)) : abs_bits(u1ij);
     if (lt(lmax, umax)) lmax = umax;
-    double aut2 = tmax(abs_bits(D.y), abs_bits(D.z));
-    aut2 = lshm::neg_if(aut2, sgn(aut1 + aut3) < 0);
+    double aut2 = D.mid;
+    double d12 = aut1, d23 = minus0(aut3);  // aut1 - aut2, aut2 - aut3 with aut2 = 0
+    if (L2 || !is_zero(aut2)) {
+        aut2 = lshm::neg_if(aut2, sgn(aut1 + aut3) < 0);
+        d12 = aut1 - aut2;
+        d23 = aut2 - aut3;
+    }
+    const double d13 = aut1 - aut3;
 
     double a0, a1, a2 = 0.0;
-    if (!abs_lt(aut1 - aut3, kEps) && !abs_lt(aut1 - aut2, kEps) && !abs_lt(aut2 - aut3, kEps)) {
+    if (!abs_lt(d13, kEps) && !abs_lt(d12, kEps) && !abs_lt(d23, kEps)) {
         if (L2 && !lt_pos(h1ij, eps) && !lt_pos(h2ij, eps)) {
-            const double d12 = aut1 - aut2, d13 = aut1 - aut3, d23 = aut2 - aut3;
             const double inv = rcp((d12 * d13) * d23);
-            const double a = (abs_bits(aut1) * d23) * inv;
+            const double a = (b1 * d23) * inv;
             const double b = -((abs_bits(aut2) * d13) * inv);
-            const double cc = (abs_bits(aut3) * d12) * inv;
+            const double cc = (b3 * d12) * inv;
             a0 = fmad(a * aut2, aut3, fmad(b * aut1, aut3, (cc * aut1) * aut2));
             a1 = -fmad(a, aut2 + aut3, fmad(b, aut1 + aut3, cc * (aut1 + aut2)));
             a2 = a + b + cc;
         } else {
-            const double inv = rcp(aut3 - aut1);
-            a0 = fmad(aut3, abs_bits(aut1), -(aut1 * abs_bits(aut3))) * inv;
-            a1 = (abs_bits(aut3) - abs_bits(aut1)) * inv;
+            const double inv = rcp(lshm::neg_if(d13, true));  // 1 / (aut3 - aut1), not 0
+            a0 = fmad(aut3, b1, -(aut1 * b3)) * inv;
+            a1 = (b3 - b1) * inv;
         }
     } else {
         a0 = lmax; a1 = 0.0;
     }
 
-    const double FAy = lt_pos(Ah1, kEps) ? 0.0 : (fA1 * Aq1) * Aq1, FBy = lt_pos(Bh1, kEps) ? 0.0 : (fB1 * Bq1) * Bq1;
+    const double FAy = lt_pos(Ah1, kEps) ? 0.0 : uA1 * Aq1, FBy = lt_pos(Bh1, kEps) ? 0.0 : uB1 * Bq1;
     const double dFx = Bq1 - Aq1, dFy = FBy - FAy;
-    double dFz = 0.0, dFw = 0.0, FAw = 0.0, FBw = 0.0;
-    if (L2) {
-        FAw = lt_pos(Ah2, kEps) ? 0.0 : (fA2 * Aq2) * Aq2;
-        FBw = lt_pos(Bh2, kEps) ? 0.0 : (fB2 * Bq2) * Bq2;
-        dFz = Bq2 - Aq2;
-        dFw = FBw - FAw;
-    }
-    tp2 = V4{tp2.x + dFx, tp2.y + dFy, tp2.z + dFz, tp2.w + dFw};
-    const double half_x = 0.5 * (dFx + tp.x), half_y = 0.5 * (dFy + tp.y);
+    const double tx = plus0(dFx), ty = p1 + dFy;
+    const double half_x = half(tx), half_y = half(ty);  // dF + pressure is ty with the terms exchanged
 
-    const double Atx = tp2.y;
-    const double Aty = fmad(gh1, tp2.z, fmad(u1ij + u1ij, tp2.y, fmad(-u1ij, u1ij, gh1) * tp2.x));
-
-    V4 I{deta1, Bq1 - Aq1, 0.0, Bq2 - Aq2};
-    if (!coul) {
-        if (gt_pos(Ah1, eps) && gt_pos(Bh1, eps)) I.x = I.x - deta2;
-        I.z = deta2;
-    }
+    double Ix = deta1;
+    if (L2 && !coul && gt_pos(Ah1, eps) && gt_pos(Bh1, eps)) Ix = Ix - deta2;
+    // deta2 is 0 without a granular layer: x - 0 is x
 
     double Qx, Qy;
     if (L2) {
-        Qx = 0.5 * fmad(a0, I.x, fmad(a1, tp2.x, a2 * Atx));
-        Qy = 0.5 * fmad(a0, I.y, fmad(a1, tp2.y, a2 * Aty));
+        const double dFz = Bq2 - Aq2;
+        const double tz = plus0(dFz);
+        const double FAw = lt_pos(Ah2, kEps) ? 0.0 : uA2 * Aq2, FBw = lt_pos(Bh2, kEps) ? 0.0 : uB2 * Bq2;
+        const double dFw = FBw - FAw;
+        const double tw = p2c + dFw;
+        const double Atx = ty;
+        const double Aty = fmad(gh1, tz, fmad(u1ij + u1ij, ty, fmad(-u1ij, u1ij, gh1) * tx));
+        Qx = half(fmad(a0, Ix, fmad(a1, tx, a2 * Atx)));
+        Qy = half(fmad(a0, dFx, fmad(a1, ty, a2 * Aty)));
+        const double Iz = coul ? 0.0 : deta2;
+        const double Atz = tw;
+        const double Atw = fmad(c.r * gh2, tx, fmad(fmad(-u2ij, u2ij, gh2), tz, (u2ij + u2ij) * tw));
+        const double Qz = half(fmad(a0, Iz, fmad(a1, tz, a2 * Atz)));
+        const double Qw = half(fmad(a0, dFz, fmad(a1, tw, a2 * Atw)));
+        const double half_z = half(tz), half_w = half(dFw + p2);
+        const double Fmz = half_z + (Aq2 - Qz), Fmw = half_w + (FAw - Qw);
+        const double Fpz = half_z + (Qz - Bq2), Fpw = half_w + (Qw - FBw);
+        const double u2t = abs_lt(Fmz, kEps) ? 0.0 : (gt0(Fmz) ? fA2 * A.qt2 : fB2 * B.qt2);
+        o.m[3] = len * Fmz; o.m[4] = len * Fmw; o.m[5] = len * (Fmz * u2t);
+        o.p[2] = len * Fpz; o.p[3] = len * Fpw;
     } else {
-        Qx = 0.5 * fmad(a0, I.x, a1 * tp2.x);
-        Qy = 0.5 * fmad(a0, I.y, a1 * tp2.y);
+        Qx = half(fmad(a0, Ix, a1 * tx));
+        Qy = half(fmad(a0, dFx, a1 * ty));
+        o.m[3] = o.m[4] = o.m[5] = o.p[2] = o.p[3] = 0.0;
     }
     const double Fmx = half_x + (Aq1 - Qx), Fmy = half_y + (FAy - Qy);
     const double Fpx = half_x + (Qx - Bq1), Fpy = half_y + (Qy - FBy);
+    const double u1t = abs_lt(Fmx, kEps) ? 0.0 : (gt0(Fmx) ? fA1 * A.qt1 : fB1 * B.qt1);
+    o.m[0] = len * Fmx; o.m[1] = len * Fmy; o.m[2] = len * (Fmx * u1t);
+    o.p[0] = len * Fpx; o.p[1] = len * Fpy;
+    if (lt_pos(lmax, eps)) lmax = lmax + eps;
+    o.wave = len * lmax;
+}
 
-    const double u1t = abs_lt(Fmx, kEps) ? 0.0 : (gt0(Fmx) ? fA1 * e.A.qt1 : fB1 * e.B.qt1);
-    const double s1 = Fmx * u1t;
-    double M[6] = {Fmx, Fmy, s1, 0.0, 0.0, 0.0};
-    double P[6] = {Fpx, Fpy, -s1, 0.0, 0.0, 0.0};
-    if (L2) {
-        const double Atz = tp2.w;
-        const double Atw = fmad(c.r * gh2, tp2.x, fmad(fmad(-u2ij, u2ij, gh2), tp2.z, (u2ij + u2ij) * tp2.w));
-        const double Qz = 0.5 * fmad(a0, I.z, fmad(a1, tp2.z, a2 * Atz));
-        const double Qw = 0.5 * fmad(a0, I.w, fmad(a1, tp2.w, a2 * Atw));
-        const double half_z = 0.5 * (dFz + tp.z), half_w = 0.5 * (dFw + tp.w);
-        const double Fmz = half_z + (Aq2 - Qz), Fmw = half_w + (FAw - Qw);
-        const double Fpz = half_z + (Qz - Bq2), Fpw = half_w + (Qw - FBw);
-        const double u2t = abs_lt(Fmz, kEps) ? 0.0 : (gt0(Fmz) ? fA2 * e.A.qt2 : fB2 * e.B.qt2);
-        const double s2 = Fmz * u2t;
-        M[3] = Fmz; M[4] = Fmw; M[5] = s2;
-        P[3] = Fpz; P[4] = Fpw; P[5] = -s2;
+// The positivity limiter's factor of one layer of an edge (Arista_kernel.cu:
+// 554-609), 1 where it does not act: m and p are the mass terms of cells 0 and
+// 1, h the cells' depths and acc the partial sums before this edge.  A side
+// limits when dt exceeds the time it takes to empty its layer, hp area /
+// (beta out + eps): tested as dt (beta out + eps) > hp area (the denominator
+// is positive), so the divisions run only on limited edges.
+LSH_HD double limiter(double m, double p, bool interior, double h0, double acc0, double area0, double inv_area0,
+                      double h1, double acc1, double area1, double inv_area1, double dt, const Consts& c) {
+    const bool oa = gt0(m), ob = interior && gt0(p);
+    double ha = 0.0, hb = 0.0, da = 1.0, db = 1.0;
+    bool lim = false;
+    if (oa) {
+        ha = fmad(dt * inv_area0, acc0, h0) * area0;
+        da = fmad(c.beta, m, kEps);
+        lim = lt(ha, dt * da);
     }
-    constexpr int KL = L2 ? 6 : 3;
-#pragma unroll
-    for (int k = 0; k < KL; ++k) { P[k] = e.len * P[k]; M[k] = e.len * M[k]; }
+    if (ob) {
+        hb = fmad(dt * inv_area1, acc1, h1) * area1;
+        db = fmad(c.beta, p, kEps);
+        lim = lim || lt(hb, dt * db);
+    }
+    if (!lim) return 1.0;
+    const double dta = oa ? div(ha, da) : kBig, dtb = ob ? div(hb, db) : kBig;
+    return div(tmin(dta, dtb), dt + kEps);
+}
 
-    const double b0 = dt * pos.inv_area(0);
-    const double hp00 = fmad(b0, pos.acch(0, 0), pos.hc(0, 0));
-    const double hp01 = L2 ? fmad(b0, pos.acch(0, 1), pos.hc(0, 1)) : 0.0;
-    double hp10 = 0.0, hp11 = 0.0;
-    if (e.interior) {
-        const double b1 = dt * pos.inv_area(1);
-        hp10 = fmad(b1, pos.acch(1, 0), pos.hc(1, 0));
-        if (L2) hp11 = fmad(b1, pos.acch(1, 1), pos.hc(1, 1));
-    }
-    const double factor = 1.0 * c.beta;
+// Whether a loss `out` (> 0) is far from emptying a layer of depth h: both
+// dt scale out and dt eps at most an eighth of h area, by the operands'
+// logarithms (log2_low is low by at most 0.0861: 3 + 3 x 0.0861 < 3.5; in half
+// units, so that four of them add up in 32 bits).  With scale >= 1, beta and
+// peso, a cell all of whose losses pass keeps at least a quarter of its
+// content whatever the order of its edges and the others' limiter, so the
+// limiter's test is false on each of its sides.
+LSH_HD bool far_from_empty(double out, double h, double area, double dt, double scale) {
+    const int32_t room = (log2_low(h) >> 1) + (log2_low(area) >> 1) - (log2_low(dt) >> 1) - 7 * (kLog2One / 4);
+    return gt_pos(h, 0x1p-900) && (log2_low(out) >> 1) + (log2_low(scale) >> 1) <= room &&
+           (log2_low(kEps) >> 1) <= room;
+}
+
+// procesarArista with the positivity limiter: the edge's terms to subtract
+// from its cells' accumulators and to add to their wave sums.
+// `pos` supplies the limiter's inputs (cell areas, cell depths and the partial
+// accumulators of the cells' depths; EdgeInPos reads them from `e`): a caller
+// may load them only where the limiter needs them, so they do not stay live
+// through the flux computation.
+template <bool L2, class Pos>
+LSH_HD void edge_flux(const EdgeIn& e, double dt, const Consts& c, EdgeOut& o, const Pos& pos) {
+    EdgeRaw w;
+    edge_raw<L2>(e.A, e.B, e.len, dt, c, w);
+    o.wave = w.wave;
 #pragma unroll
-    for (int layer = 0; layer < (L2 ? 2 : 1); ++layer) {
-        const int k = 3 * layer;
-        // limited when dt exceeds the time a side takes to empty its layer,
-        // hp area / (beta M + eps): tested as dt (beta M + eps) > hp area (the
-        // denominator is positive), so the divisions run only on limited edges
-        const bool oa = gt0(M[k]), ob = e.interior && gt0(P[k]);
-        const double ha = (layer ? hp01 : hp00) * pos.area(0), hb = (layer ? hp11 : hp10) * pos.area(1);
-        const double da = oa ? fmad(factor, M[k], kEps) : 1.0, db = ob ? fmad(factor, P[k], kEps) : 1.0;
-        const bool lim = (oa && lt(ha, dt * da)) || (ob && lt(hb, dt * db));
-        if (lim) {
-            const double dta = oa ? div(ha, da) : kBig, dtb = ob ? div(hb, db) : kBig;
-            const double dtl = tmin(dta, dtb);
-            const double alpha = div(dtl, dt + kEps);
+    for (int l = 0; l < 2; ++l) {
+        const int k = 3 * l;
+        o.m[k] = w.m[k]; o.m[k + 1] = w.m[k + 1]; o.m[k + 2] = w.m[k + 2];
+        o.p[k] = w.p[2 * l]; o.p[k + 1] = w.p[2 * l + 1]; o.p[k + 2] = lshm::neg_if(w.m[k + 2], true);
+        if (l == 1 && !L2) break;
+        if (gt0(o.m[k]) || (e.interior && gt0(o.p[k]))) {
+            const double alpha = limiter(o.m[k], o.p[k], e.interior, pos.hc(0, l), pos.acch(0, l), pos.area(0),
+                                         pos.inv_area(0), pos.hc(1, l), pos.acch(1, l), pos.area(1), pos.inv_area(1),
+                                         dt, c);
+            if (lshm::bits_of(alpha) != lshm::bits_of(1.0)) {
 #pragma unroll
-            for (int q = 0; q < 3; ++q) { M[k + q] = alpha * M[k + q]; P[k + q] = alpha * P[k + q]; }
+                for (int q = 0; q < 3; ++q) { o.m[k + q] = alpha * o.m[k + q]; o.p[k + q] = alpha * o.p[k + q]; }
+            }
         }
     }
-
-    if (lt_pos(lmax, eps)) lmax = lmax + eps;
-    o.wave = e.len * lmax;
+    if (!L2) { o.p[3] = o.p[4] = o.p[5] = 0.0; }
     if (lshm::bits_of(c.peso) != lshm::bits_of(1.0)) {
         o.wave = o.wave * c.inv_peso;
 #pragma unroll
-        for (int k = 0; k < 6; ++k) { M[k] = c.peso * M[k]; P[k] = c.peso * P[k]; }
+        for (int k = 0; k < 6; ++k) { o.m[k] = c.peso * o.m[k]; o.p[k] = c.peso * o.p[k]; }
     }
-#pragma unroll
-    for (int k = 0; k < 6; ++k) { o.m[k] = M[k]; o.p[k] = P[k]; }
 }
 
 template <bool L2>
@@ -417,16 +523,16 @@ LSH_HD void edge_flux(const EdgeIn& e, double dt, const Consts& c, EdgeOut& o) {
 // procesarAristaDeltaTInicial: wave-speed bound for the initial dt.
 LSH_HD double edge_initial_wave(const Face& A, const Face& B, double len, const Consts& c) {
     const double eps = c.eps_h;
-    const double h1ij = 0.5 * (A.h1 + B.h1);
+    const double h1ij = half(A.h1 + B.h1);
     const double fA1 = vfac(A.h1, eps), fB1 = vfac(B.h1, eps);
     double sa = root(A.h1), sb = root(B.h1);
     const double u1ij = div(fmad(sa, fA1 * A.qn1, sb * (fB1 * B.qn1)), sa + sb + kEps);
-    const double h2ij = 0.5 * (A.h2 + B.h2);
+    const double h2ij = half(A.h2 + B.h2);
     const double fA2 = vfac(A.h2, eps), fB2 = vfac(B.h2, eps);
     sa = root(A.h2); sb = root(B.h2);
     const double u2ij = div(fmad(sa, fA2 * A.qn2, sb * (fB2 * B.qn2)), sa + sb + kEps);
-    const V4 D = eig<true>(h1ij, h2ij, u1ij, u2ij, fmad(h1ij, u1ij, h2ij * u2ij), c);
-    double lmax = tmax(D.x, D.w);
+    const EigBounds D = eig_edge<true>(h1ij, h2ij, u1ij, u2ij, fmad(h1ij, u1ij, h2ij * u2ij), c);
+    double lmax = tmax(D.lo, D.hi);
     const double b = tmax(abs_bits(u1ij), abs_bits(u2ij));
     if (lt(lmax, b)) lmax = b;
     if (lt_pos(lmax, eps)) lmax = lmax + eps;
@@ -442,12 +548,13 @@ LSH_HD void filtro(double w[6], double dt, const Consts& c) {
 #pragma unroll
     for (int layer = 0; layer < (L2 ? 2 : 1); ++layer) {
         const int k = 3 * layer;
+        // exp(-dt/d), d = (w/eps_h)^4 + EPSILON, is exactly 1 once dt/d < 2^-54:
+        // skipped by the operands' logarithms (log2_low: 4 log2(w/eps_h) above
+        // log2 dt + 54 + 0.1 with a margin of 0.4 for the roundings)
+        if ((log2_low(dt) >> 2) + 13 * kLog2One + 5 * (kLog2One / 8) < log2_low(w[k]) + log2_low(c.inv_eps)) continue;
         const double x = w[k] * c.inv_eps;
         const double x2 = x * x;
         const double d = fmad(x2, x2, kEps);
-        // exp(-dt/d) is exactly 1 once dt/d < 2^-54: skip the division below a
-        // bound that holds with ample margin over the roundings
-        if (lt_pos(dt, d * 0x1.fp-55)) continue;  // d >= EPSILON: the bound is positive
         const double aux = exp_neg(dt * rcp(d));
         w[k + 1] = w[k + 1] * aux;
         w[k + 2] = w[k + 2] * aux;
@@ -470,6 +577,13 @@ LSH_HD void filtro(double w[6], double dt, const Consts& c) {
     }
 }
 
+// X < 2^-55 max(h, EPSILON) for h >= 1, X < 2^-55 EPSILON below, by the
+// operands' logarithms (log2_low)
+LSH_HD bool still_water(double X, double h) {
+    const int32_t lh = log2_low(h), le = log2_low(kEps);
+    return log2_low(X) + kLog2One / 8 < ((lh > 0) ? lh : le) - 55 * kLog2One;
+}
+
 // disImplicita (Volumen_kernel.cu:31-90).  L2 == false: the new and the old
 // granular layer are empty (h2 = q2 = 0): only the water-bottom branch can run.
 // fo1 = vfac(wo[0]), the old state's water factor, computed by the caller.
@@ -486,7 +600,11 @@ LSH_HD void dis_implicita(const double wo[6], double w[6], double dt, const Cons
         // bottom friction h u / (1 + c1), 1/(1 + X/Y) = Y/(Y + X); above
         // eps_h, h u is q itself
         if (gt0(h1)) {
-            const double Y = pow43(h1) + kEps, X = (dt * c.g_mf02) * u1;
+            const double X = (dt * c.g_mf02) * u1;
+            // X below 2^-54 of Y >= max(min(h, h^(4/3)), EPSILON): Y + X is Y and
+            // inv is 1 (h at least 1 there, so h <= h^(4/3))
+            if (gt_pos(h1, eps) && still_water(X, h1)) return;
+            const double Y = pow43(h1) + kEps;
             const double inv = div(Y, Y + X);
             if (gt_pos(h1, eps)) { w[1] = w[1] * inv; w[2] = w[2] * inv; }
             else {
