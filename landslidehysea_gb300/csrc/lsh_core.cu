@@ -99,6 +99,8 @@ struct lsh_ctx {
     double* eta_max = nullptr;
     double* eta_time = nullptr;
     unsigned char* szero = nullptr;  // order 2: per-cell "stored slopes are zero" flags
+    void* edge_mem = nullptr;        // the flux pass's edge buffers (null: the colour passes run)
+    FluxMem flux{};
     unsigned* dep_ctr = nullptr;     // pass-overlap counters: kernels_per_step segments of dep_stride
     int dep_stride = 0;              // 0: the step's passes run as plain, fully ordered launches
     double* geo_buf = nullptr;
@@ -158,61 +160,65 @@ dim3 grid_h(const lsh_ctx* ctx, int par) { return edge_grid_h(ctx->p.nx, ctx->p.
 dim3 grid_v(const lsh_ctx* ctx, int par) { return edge_grid_v(ctx->p.nx, ctx->p.ny, par); }
 
 
-template <int ORDER>
-void enqueue_passes(const lsh_ctx* ctx, const KArgs& a, cudaStream_t s) {
-    k_edges_h<true, ORDER><<<grid_h(ctx, 0), edge_block_h(), 0, s>>>(a, 0);
-    k_edges_h<false, ORDER><<<grid_h(ctx, 1), edge_block_h(), 0, s>>>(a, 1);
-    k_edges_v<ORDER><<<grid_v(ctx, 0), edge_block_v(), 0, s>>>(a, 0);
-    k_edges_v<ORDER><<<grid_v(ctx, 1), edge_block_v(), 0, s>>>(a, 1);
+// The arguments of a step's stages: order 1 in place; order 2 X -> Y, then
+// Y -> X with the average.
+void stage_args(const lsh_ctx* ctx, KArgs& a1, KArgs& a2) {
+    a1 = a2 = base_args(ctx);
+    for (int k = 0; k < 7; ++k) a1.W[k] = a2.W[k] = ctx->X[k];
+    for (int k = 0; k < 6; ++k) {
+        a1.Wout[k] = (ctx->p.order == 1) ? ctx->X[k] : ctx->Y[k];
+        a2.W[k] = ctx->Y[k];
+        a2.Wout[k] = ctx->X[k];
+        a2.Xavg[k] = ctx->X[k];
+    }
+    if (!ctx->edge_mem) return;
+    a1.eb = a2.eb = ctx->flux.eb;
+    a2.eb.stage = 1;
+    for (int l = 0; l < 2; ++l) {
+        if (ctx->p.order == 1) a1.eb.depth[l] = a1.eb.depth_out[l] = ctx->Y[3 * l];
+        else { a1.eb.depth[l] = a1.W[3 * l]; a2.eb.depth[l] = a2.W[3 * l]; }
+    }
 }
 
-// Enqueue one time step; returns the number of kernels launched.
-int enqueue_step(const lsh_ctx* ctx, cudaStream_t s) {
-    const dim3 nbc = cell_grid(ctx->p.nx, ctx->p.ny);
-    if (ctx->dep_ctr) {
-        KArgs a1 = base_args(ctx), a2 = base_args(ctx);
-        for (int k = 0; k < 7; ++k) a1.W[k] = ctx->X[k];
-        if (ctx->p.order == 1) {
-            for (int k = 0; k < 6; ++k) a1.Wout[k] = ctx->X[k];
-        } else {
-            for (int k = 0; k < 6; ++k) a1.Wout[k] = ctx->Y[k];
-            for (int k = 0; k < 6; ++k) a2.W[k] = ctx->Y[k];
-            a2.W[6] = ctx->X[6];
-            for (int k = 0; k < 6; ++k) { a2.Wout[k] = ctx->X[k]; a2.Xavg[k] = ctx->X[k]; }
-        }
-        return enqueue_step_overlap(ctx->p.nx, ctx->p.ny, ctx->p.order, a1, a2, ctx->dep_ctr, ctx->dep_stride, ctx->tm,
-                                    2.0 * ctx->p.cfl, s);
+// Enqueue one time step; returns the number of kernels launched.  `mark` is
+// called after each launch where they run one after the other.
+template <class Mark>
+int enqueue_step(const lsh_ctx* ctx, cudaStream_t s, bool ordered, Mark&& mark) {
+    KArgs a1, a2;
+    stage_args(ctx, a1, a2);
+    const int nx = ctx->p.nx, ny = ctx->p.ny, order = ctx->p.order;
+    const double two_cfl = 2.0 * ctx->p.cfl;
+    if (ctx->edge_mem)
+        return enqueue_flux_step(a1, a2, ctx->flux.map, ordered ? nullptr : ctx->dep_ctr, two_cfl, s, mark);
+    if (ctx->dep_ctr && !ordered)
+        return enqueue_step_overlap(nx, ny, order, a1, a2, ctx->dep_ctr, ctx->dep_stride, ctx->tm, two_cfl, s);
+    const dim3 nbc = cell_grid(nx, ny);
+    auto edges = [&](auto ord, const KArgs& a) {
+        constexpr int O = decltype(ord)::value;
+        k_edges_h<true, O><<<grid_h(ctx, 0), edge_block_h(), 0, s>>>(a, 0); mark();
+        k_edges_h<false, O><<<grid_h(ctx, 1), edge_block_h(), 0, s>>>(a, 1); mark();
+        k_edges_v<O><<<grid_v(ctx, 0), edge_block_v(), 0, s>>>(a, 0); mark();
+        k_edges_v<O><<<grid_v(ctx, 1), edge_block_v(), 0, s>>>(a, 1); mark();
+    };
+    if (order == 1) {
+        edges(std::integral_constant<int, 1>(), a1);
+        k_volume<0><<<nbc, cell_block(), 0, s>>>(a1); mark();
+    } else {
+        k_recon<<<nbc, cell_block(), 0, s>>>(a1); mark();
+        edges(std::integral_constant<int, 2>(), a1);
+        k_volume<1><<<nbc, cell_block(), 0, s>>>(a1); mark();
+        k_recon<<<nbc, cell_block(), 0, s>>>(a2); mark();
+        edges(std::integral_constant<int, 2>(), a2);
+        k_volume<2><<<nbc, cell_block(), 0, s>>>(a2); mark();
     }
-    if (ctx->p.order == 1) {
-        KArgs a = base_args(ctx);
-        for (int k = 0; k < 7; ++k) a.W[k] = ctx->X[k];
-        for (int k = 0; k < 6; ++k) a.Wout[k] = ctx->X[k];
-        enqueue_passes<1>(ctx, a, s);
-        k_volume<0><<<nbc, cell_block(), 0, s>>>(a);
-        k_advance<<<1, 1, 0, s>>>(ctx->tm, 2.0 * ctx->p.cfl);
-        return 6;
-    }
-    KArgs a1 = base_args(ctx);
-    for (int k = 0; k < 7; ++k) a1.W[k] = ctx->X[k];
-    for (int k = 0; k < 6; ++k) a1.Wout[k] = ctx->Y[k];
-    k_recon<<<nbc, cell_block(), 0, s>>>(a1);
-    enqueue_passes<2>(ctx, a1, s);
-    k_volume<1><<<nbc, cell_block(), 0, s>>>(a1);
-    KArgs a2 = base_args(ctx);
-    for (int k = 0; k < 6; ++k) a2.W[k] = ctx->Y[k];
-    a2.W[6] = ctx->X[6];
-    for (int k = 0; k < 6; ++k) { a2.Wout[k] = ctx->X[k]; a2.Xavg[k] = ctx->X[k]; }
-    k_recon<<<nbc, cell_block(), 0, s>>>(a2);
-    enqueue_passes<2>(ctx, a2, s);
-    k_volume<2><<<nbc, cell_block(), 0, s>>>(a2);
-    k_advance<<<1, 1, 0, s>>>(ctx->tm, 2.0 * ctx->p.cfl);
-    return 13;
+    k_advance<<<1, 1, 0, s>>>(ctx->tm, two_cfl); mark();
+    return ctx->kernels_per_step;
 }
 
 int build_graph(lsh_ctx* ctx, int nsteps, cudaGraphExec_t* out) {
     cudaGraph_t graph = nullptr;
     LSH_CUDA(cudaStreamBeginCapture(ctx->own, cudaStreamCaptureModeThreadLocal));
-    for (int i = 0; i < nsteps; ++i) enqueue_step(ctx, ctx->own);
+    for (int i = 0; i < nsteps; ++i) enqueue_step(ctx, ctx->own, false, [] {});
     cudaError_t e = cudaStreamEndCapture(ctx->own, &graph);
     if (e != cudaSuccess) return fail_cuda(e, "cudaStreamEndCapture");
     e = cudaGraphInstantiate(out, graph, 0);
@@ -247,6 +253,10 @@ int upload_state(lsh_ctx* ctx, const double* const src[LSH_NVARS], cudaMemcpyKin
     k_cell_dt<<<nbc, cell_block(), 0, s>>>(a);
     k_init_finish<<<1, 1, 0, s>>>(ctx->tm, 2.0 * ctx->p.cfl);
     ctx->launches += 7;
+    if (ctx->edge_mem) {
+        launch_all_busy(ctx->flux.map, s);
+        ctx->launches += 1;
+    }
     LSH_CUDA(cudaGetLastError());
     LSH_CUDA(cudaMemcpyAsync(ctx->tm_host, ctx->tm, sizeof(TimeRec), cudaMemcpyDeviceToHost, s));
     LSH_CUDA(cudaStreamSynchronize(s));
@@ -345,29 +355,53 @@ int lsh_create(const lsh_params* p, int device, lsh_ctx** out) {
         if (e != cudaSuccess) return bail(fail_cuda(e, "cudaStreamCreate"));
         ctx->stream = ctx->own;
     }
-    // one slab: X(7) + Y(6) + acc(7) + eta(2) [+ sx, sy (14)] arrays of N, geometry, time record
+    // one slab: X(7) + Y(6) + acc + eta(2) [+ sx, sy (14)] arrays of N, geometry, time record
     const size_t n_pad = (ctx->N + 31) & ~size_t(31);  // 256-byte aligned arrays
-    const int n_arrays = 7 + 6 + 7 + 2 + ((p->order == 2) ? 14 : 0);
     const size_t geo_n = size_t(7) * (p->ny + 1);
-    // pass-overlap counters: one per block row of each pass of a step (the
-    // block rows of the edge and cell kernels), when the grids cover every
-    // row in one launch
-    const int dep_stride = dep_stride_for(p->nx, p->ny);
-    const int kps = (p->order == 1) ? 6 : 13;
-    const size_t dep_bytes = size_t(dep_stride) * kps * sizeof(unsigned);
-    const size_t bytes = (size_t(n_arrays) * n_pad + ((geo_n + 31) & ~size_t(31))) * sizeof(double) + 256 +
-                         ((p->order == 2) ? n_pad : 0) +  // + one byte per cell: slopes-are-zero flags
-                         ((dep_bytes + 255) & ~size_t(255));
+    size_t dep_bytes = 0;
+    // The slab of the flux pass and cell update (`flux`: only the wave
+    // accumulator, which the initial-dt pass uses) or of the colour passes,
+    // with the pass-overlap counters: one per tile row (block row) of each
+    // pass of a step, when a launch of rows up to 65535 covers the grid.
+    auto slab_bytes = [&](bool flux) {
+        const int n_arrays = 7 + 6 + (flux ? 1 : 7) + 2 + ((p->order == 2) ? 14 : 0);
+        ctx->kernels_per_step = (p->order == 1) ? 6 : 13;
+        if (flux) ctx->dep_stride = (tiles_y(p->ny) <= 65535) ? flux_dep_stride(p->ny) : 0;
+        else ctx->dep_stride = dep_stride_for(p->nx, p->ny);
+        dep_bytes = size_t(ctx->dep_stride) * ctx->kernels_per_step * sizeof(unsigned);
+        return (size_t(n_arrays) * n_pad + ((geo_n + 31) & ~size_t(31))) * sizeof(double) + 256 +
+               ((p->order == 2) ? n_pad : 0) +  // + one byte per cell: slopes-are-zero flags
+               ((dep_bytes + 255) & ~size_t(255));
+    };
+    // The flux pass and cell update where the parameters allow it and its edge
+    // buffers fit the device beside the rest; the colour passes, which need 0.6
+    // of the memory, where they do not.
+    if (lsh::flux_fits(*p)) {
+        cudaError_t e = cudaMalloc(&ctx->edge_mem, FluxMem{}.layout(nullptr, p->nx, p->ny));
+        if (e == cudaSuccess) e = cudaMalloc(&ctx->slab, slab_bytes(true));
+        if (e != cudaSuccess) {
+            if (ctx->edge_mem) cudaFree(ctx->edge_mem);
+            ctx->edge_mem = ctx->slab = nullptr;
+            if (e != cudaErrorMemoryAllocation) return bail(fail_cuda(e, "cudaMalloc edge buffers"));
+            (void)cudaGetLastError();
+        }
+    }
     {
-        cudaError_t e = cudaMalloc(&ctx->slab, bytes);
+        cudaError_t e = ctx->slab ? cudaSuccess : cudaMalloc(&ctx->slab, slab_bytes(false));
         if (e != cudaSuccess) return bail(fail_cuda(e, "cudaMalloc"));
         e = cudaMallocHost((void**)&ctx->tm_host, sizeof(TimeRec));
         if (e != cudaSuccess) return bail(fail_cuda(e, "cudaMallocHost"));
     }
+    if (ctx->edge_mem) {
+        ctx->flux.layout(static_cast<unsigned char*>(ctx->edge_mem), p->nx, p->ny);
+        cudaError_t e = cudaMemsetAsync(ctx->flux.clear, 0, ctx->flux.clear_bytes, ctx->own);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->own);
+        if (e != cudaSuccess) return bail(fail_cuda(e, "cudaMemset cell marks"));
+    }
     double* cur = static_cast<double*>(ctx->slab);
     for (int k = 0; k < 7; ++k) { ctx->X[k] = cur; cur += n_pad; }
     for (int k = 0; k < 6; ++k) { ctx->Y[k] = cur; cur += n_pad; }
-    for (int k = 0; k < 7; ++k) { ctx->acc[k] = cur; cur += n_pad; }
+    for (int k = ctx->edge_mem ? 6 : 0; k < 7; ++k) { ctx->acc[k] = cur; cur += n_pad; }
     ctx->eta_max = cur; cur += n_pad;
     ctx->eta_time = cur; cur += n_pad;
     if (p->order == 2) {
@@ -386,9 +420,8 @@ int lsh_create(const lsh_params* p, int device, lsh_ctx** out) {
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->own);
         if (e != cudaSuccess) return bail(fail_cuda(e, "cudaMemset slope flags"));
     }
-    if (dep_stride) {
+    if (ctx->dep_stride) {
         ctx->dep_ctr = reinterpret_cast<unsigned*>(tail);
-        ctx->dep_stride = dep_stride;
         cudaError_t e = cudaMemsetAsync(ctx->dep_ctr, 0, dep_bytes, ctx->own);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->own);
         if (e != cudaSuccess) return bail(fail_cuda(e, "cudaMemset pass counters"));
@@ -408,7 +441,6 @@ int lsh_create(const lsh_params* p, int device, lsh_ctx** out) {
     ctx->geo.wx = ctx->geo_buf + 4 * st;
     ctx->geo.wy = ctx->geo_buf + 5 * st;
     ctx->geo.inv_area = ctx->geo_buf + 6 * st;
-    ctx->kernels_per_step = (p->order == 1) ? 6 : 13;
     *out = ctx;
     return LSH_OK;
 }
@@ -419,6 +451,7 @@ int lsh_destroy(lsh_ctx* ctx) {
     if (ctx->g_chunk) cudaGraphExecDestroy(ctx->g_chunk);
     if (ctx->g_one) cudaGraphExecDestroy(ctx->g_one);
     if (ctx->slab) cudaFree(ctx->slab);
+    if (ctx->edge_mem) cudaFree(ctx->edge_mem);
     if (ctx->gauge_cells) cudaFree(ctx->gauge_cells);
     if (ctx->tm_host) cudaFreeHost(ctx->tm_host);
     if (ctx->own) cudaStreamDestroy(ctx->own);
@@ -570,41 +603,10 @@ int lsh_profile_step(lsh_ctx* ctx, float* ms_out, int cap, int* n_kernels) {
     const int nk = ctx->kernels_per_step;
     std::vector<cudaEvent_t> ev(nk + 1);
     for (auto& e : ev) LSH_CUDA(cudaEventCreate(&e));
-    const dim3 nbc = cell_grid(ctx->p.nx, ctx->p.ny);
     int i = 0;
     auto mark = [&]() { cudaEventRecord(ev[i++], s); };
     mark();
-    if (ctx->p.order == 1) {
-        KArgs a = base_args(ctx);
-        for (int k = 0; k < 7; ++k) a.W[k] = ctx->X[k];
-        for (int k = 0; k < 6; ++k) a.Wout[k] = ctx->X[k];
-        k_edges_h<true, 1><<<grid_h(ctx, 0), edge_block_h(), 0, s>>>(a, 0); mark();
-        k_edges_h<false, 1><<<grid_h(ctx, 1), edge_block_h(), 0, s>>>(a, 1); mark();
-        k_edges_v<1><<<grid_v(ctx, 0), edge_block_v(), 0, s>>>(a, 0); mark();
-        k_edges_v<1><<<grid_v(ctx, 1), edge_block_v(), 0, s>>>(a, 1); mark();
-        k_volume<0><<<nbc, cell_block(), 0, s>>>(a); mark();
-    } else {
-        for (int stage = 0; stage < 2; ++stage) {
-            KArgs a = base_args(ctx);
-            if (stage == 0) {
-                for (int k = 0; k < 7; ++k) a.W[k] = ctx->X[k];
-                for (int k = 0; k < 6; ++k) a.Wout[k] = ctx->Y[k];
-            } else {
-                for (int k = 0; k < 6; ++k) a.W[k] = ctx->Y[k];
-                a.W[6] = ctx->X[6];
-                for (int k = 0; k < 6; ++k) { a.Wout[k] = ctx->X[k]; a.Xavg[k] = ctx->X[k]; }
-            }
-            k_recon<<<nbc, cell_block(), 0, s>>>(a); mark();
-            k_edges_h<true, 2><<<grid_h(ctx, 0), edge_block_h(), 0, s>>>(a, 0); mark();
-            k_edges_h<false, 2><<<grid_h(ctx, 1), edge_block_h(), 0, s>>>(a, 1); mark();
-            k_edges_v<2><<<grid_v(ctx, 0), edge_block_v(), 0, s>>>(a, 0); mark();
-            k_edges_v<2><<<grid_v(ctx, 1), edge_block_v(), 0, s>>>(a, 1); mark();
-            if (stage == 0) k_volume<1><<<nbc, cell_block(), 0, s>>>(a);
-            else k_volume<2><<<nbc, cell_block(), 0, s>>>(a);
-            mark();
-        }
-    }
-    k_advance<<<1, 1, 0, s>>>(ctx->tm, 2.0 * ctx->p.cfl); mark();
+    enqueue_step(ctx, s, true, mark);
     ctx->launches += nk;
     int status = LSH_OK;
     cudaError_t e = cudaGetLastError();

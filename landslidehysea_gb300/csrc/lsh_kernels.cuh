@@ -285,10 +285,8 @@ __global__ void LSH_CELL_BOUNDS k_volume(KArgs a, Dep d = Dep{}) {
 
 
 // Advance the device clock: t += dt, dt = min per-cell dt (ShallowWater.cu:436-442).
-// With `ctr`, its threads also zero the n_ctr pass-overlap counters of the step.
-__global__ void k_advance(TimeRec* tm, double two_cfl, unsigned* ctr = nullptr, int n_ctr = 0) {
-    for (int i = threadIdx.x; i < n_ctr; i += blockDim.x) ctr[i] = 0u;
-    if (threadIdx.x != 0 || tm->done) return;
+__device__ __forceinline__ void advance_clock(TimeRec* tm, double two_cfl) {
+    if (tm->done) return;
     tm->t += tm->dt;
     tm->steps += 1;
     const double nd = lsh::dt_of(tm->rmax_bits, two_cfl);
@@ -297,6 +295,13 @@ __global__ void k_advance(TimeRec* tm, double two_cfl, unsigned* ctr = nullptr, 
     if (tm->t >= tm->t_end) tm->done = 1;
     if (tm->dt_min > 0.0 && nd < tm->dt_min) { tm->err |= 1 << LSH_ERR_STALL; tm->done = 1; }
     if (tm->err) tm->done = 1;
+}
+
+// The clock of a step of colour passes.  With `ctr`, its threads also zero the
+// n_ctr pass-overlap counters of the step.
+__global__ void k_advance(TimeRec* tm, double two_cfl, unsigned* ctr = nullptr, int n_ctr = 0) {
+    for (int i = threadIdx.x; i < n_ctr; i += blockDim.x) ctr[i] = 0u;
+    if (threadIdx.x == 0) advance_clock(tm, two_cfl);
 }
 
 // Initial-dt edge pass (procesarAristasDeltaTInicialGPU), writing acc[6]:
@@ -351,6 +356,210 @@ __global__ void __launch_bounds__(kCellBlock) k_init_eta(KArgs a) {
     if (id < 0) return;
     a.eta_max[id] = a.W[0][id] + a.W[3][id] - a.W[6][id];
     a.eta_time[id] = 0.0;
+}
+
+// ---------------------------------------------------------------- flux pass and cell update
+//
+// The single-grid step: per stage the reconstruction (second order), one flux
+// pass over all edges and the cells' update (lsh_passes.cuh), on tiles of 16
+// columns by 4 rows.  A tile is two warps of the cell passes (two rows each)
+// and four of the flux pass (two rows each of its horizontal edges, between its
+// rows and the rows above them, and of its vertical ones); tiles past the last
+// column and row hold the outer edges.  Against the four colour passes and the
+// volume kernel, an edge's faces are loaded once instead of an accumulator pass
+// per colour, and a stage's chain is three passes instead of six.
+//
+// Tiles that nothing can reach in a step are left out: the clock kernel lists,
+// per tile row, the tiles with a busy tile (TileMap::busy) at most two away.
+// A tile is busy when, in the step's last update of either stage, one of its
+// cells' input or output state was not all +0 or one of their edges was not
+// dry.  A stage carries state one tile further at most (an edge's flux, or a
+// limiter, reads two cells), so a tile left out holds +0 in both state buffers
+// before and after the step, its edges' kinds are dry, its slopes are zero and
+// flagged so (the reconstruction ran on it, and its neighbours, empty), and its
+// maximum of eta1 has seen the empty state.  On the 2048^2 fjord, 14% wet, the
+// blocks of dry tiles took 490 of the step's 1295 us; after a new state every
+// tile is busy.
+//
+// The flux pass is launched as four consecutive ranges of its blocks, the four
+// edge launches a step has always had (lsh_profile_step,
+// lsh_get_launch_count); nothing orders them, so a small grid's run side by
+// side and a large one's follow each other as one grid's blocks would.
+// Overlap as above (programmatic dependent launches), by tile rows: a block
+// adds 1 to its tile row's counter, and waits for its producer's listed tiles
+// in the rows around its own: the flux pass for the row itself and the one
+// above (it reads the cells above its first row), the update and the
+// reconstruction for one row on each side (the limiter's recursion reads edges
+// and depths up to two cells away, the stencil one cell).
+constexpr int kTileX = 16, kTileY = 4;
+constexpr int kCellWarps = 2, kFluxWarps = 4, kFluxParts = 4;  // warps per tile, and launches of the flux pass
+#ifndef LSH_FLUX_MINB
+#define LSH_FLUX_MINB 8
+#endif
+#ifndef LSH_UPDATE_MINB
+#define LSH_UPDATE_MINB 20
+#endif
+#ifndef LSH_SLOPES_MINB
+#define LSH_SLOPES_MINB 32
+#endif
+
+inline __host__ __device__ int tiles_x(int nx) { return (nx + 1 + kTileX - 1) / kTileX; }
+inline __host__ __device__ int tiles_y(int ny) { return (ny + 1 + kTileY - 1) / kTileY; }
+
+struct TileMap {
+    int ntx, nty;
+    int* list;               // per tile row: the listed tiles' columns, ascending
+    int* count;              // per tile row: how many
+    // per stage and tile, one byte for each of its warps of the cell passes
+    unsigned short* busy[2];
+};
+
+struct TileDep {
+    const unsigned* wait = nullptr;  // producer's counters per tile row (null: no wait)
+    unsigned* done = nullptr;        // this pass's (null: none)
+    unsigned per = 0;                // producer blocks per listed tile
+};
+
+// The tile of unit `u` (warp number of a pass with `warps` per tile, first
+// warp of the block): false when its row lists fewer.
+__device__ __forceinline__ bool tile_of(const TileMap& m, unsigned u, int warps, int& tx, int& ty) {
+    const unsigned t = u / (unsigned)warps;
+    ty = (int)(t / (unsigned)m.ntx);
+    const int k = (int)(t - (unsigned)ty * (unsigned)m.ntx);
+    if (ty >= m.nty || k >= m.count[ty]) return false;
+    tx = m.list[(size_t)ty * m.ntx + k];
+    return true;
+}
+
+// Start of a block on tile row t: lets the next pass be scheduled, then waits
+// for the producer's blocks on tile rows [t - 1, t + after] (one thread per
+// row; bounded as dep_begin).
+__device__ __forceinline__ void tile_begin(const TileDep& d, const TileMap& m, TimeRec* tm, int t, int after) {
+    if (d.done) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!d.wait) return;
+    const int r = max(t - 1, 0) + (int)threadIdx.x;
+    if (r <= min(t + after, m.nty - 1)) {
+        const unsigned target = d.per * (unsigned)m.count[r];
+        const int tbit = 1 << LSH_ERR_TIMEOUT;
+        volatile int* err = &tm->err;
+        unsigned long long start = 0;
+        unsigned ns = 32;
+        for (;;) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(d.wait + r) : "memory");
+            if (v >= target) break;
+            if (*err & tbit) break;
+            unsigned long long now;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+            if (start == 0) start = now;
+            else if (now - start > 2000000000ull) { atomicOr(&tm->err, tbit); break; }
+            __nanosleep(ns);
+            if (ns < 256) ns *= 2;
+        }
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ void tile_end(const TileDep& d, int t) {
+    if (!d.done) return;
+    __syncthreads();
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(d.done + t) : "memory");
+}
+
+// The warp's largest rate into *target, which only grows: most warps find it
+// larger already and leave it.
+__device__ __forceinline__ void warp_max_bits(unsigned long long v, unsigned long long* target) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long w = __shfl_down_sync(0xffffffffu, v, o);
+        v = (w > v) ? w : v;
+    }
+    if ((threadIdx.x & 31) == 0 && v > *(volatile unsigned long long*)target) atomicMax(target, v);
+}
+
+// Blocks first, first + 1, ... of the flux pass: one to four warps of a tile each.
+template <int ORDER>
+__global__ void __launch_bounds__(32 * kFluxWarps, LSH_FLUX_MINB)
+    k_flux(const __grid_constant__ KArgs a, const __grid_constant__ TileMap m, TileDep d, unsigned first) {
+    if (a.tm->done) return;
+    const unsigned bw = blockDim.x / 32, u0 = (first + blockIdx.x) * bw;
+    int tx, ty;
+    if (!tile_of(m, u0, kFluxWarps, tx, ty)) return;
+    tile_begin(d, m, a.tm, ty, 0);
+    const int nx = a.c.nx, ny = a.c.ny;
+    const int q = (int)((u0 + threadIdx.x / 32) % kFluxWarps), lane = threadIdx.x & 31;
+    const int x = tx * kTileX + (lane & (kTileX - 1)), y = ty * kTileY + (q & 1) * 2 + lane / kTileX;
+    const double dt = a.tm->dt;
+    if (q & 2) { if (x <= nx && y < ny) lsh::flux_edge<1, ORDER>(a, x, y, dt); }
+    else { if (x < nx && y <= ny) lsh::flux_edge<0, ORDER>(a, x, y, dt); }
+    tile_end(d, ty);
+}
+
+// The cell of a thread of the cell passes, or false.
+__device__ __forceinline__ bool tile_cell(const KArgs& a, int tx, int ty, unsigned u0, int& half, int& i, int& j) {
+    const int lane = threadIdx.x & 31;
+    half = (int)((u0 + threadIdx.x / 32) % kCellWarps);
+    i = tx * kTileX + (lane & (kTileX - 1));
+    j = ty * kTileY + 2 * half + lane / kTileX;
+    return i < a.c.nx && j < a.c.ny;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(32 * kCellWarps, LSH_UPDATE_MINB)
+    k_update(const __grid_constant__ KArgs a, const __grid_constant__ TileMap m, TileDep d) {
+    if (a.tm->done) return;
+    const unsigned u0 = blockIdx.x * (blockDim.x / 32);
+    int tx, ty, half, i, j;
+    if (!tile_of(m, u0, kCellWarps, tx, ty)) return;
+    tile_begin(d, m, a.tm, ty, 1);
+    const bool in = tile_cell(a, tx, ty, u0, half, i, j);
+    unsigned long long bits = kRateInitBits;
+    bool busy = false;
+    if (in) bits = lsh::update_cell<MODE>(a, i, j, a.tm->dt, busy);
+    __syncwarp();
+    busy = __any_sync(0xffffffffu, busy);
+    if ((threadIdx.x & 31) == 0)
+        reinterpret_cast<unsigned char*>(m.busy[MODE == 1 ? 1 : 0] + (size_t)ty * m.ntx + tx)[half] = busy;
+    if (MODE != 2) warp_max_bits(bits, &a.tm->rmax_bits);
+    tile_end(d, ty);
+}
+
+__global__ void __launch_bounds__(32 * kCellWarps, LSH_SLOPES_MINB)
+    k_slopes(const __grid_constant__ KArgs a, const __grid_constant__ TileMap m, TileDep d) {
+    if (a.tm->done) return;
+    const unsigned u0 = blockIdx.x * (blockDim.x / 32);
+    int tx, ty, half, i, j;
+    if (!tile_of(m, u0, kCellWarps, tx, ty)) return;
+    tile_begin(d, m, a.tm, ty, 1);
+    if (tile_cell(a, tx, ty, u0, half, i, j)) lsh::recon_cell(a, j * a.c.nx + i);
+    tile_end(d, ty);
+}
+
+// The clock of a step of the flux pass and cell update: t and dt advance
+// (k_advance), the n_ctr pass counters go back to zero, and the next step's
+// tiles are listed, one warp per tile row.  `tm` null: the list alone.
+__global__ void __launch_bounds__(256) k_clock(TimeRec* tm, double two_cfl, unsigned* ctr, int n_ctr, TileMap m) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_ctr; i += gridDim.x * blockDim.x) ctr[i] = 0u;
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x / 32);
+    for (int r = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; r < m.nty; r += warps) {
+        int n = 0;
+        for (int c0 = 0; c0 < m.ntx; c0 += 32) {
+            const int c = c0 + lane;
+            unsigned v = 0;
+            if (c < m.ntx) {
+                for (int y = max(r - 2, 0); y <= min(r + 2, m.nty - 1); ++y)
+                    for (int x = max(c - 2, 0); x <= min(c + 2, m.ntx - 1); ++x) {
+                        const size_t t = (size_t)y * m.ntx + x;
+                        v |= m.busy[0][t] | m.busy[1][t];
+                    }
+            }
+            const unsigned on = __ballot_sync(0xffffffffu, v != 0);
+            if (v) m.list[(size_t)r * m.ntx + n + __popc(on & ((1u << lane) - 1u))] = c;
+            n += __popc(on);
+        }
+        if (lane == 0) m.count[r] = n;
+    }
+    if (tm && blockIdx.x == 0 && threadIdx.x == 0) advance_clock(tm, two_cfl);
 }
 
 // ---------------------------------------------------------------- overlapped launches
@@ -453,6 +662,106 @@ inline int enqueue_step_overlap(int nx, int ny, int order, const KArgs& a1, cons
     // a plain launch: waits for the whole step, then zeroes the counters
     k_advance<<<1, 256, 0, s>>>(tm, two_cfl, c, nk * st);
     return nk;
+}
+
+// What the flux pass and cell update hold beside the state: edge planes and
+// kinds, the cells' marks, the tile lists.  layout() places it in `mem` (256-byte
+// aligned; null: the size alone) and returns the bytes; marks and busy flags lie
+// next to each other in [clear, clear + clear_bytes).
+struct FluxMem {
+    lsh::EdgeBuf eb{};
+    TileMap map{};
+    unsigned char* clear = nullptr;
+    size_t clear_bytes = 0;
+    size_t layout(unsigned char* mem, int nx, int ny) {
+        const size_t N = size_t(nx) * ny, tiles = size_t(tiles_x(nx)) * tiles_y(ny);
+        size_t at = 0;
+        auto take = [&](size_t bytes) { unsigned char* q = mem + at; at += (bytes + 255) & ~size_t(255); return q; };
+        const size_t n[2] = {(N + nx + 31) & ~size_t(31), (N + ny + 31) & ~size_t(31)};
+        for (int d = 0; d < 2; ++d) {
+            eb.plane[d] = n[d];
+            eb.q[d] = reinterpret_cast<double*>(take(lsh::kEdgePlanes * n[d] * sizeof(double)));
+            eb.kind[d] = take(n[d]);
+        }
+        map.ntx = tiles_x(nx);
+        map.nty = tiles_y(ny);
+        map.list = reinterpret_cast<int*>(take(tiles * sizeof(int)));
+        map.count = reinterpret_cast<int*>(take(map.nty * sizeof(int)));
+        clear = mem + at;
+        for (int l = 0; l < 2; ++l) eb.mark[l] = reinterpret_cast<unsigned*>(take(N * sizeof(unsigned)));
+        for (int l = 0; l < 2; ++l) map.busy[l] = reinterpret_cast<unsigned short*>(take(tiles * sizeof(unsigned short)));
+        clear_bytes = size_t(mem + at - clear);
+        return at;
+    }
+};
+
+inline unsigned clock_blocks(const TileMap& m) { return (unsigned)std::min((m.nty + 7) / 8, 1024); }
+
+// A new state: every tile is busy (any byte but 0 says so).  Marks of an old
+// run cost an evaluation at most.
+inline void launch_all_busy(const TileMap& m, cudaStream_t s) {
+    for (int l = 0; l < 2; ++l)
+        (void)cudaMemsetAsync(m.busy[l], 1, size_t(m.ntx) * m.nty * sizeof(unsigned short), s);
+    k_clock<<<clock_blocks(m), 256, 0, s>>>(nullptr, 0.0, nullptr, 0, m);
+}
+
+// Passes of a step before the clock, and the counters of each: one per tile
+// row, rounded up.
+inline int flux_step_passes(int order) { return (order == 1) ? 2 : 6; }
+inline int flux_dep_stride(int ny) { return (tiles_y(ny) + 63) & ~63; }
+
+// One time step: a1 the stage 1 arguments (order 1: in place), a2 stage 2's
+// (with their edge buffers).  `c` (may be null: full-grid launches one after
+// the other): flux_dep_stride counters for each pass, which the clock kernel
+// zeroes.  `mark` is called after each launch.  Returns the kernels launched.
+// A grid of few tiles takes blocks of one warp, so that every SM's FP64 unit
+// has work; a large one a tile per block.
+template <class Mark>
+inline int enqueue_flux_step(const KArgs& a1, const KArgs& a2, const TileMap& m, unsigned* c, double two_cfl,
+                             cudaStream_t s, Mark&& mark) {
+    const int order = a1.c.order, st = flux_dep_stride(a1.c.ny), last = flux_step_passes(order) - 1;
+    const unsigned tiles = unsigned(m.ntx) * unsigned(m.nty);
+    const bool spread = tiles <= 2048;
+    const unsigned cw = spread ? 1 : kCellWarps, fw = spread ? 1 : kFluxWarps;  // warps per block
+    const unsigned nf = tiles * (kFluxWarps / fw), nc = tiles * (kCellWarps / cw);
+    TileDep d;  // the pass before as producer, this pass's own counters
+    int pass = 0;
+    auto begin = [&] { if (c) d.done = (pass < last) ? c + pass * st : nullptr; };
+    auto end = [&](unsigned per) {
+        if (c) { d.wait = d.done; d.per = per; }
+        ++pass;
+    };
+    auto cells = [&](auto kernel, const KArgs& a) {
+        begin();
+        launch_pass(d.wait != nullptr, dim3(nc), dim3(32 * cw), s, kernel, a, m, d);
+        mark();
+        end(kCellWarps / cw);
+    };
+    auto flux = [&](auto kernel, const KArgs& a) {
+        begin();
+        for (int q = 0; q < kFluxParts; ++q) {
+            const unsigned b0 = unsigned((unsigned long long)nf * q / kFluxParts);
+            const unsigned b1 = unsigned((unsigned long long)nf * (q + 1) / kFluxParts);
+            launch_pass(c && (q > 0 || d.wait), dim3(b1 - b0), dim3(32 * fw), s, kernel, a, m, d, b0);
+            mark();
+        }
+        end(kFluxWarps / fw);
+    };
+    if (order == 1) {
+        flux(k_flux<1>, a1);
+        cells(k_update<0>, a1);
+    } else {
+        cells(k_slopes, a1);
+        flux(k_flux<2>, a1);
+        cells(k_update<1>, a1);
+        cells(k_slopes, a2);
+        flux(k_flux<2>, a2);
+        cells(k_update<2>, a2);
+    }
+    // a plain launch: waits for the whole step, then zeroes the counters
+    k_clock<<<clock_blocks(m), 256, 0, s>>>(a1.tm, two_cfl, c, c ? pass * st : 0, m);
+    mark();
+    return (order == 1) ? 6 : 13;
 }
 
 }  // namespace

@@ -44,6 +44,26 @@ LSH_HD bool warp_any(bool p) {
 #endif
 }
 
+// Per-edge results of a stage's flux pass (flux_edge), read by its cells'
+// update (update_cell).  Horizontal edge row y, column x: index y nx + x;
+// vertical edge column x, row y: y (nx + 1) + x.  Eleven planes each: m[0..2],
+// p[0..1], wave, and with a granular layer m[3..5], p[2..3] (EdgeRaw).
+constexpr int kEdgePlanes = 11;
+enum EdgeKind : unsigned char { kEdgeDry = 0, kEdgeSingle = 1, kEdgeBoth = 2 };
+struct EdgeBuf {
+    double* q[2];             // horizontal, vertical
+    size_t plane[2];          // doubles between planes
+    unsigned char* kind[2];   // EdgeKind of each edge
+    // per cell and layer: the stage number (2 steps + stage, 32 bits) in which
+    // one of its edges may empty the layer, so that the limiter has to be
+    // evaluated around it; an old number that comes round again costs that
+    // evaluation only
+    unsigned* mark[2];
+    unsigned stage;           // 0 or 1, the stage of the step
+    const double* depth[2];   // the cells' depths h1, h2 as the limiter reads them
+    double* depth_out[2];     // where the flux pass leaves them (null: they stay in W)
+};
+
 struct KArgs {
     Consts c;
     Geo geo;
@@ -65,6 +85,7 @@ struct KArgs {
     // reads, which the reverse sweep needs at exactly those cells
     double* snap[2];
     unsigned* tape;       // the recomputation's reconstruction branch tape (kOpReconTape; null otherwise)
+    EdgeBuf eb;           // the flux pass's results (q[0] null: the colour passes run instead)
 };
 
 // Depths of a face (first order: the cell's; second order: reconstructed).
@@ -119,12 +140,12 @@ LSH_HD void scatter_edge(const KArgs& a, int id0, int id1, bool interior, const 
                          double wave) {
     if (FIRST) {
 #pragma unroll
-        for (int k = 0; k < 6; ++k) a.acc[k][id0] = (k < KL) ? 0.0 - d0[k] : 0.0;
-        a.acc[6][id0] = 0.0 + wave;
+        for (int k = 0; k < 6; ++k) a.acc[k][id0] = (k < KL) ? lsh::minus0(d0[k]) : 0.0;
+        a.acc[6][id0] = lsh::plus0(wave);
         if (interior) {
 #pragma unroll
-            for (int k = 0; k < 6; ++k) a.acc[k][id1] = (k < KL) ? 0.0 - d1[k] : 0.0;
-            a.acc[6][id1] = 0.0 + wave;
+            for (int k = 0; k < 6; ++k) a.acc[k][id1] = (k < KL) ? lsh::minus0(d1[k]) : 0.0;
+            a.acc[6][id1] = lsh::plus0(wave);
         }
     } else {
 #pragma unroll
@@ -158,56 +179,80 @@ struct LazyPos {
     }
 };
 
-// One edge: gather both sides, evaluate, scatter to the accumulators.
+// The sides of one edge.
 // dir 0: horizontal edge row y between rows y-1 and y, column x.
 // dir 1: vertical edge column x between columns x-1 and x, row y.
-template <int DIR, bool FIRST, int ORDER>
-LSH_HD void do_edge(const KArgs& a, int x, int y, double dt) {
+struct EdgeSides { int id0, id1, side0, row0, row1; bool interior, pos_normal; double bor, len; };
+template <int DIR>
+LSH_HD EdgeSides edge_sides(const KArgs& a, int x, int y) {
     const int nx = a.c.nx, ny = a.c.ny;
-    lsh::EdgeIn e;
-    int id0, id1 = -1, side0, row0, row1 = 0;
-    double bor = 0.0;
-    bool pos_normal = true;
+    EdgeSides s;
+    s.id1 = -1; s.row1 = 0; s.bor = 0.0; s.pos_normal = true;
     if (DIR == 0) {
-        e.len = a.geo.len_h[y];
-        if (y == 0) { id0 = x; row0 = 0; pos_normal = false; bor = a.c.borde_sup; side0 = 2; }
-        else if (y == ny) { id0 = (ny - 1) * nx + x; row0 = ny - 1; bor = a.c.borde_inf; side0 = 3; }
-        else { id0 = (y - 1) * nx + x; id1 = id0 + nx; row0 = y - 1; row1 = y; side0 = 3; }
+        s.len = a.geo.len_h[y];
+        if (y == 0) { s.id0 = x; s.row0 = 0; s.pos_normal = false; s.bor = a.c.borde_sup; s.side0 = 2; }
+        else if (y == ny) { s.id0 = (ny - 1) * nx + x; s.row0 = ny - 1; s.bor = a.c.borde_inf; s.side0 = 3; }
+        else { s.id0 = (y - 1) * nx + x; s.id1 = s.id0 + nx; s.row0 = y - 1; s.row1 = y; s.side0 = 3; }
     } else {
-        e.len = a.geo.len_v[y];
-        row0 = row1 = y;
-        if (x == 0) { id0 = y * nx; pos_normal = false; bor = a.c.borde_izq; side0 = 0; }
-        else if (x == nx) { id0 = y * nx + nx - 1; bor = a.c.borde_der; side0 = 1; }
-        else { id0 = y * nx + x - 1; id1 = id0 + 1; side0 = 1; }
+        s.len = a.geo.len_v[y];
+        s.row0 = s.row1 = y;
+        if (x == 0) { s.id0 = y * nx; s.pos_normal = false; s.bor = a.c.borde_izq; s.side0 = 0; }
+        else if (x == nx) { s.id0 = y * nx + nx - 1; s.bor = a.c.borde_der; s.side0 = 1; }
+        else { s.id0 = y * nx + x - 1; s.id1 = s.id0 + 1; s.side0 = 1; }
     }
-    e.interior = (id1 >= 0);
+    s.interior = (s.id1 >= 0);
+    return s;
+}
+
+// The face depths of an edge; false for a dry edge, which adds nothing.
+template <int DIR, int ORDER>
+LSH_HD bool edge_wet(const KArgs& a, const EdgeSides& s, Face& A, Face& B) {
+    using lsh::is_zero;
     const int side1 = (DIR == 0) ? 2 : 0;
     // Both cells empty (h1 = h2 = 0) with zero stored slopes (second order:
     // the slope-zero flags): every face depth is exactly 0, so the dry test
     // below would find the edge dry.  Integer tests only, and no slope loads:
     // most edges of a flooded-coast grid are such edges.
     if (ORDER == 1 || a.szero) {
-        using lsh::is_zero;
-        bool empty = is_zero(a.W[0][id0]) && is_zero(a.W[3][id0]) && (ORDER == 1 || a.szero[id0]);
-        if (empty && e.interior) empty = is_zero(a.W[0][id1]) && is_zero(a.W[3][id1]) && (ORDER == 1 || a.szero[id1]);
-        if (empty) {
-            if (FIRST) {
-#pragma unroll
-                for (int k = 0; k < 7; ++k) a.acc[k][id0] = 0.0;
-                if (e.interior) {
-#pragma unroll
-                    for (int k = 0; k < 7; ++k) a.acc[k][id1] = 0.0;
-                }
-            }
-            return;
-        }
+        bool empty = is_zero(a.W[0][s.id0]) && is_zero(a.W[3][s.id0]) && (ORDER == 1 || a.szero[s.id0]);
+        if (empty && s.interior)
+            empty = is_zero(a.W[0][s.id1]) && is_zero(a.W[3][s.id1]) && (ORDER == 1 || a.szero[s.id1]);
+        if (empty) return false;
     }
-    face_depths<ORDER>(a, id0, side0, e.A.h1, e.A.h2);
-    if (e.interior) face_depths<ORDER>(a, id1, side1, e.B.h1, e.B.h2);
-    else { e.B.h1 = e.A.h1; e.B.h2 = e.A.h2; }
-    // dry edge (Arista_kernel.cu:397): nothing to add; the first pass still
-    // writes the zeros that initialise the accumulators
-    if (lshm::lt_pos(0.5 * (e.A.h1 + e.B.h1), lsh::kEps) && lshm::lt_pos(0.5 * (e.A.h2 + e.B.h2), lsh::kEps)) {
+    face_depths<ORDER>(a, s.id0, s.side0, A.h1, A.h2);
+    if (s.interior) face_depths<ORDER>(a, s.id1, side1, B.h1, B.h2);
+    else { B.h1 = A.h1; B.h2 = A.h2; }
+    // dry edge (Arista_kernel.cu:397)
+    return !(lshm::lt_pos(lsh::half(A.h1 + B.h1), lsh::kEps) && lshm::lt_pos(lsh::half(A.h2 + B.h2), lsh::kEps));
+}
+
+// The rest of a wet edge's faces (the ghost's at a boundary).
+template <int DIR, int ORDER>
+LSH_HD void edge_faces(const KArgs& a, const EdgeSides& s, Face& A, Face& B) {
+    face_rest<DIR, ORDER>(a, s.id0, s.side0, s.pos_normal, A);
+    if (s.interior) {
+        face_rest<DIR, ORDER>(a, s.id1, (DIR == 0) ? 2 : 0, s.pos_normal, B);
+    } else {
+        // ghost: the cell's face with the normal discharges times the boundary factor
+        B = A;
+        B.qn1 = A.qn1 * s.bor;
+        B.qn2 = A.qn2 * s.bor;
+    }
+}
+
+// One edge of a colour pass: gather both sides, evaluate, scatter to the
+// accumulators.
+template <int DIR, bool FIRST, int ORDER>
+LSH_HD void do_edge(const KArgs& a, int x, int y, double dt) {
+    const EdgeSides s = edge_sides<DIR>(a, x, y);
+    const int id0 = s.id0, id1 = s.id1, row0 = s.row0, row1 = s.row1;
+    const bool pos_normal = s.pos_normal;
+    lsh::EdgeIn e;
+    e.len = s.len;
+    e.interior = s.interior;
+    if (!edge_wet<DIR, ORDER>(a, s, e.A, e.B)) {
+        // nothing to add; the first pass still writes the zeros that
+        // initialise the accumulators
         if (FIRST) {
 #pragma unroll
             for (int k = 0; k < 7; ++k) a.acc[k][id0] = 0.0;
@@ -226,15 +271,7 @@ LSH_HD void do_edge(const KArgs& a, int x, int y, double dt) {
             a.snap[1][id1] = a.acc[3][id1];
         }
     }
-    face_rest<DIR, ORDER>(a, id0, side0, pos_normal, e.A);
-    if (e.interior) {
-        face_rest<DIR, ORDER>(a, id1, side1, pos_normal, e.B);
-    } else {
-        // ghost: the cell's face with the normal discharges times the boundary factor
-        e.B = e.A;
-        e.B.qn1 = e.A.qn1 * bor;
-        e.B.qn2 = e.A.qn2 * bor;
-    }
+    edge_faces<DIR, ORDER>(a, s, e.A, e.B);
     // the limiter's inputs are loaded where it reads them (LazyPos), not kept
     // live through the flux computation
     const LazyPos<FIRST> pos{a, id0, id1, row0, row1};
@@ -330,11 +367,11 @@ LSH_HD void recon_cell_from(const KArgs& a, int id, int i, int j, const Acc& w) 
     const bool inx = (i > 0 && i < nx - 1), iny = (j > 0 && j < ny - 1);
     auto slope_x = [&](int k) {
         const double pc = rv(k, 0, 0);
-        return inx ? 0.5 * minmod(pc - rv(k, -1, 0), rv(k, 1, 0) - pc) : 0.0;
+        return inx ? lsh::half(minmod(pc - rv(k, -1, 0), rv(k, 1, 0) - pc)) : 0.0;
     };
     auto slope_y = [&](int k) {
         const double pc = rv(k, 0, 0);
-        return iny ? 0.5 * minmod(pc - rv(k, 0, -1), rv(k, 0, 1) - pc) : 0.0;
+        return iny ? lsh::half(minmod(pc - rv(k, 0, -1), rv(k, 0, 1) - pc)) : 0.0;
     };
     // No granular layer anywhere in the stencil (h2 = q2 = 0 at the cell and
     // the neighbours it reads): eta2 = 0 - H, whose differences are exactly
@@ -426,19 +463,15 @@ __device__ __forceinline__ void block_max_bits(unsigned long long v, unsigned lo
 }
 #endif
 
-// One cell of the Euler-stage update (k_volume); returns the bits of the
-// cell's acc_w / area for the dt reduction.
+// One cell of the Euler-stage update given its state wo and accumulators acc
+// (changed); returns the bits of the cell's acc_w / area for the dt reduction.
 // MODE 0: order 1, in place.  MODE 1: order 2 stage 1 (W -> Wout).
 // MODE 2: order 2 stage 2, Wout = (Xavg + E(W)) / 2.
+// `busy` (may be null): set where the input or the output state is not all +0.
 template <int MODE>
-LSH_HD unsigned long long volume_cell(const KArgs& a, int id, double dt) {
-    const int nx = a.c.nx;
-    const int j = id / nx;
-    double wo[6], acc[7], w[6], rate;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) wo[k] = a.W[k][id];
-#pragma unroll
-    for (int k = 0; k < 7; ++k) acc[k] = a.acc[k][id];
+LSH_HD unsigned long long volume_finish(const KArgs& a, int id, int j, double dt, const double wo[6], double acc[7],
+                                        bool* busy = nullptr) {
+    double w[6], rate;
     if (MODE != 2 && a.c.track_eta) {
         // actualizarEta1MaximaGPU (Volumen_kernel.cu:182-213): state before the step
         const double v = wo[0] - a.W[6][id];
@@ -466,6 +499,8 @@ LSH_HD unsigned long long volume_cell(const KArgs& a, int id, double dt) {
         using lsh::is_zero;
         bool one = is_zero(wo[3]) && is_zero(wo[4]) && is_zero(wo[5]) && lshm::bits_of(acc[3]) == 0 &&
                    lshm::bits_of(acc[4]) == 0 && lshm::bits_of(acc[5]) == 0;
+        // times peso, whose usual value is 1
+        auto times_peso = [&](double v) { return (lshm::bits_of(a.c.peso) != lshm::bits_of(1.0)) ? a.c.peso * v : v; };
         double s0x = 0.0, s3x = 0.0, s0y = 0.0, s3y = 0.0;
         if (a.c.order == 2) {
             s0x = a.sx[0][id]; s3x = a.sx[3][id]; s0y = a.sy[0][id]; s3y = a.sy[3][id];
@@ -475,21 +510,21 @@ LSH_HD unsigned long long volume_cell(const KArgs& a, int id, double dt) {
             if (a.c.order == 2) {
                 const double gh1 = a.c.g * wo[0];
                 const double wx = a.geo.wx[j], wy = a.geo.wy[j];
-                acc[1] -= a.c.peso * ((gh1 * (2.0 * s0x)) * wx);
-                acc[2] -= a.c.peso * ((gh1 * (2.0 * s0y)) * wy);
+                acc[1] -= times_peso((gh1 * lsh::twice(s0x)) * wx);
+                acc[2] -= times_peso((gh1 * lsh::twice(s0y)) * wy);
             }
             lsh::volume_update<true>(wo, acc, w, rate, a.geo.inv_area[j], a.geo.tanR[j], dt, a.c);
         } else {
             if (a.c.order == 2) {
                 // cell-midpoint integral of g h d(eta) over the reconstructed cell
                 const double gh1 = a.c.g * wo[0], gh2 = a.c.g * wo[3];
-                const double e1x = 2.0 * s0x, e2x = 2.0 * s3x;
-                const double e1y = 2.0 * s0y, e2y = 2.0 * s3y;
+                const double e1x = lsh::twice(s0x), e2x = lsh::twice(s3x);
+                const double e1y = lsh::twice(s0y), e2y = lsh::twice(s3y);
                 const double wx = a.geo.wx[j], wy = a.geo.wy[j];
-                acc[1] -= a.c.peso * ((gh1 * e1x) * wx);
-                acc[4] -= a.c.peso * ((gh2 * lsh::fmad(a.c.omr, e2x, a.c.r * e1x)) * wx);
-                acc[2] -= a.c.peso * ((gh1 * e1y) * wy);
-                acc[5] -= a.c.peso * ((gh2 * lsh::fmad(a.c.omr, e2y, a.c.r * e1y)) * wy);
+                acc[1] -= times_peso((gh1 * e1x) * wx);
+                acc[4] -= times_peso((gh2 * lsh::fmad(a.c.omr, e2x, a.c.r * e1x)) * wx);
+                acc[2] -= times_peso((gh1 * e1y) * wy);
+                acc[5] -= times_peso((gh2 * lsh::fmad(a.c.omr, e2y, a.c.r * e1y)) * wy);
             }
             lsh::volume_update(wo, acc, w, rate, a.geo.inv_area[j], a.geo.tanR[j], dt, a.c);
         }
@@ -524,8 +559,14 @@ LSH_HD unsigned long long volume_cell(const KArgs& a, int id, double dt) {
             for (int k = 0; k < 6; ++k) w[k] = lshm::from_bits(lshm::bits_of(x[k]) & lshm::bits_of(w[k]));
         } else {
 #pragma unroll
-            for (int k = 0; k < 6; ++k) w[k] = 0.5 * (x[k] + w[k]);
+            for (int k = 0; k < 6; ++k) w[k] = lsh::half(x[k] + w[k]);
         }
+    }
+    if (busy) {
+        uint64_t u = 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) u |= lshm::bits_of(wo[k]) | lshm::bits_of(w[k]);
+        *busy |= (u != 0);
     }
     if (keep) return (unsigned long long)lshm::bits_of(rate);
     bool bad = false;
@@ -533,6 +574,228 @@ LSH_HD unsigned long long volume_cell(const KArgs& a, int id, double dt) {
     for (int k = 0; k < 6; ++k) { a.Wout[k][id] = w[k]; bad |= lsh::is_bad(w[k]); }
     if (bad) err_or(&a.tm->err, 1 << LSH_ERR_NUMERIC);
     return (unsigned long long)lshm::bits_of(rate);
+}
+
+// One cell of the Euler-stage update after the colour passes.
+template <int MODE>
+LSH_HD unsigned long long volume_cell(const KArgs& a, int id, double dt) {
+    double wo[6], acc[7];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) wo[k] = a.W[k][id];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) acc[k] = a.acc[k][id];
+    return volume_finish<MODE>(a, id, id / a.c.nx, dt, wo, acc);
+}
+
+// ---------------------------------------------------------------- flux pass and cell update
+//
+// An edge's flux needs nothing that another edge computes: only the
+// positivity limiter reads the partial sums of the edges before it in the
+// reference's colour order (even rows, odd rows, even columns, odd columns;
+// ShallowWater.cu:391-427).  So one pass evaluates every edge at once, without
+// the limiter (flux_edge), and the cells' update (update_cell) sums each cell's
+// four edges in colour order, which gives the colour passes' bits.  Where the
+// limiter cannot act (far_from_empty on every side of the edge's two cells) the
+// sums are all there is; around a marked cell the limiter's factors are
+// evaluated as the colour passes would, edge by edge (partial_mass).
+//
+// That an unmarked cell is never limited needs its partial sums not to fall
+// below what its own edges take, so the limiter's factors must not be
+// negative: a limited edge takes at most peso / beta of a cell's content, and
+// flux_fits asks for peso = 1 and beta >= 1 (the reference's values, both 1).
+// The colour passes take the other parameters.
+
+inline bool flux_fits(const lsh_params& p) { return p.peso == 1.0 && p.beta >= 1.0; }
+
+LSH_HD unsigned stage_mark(const KArgs& a) { return 2u * (unsigned)a.tm->steps + a.eb.stage + 1u; }
+
+// One edge of the flux pass.
+template <int DIR, int ORDER>
+LSH_HD void flux_edge(const KArgs& a, int x, int y, double dt) {
+    const EdgeSides s = edge_sides<DIR>(a, x, y);
+    const size_t e = (size_t)y * (a.c.nx + DIR) + x, np = a.eb.plane[DIR];
+    double* const q = a.eb.q[DIR];
+    if (DIR == 0 && a.eb.depth_out[0] && y < a.c.ny) {
+        // order 1 updates in place: the limiter reads this copy, since a
+        // neighbour may already hold its new depth
+        const int id = y * a.c.nx + x;
+        a.eb.depth_out[0][id] = a.W[0][id];
+        a.eb.depth_out[1][id] = a.W[3][id];
+    }
+    Face A, B;
+    if (!edge_wet<DIR, ORDER>(a, s, A, B)) {
+        a.eb.kind[DIR][e] = kEdgeDry;
+        return;
+    }
+    edge_faces<DIR, ORDER>(a, s, A, B);
+    const bool single = is_zero(A.h2) && is_zero(B.h2) && is_zero(A.qn2) && is_zero(B.qn2);
+    EdgeRaw r;
+    if (single) edge_raw<false>(A, B, s.len, dt, a.c, r);
+    else edge_raw<true>(A, B, s.len, dt, a.c, r);
+    a.eb.kind[DIR][e] = single ? kEdgeSingle : kEdgeBoth;
+    q[e] = r.m[0]; q[e + np] = r.m[1]; q[e + 2 * np] = r.m[2];
+    q[e + 3 * np] = r.p[0]; q[e + 4 * np] = r.p[1]; q[e + 5 * np] = r.wave;
+    if (!single) {
+        q[e + 6 * np] = r.m[3]; q[e + 7 * np] = r.m[4]; q[e + 8 * np] = r.m[5];
+        q[e + 9 * np] = r.p[2]; q[e + 10 * np] = r.p[3];
+    }
+    const double scale = tmax(1.0, tmax(a.c.beta, a.c.peso));
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+        if (l == 1 && single) break;
+        const double m = l ? r.m[3] : r.m[0], p = l ? r.p[2] : r.p[0];
+        if (gt0(m) && !far_from_empty(m, a.W[3 * l][s.id0], a.geo.area[s.row0], dt, scale))
+            a.eb.mark[l][s.id0] = stage_mark(a);
+        if (s.interior && gt0(p) && !far_from_empty(p, a.W[3 * l][s.id1], a.geo.area[s.row1], dt, scale))
+            a.eb.mark[l][s.id1] = stage_mark(a);
+    }
+}
+
+#if defined(__CUDACC__)
+#define LSH_RECURSE static __host__ __device__ __noinline__
+#else
+#define LSH_RECURSE static
+#endif
+
+// The colour-C edge of cell (i, j): its direction, place, and whether the cell
+// is its second one.
+struct CellEdge { int x, y; bool second, boundary; };
+template <int C>
+LSH_HD CellEdge cell_edge(int i, int j) {
+    CellEdge e;
+    if (C < 2) {
+        e.x = i;
+        e.y = ((j & 1) == C) ? j : j + 1;
+        e.second = (e.y == j) && j > 0;
+        e.boundary = (e.y == 0);
+    } else {
+        e.y = j;
+        e.x = ((i & 1) == C - 2) ? i : i + 1;
+        e.second = (e.x == i) && i > 0;
+        e.boundary = (e.x == 0);
+    }
+    return e;
+}
+
+// The limiter's factors on the edges of cell (i, j) before colour C, in colour
+// order (factors[0 .. C), may be null), and the mass terms that those edges
+// leave in the cell's accumulator of `layer` -- what the colour passes' limiter
+// reads.  An edge with neither cell marked has factor 1.  The other cell's
+// partial sum comes from the same function with the edge's colour, so at most
+// 2^C - 1 edges are visited, and few where marked cells are.
+template <int C>
+LSH_RECURSE double partial_mass(const KArgs& a, int i, int j, int layer, double dt, double* factors);
+template <>
+LSH_HD double partial_mass<0>(const KArgs&, int, int, int, double, double*) { return 0.0; }
+
+// One colour of partial_mass: the mass the colour-P edge takes from the cell
+// whose partial sum before it is acc.
+template <int P>
+LSH_HD double limited_mass(const KArgs& a, int i, int j, int layer, double dt, double acc, double* factor) {
+    constexpr int DIR = P / 2;
+    const CellEdge e = cell_edge<P>(i, j);
+    const size_t at = (size_t)e.y * (a.c.nx + DIR) + e.x, np = a.eb.plane[DIR];
+    if (factor) *factor = 1.0;
+    if (a.eb.kind[DIR][at] <= layer) return 0.0;
+    const double m = a.eb.q[DIR][at + (layer ? 6 : 0) * np], p = a.eb.q[DIR][at + (layer ? 9 : 3) * np];
+    const double own = e.second ? p : m;
+    const EdgeSides s = edge_sides<DIR>(a, e.x, e.y);
+    const unsigned now = stage_mark(a);
+    const unsigned* mark = a.eb.mark[layer];
+    if (!(mark[s.id0] == now || (s.interior && mark[s.id1] == now))) return own;
+    if (!gt0(m) && !(s.interior && gt0(p))) return own;
+    double other = 0.0;
+    if (s.interior) {
+        const int io = e.second ? s.id0 - s.row0 * a.c.nx : s.id1 - s.row1 * a.c.nx;
+        other = partial_mass<P>(a, io, e.second ? s.row0 : s.row1, layer, dt, nullptr);
+    }
+    const int row1 = s.interior ? s.row1 : s.row0;
+    const double f = limiter(m, p, s.interior, a.eb.depth[layer][s.id0], e.second ? other : acc, a.geo.area[s.row0],
+                             a.geo.inv_area[s.row0], s.interior ? a.eb.depth[layer][s.id1] : 0.0,
+                             e.second ? acc : other, a.geo.area[row1], a.geo.inv_area[row1], dt, a.c);
+    if (factor) *factor = f;
+    return (lshm::bits_of(f) != lshm::bits_of(1.0)) ? f * own : own;
+}
+
+template <int C>
+LSH_RECURSE double partial_mass(const KArgs& a, int i, int j, int layer, double dt, double* factors) {
+    const double acc = partial_mass<C - 1>(a, i, j, layer, dt, factors);
+    const double d = limited_mass<C - 1>(a, i, j, layer, dt, acc, factors ? factors + (C - 1) : nullptr);
+    return acc - d;
+}
+
+// Subtracts the colour-C edge's terms from the cell's accumulators (the first
+// colour writes them), as do_edge's scatter does.  `f`: the limiter's factors
+// of the two layers' edges by colour (null: all 1).
+template <int C>
+LSH_HD void add_edge(const KArgs& a, int i, int j, int kind, const double* f1, const double* f2, double acc[7]) {
+    constexpr int DIR = C / 2;
+    if (kind == kEdgeDry) return;
+    const CellEdge e = cell_edge<C>(i, j);
+    const size_t at = (size_t)e.y * (a.c.nx + DIR) + e.x, np = a.eb.plane[DIR];
+    const double* q = a.eb.q[DIR] + at;
+    // back to x/y: DIR 1: (qx, qy) = sg (fn, ft); DIR 0: qx = -sg ft, qy = sg fn
+    const bool neg = e.boundary;  // normal toward -x, -y
+    auto take = [&](int l, const double* f, double v0, double v1, double v2) {
+        if (f && lshm::bits_of(f[C]) != lshm::bits_of(1.0)) { v0 = f[C] * v0; v1 = f[C] * v1; v2 = f[C] * v2; }
+        const double dn = lshm::neg_if(v1, neg), dq = lshm::neg_if(v2, (DIR == 1) ? neg : !neg);
+        const double dx = (DIR == 1) ? dn : dq, dy = (DIR == 1) ? dq : dn;
+        const int k = 3 * l;
+        if (C == 0) { acc[k] = minus0(v0); acc[k + 1] = minus0(dx); acc[k + 2] = minus0(dy); }
+        else { acc[k] = acc[k] - v0; acc[k + 1] = acc[k + 1] - dx; acc[k + 2] = acc[k + 2] - dy; }
+    };
+    // the second cell's tangential momentum is the first's, negated
+    take(0, f1, q[(e.second ? 3 : 0) * np], q[(e.second ? 4 : 1) * np], lshm::neg_if(q[2 * np], e.second));
+    if (kind == kEdgeBoth)
+        take(1, f2, q[(e.second ? 9 : 6) * np], q[(e.second ? 10 : 7) * np], lshm::neg_if(q[8 * np], e.second));
+    const double w = q[5 * np];
+    acc[6] = (C == 0) ? plus0(w) : acc[6] + w;
+}
+
+// One cell of the Euler-stage update after the flux pass (MODE as volume_finish).
+// `busy` is set where the cell's input or output state is not all +0 or one of
+// its edges is not dry.
+template <int MODE>
+LSH_HD unsigned long long update_cell(const KArgs& a, int i, int j, double dt, bool& busy) {
+    const int nx = a.c.nx, ny = a.c.ny, id = j * nx + i;
+    const unsigned char* kh = a.eb.kind[0] + id;
+    const unsigned char* kv = a.eb.kind[1] + (size_t)j * (nx + 1) + i;
+    const int kb = kh[0], kt = kh[nx], kl = kv[0], kr = kv[1], any = kb | kt | kl | kr;
+    busy |= (any != 0);
+    // an edge is limited only where one of its two cells is marked
+    bool limit[2] = {false, false};
+    double f[8];
+    if (any) {
+        const unsigned now = stage_mark(a);
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+            if (l == 1 && !(any & kEdgeBoth)) break;
+            const unsigned* mk = a.eb.mark[l] + id;
+            bool m = (mk[0] == now);
+            if (j > 0) m |= (mk[-nx] == now);
+            if (j < ny - 1) m |= (mk[nx] == now);
+            if (i > 0) m |= (mk[-1] == now);
+            if (i < nx - 1) m |= (mk[1] == now);
+            limit[l] = m;
+        }
+        if (limit[0]) partial_mass<4>(a, i, j, 0, dt, f);
+        if (limit[1]) partial_mass<4>(a, i, j, 1, dt, f + 4);
+    }
+    double wo[6], acc[7];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) wo[k] = a.W[k][id];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) acc[k] = 0.0;
+    if (any) {
+        const bool je = !(j & 1), ie = !(i & 1);
+        const double* f1 = limit[0] ? f : nullptr;
+        const double* f2 = limit[1] ? f + 4 : nullptr;
+        add_edge<0>(a, i, j, je ? kb : kt, f1, f2, acc);
+        add_edge<1>(a, i, j, je ? kt : kb, f1, f2, acc);
+        add_edge<2>(a, i, j, ie ? kl : kr, f1, f2, acc);
+        add_edge<3>(a, i, j, ie ? kr : kl, f1, f2, acc);
+    }
+    return volume_finish<MODE>(a, id, j, dt, wo, acc, &busy);
 }
 
 // dt from the largest acc_w / area: 2 CFL / max rate, 1e30 when no cell has a wave speed
