@@ -124,6 +124,16 @@ LSH_HD double from_halves(uint32_t lo, uint32_t hi) {
 #endif
 }
 
+// At the head of a rarely taken block of a few FP64 instructions: keeps it a
+// branch.  The compiler would otherwise predicate the block into every warp's
+// stream, and an FP64 instruction predicated off holds the FP64 unit like any
+// other (counted with ncu: a warp barrier in the block is not predicated).
+LSH_HD void rare() {
+#if defined(__CUDA_ARCH__)
+    __syncwarp(__activemask());
+#endif
+}
+
 // c ? -x : x by flipping the sign bit (integer pipe): the bits of -x
 LSH_HD double neg_if(double x, bool c) {
     uint32_t lo, hi;
@@ -155,17 +165,30 @@ LSH_HD bool lt0(double x) {
 // patterns, and every negative pattern (-0 included) is below c's
 LSH_HD bool lt_pos(double x, double c) { return (int64_t)bits_of(x) < (int64_t)bits_of(c); }
 LSH_HD bool gt_pos(double x, double c) { return (int64_t)bits_of(x) > (int64_t)bits_of(c); }
-// |x| by clearing the sign bit (integer pipe): the bits fabs gives.  A
-// fabs whose result feeds an integer-pipe compare would otherwise be
-// materialised by an FP64 instruction.
-LSH_HD double abs_bits(double x) { return from_bits(bits_of(x) & kMag); }
+// |x| by clearing the sign bit (integer pipe): the bits fabs gives.  Through
+// halves: a fabs that the compiler recognises, and whose result feeds an
+// integer-pipe compare, is materialised by an FP64 instruction.
+LSH_HD uint64_t mag_bits(double x) {
+    uint32_t lo, hi;
+    halves(x, lo, hi);
+    return ((uint64_t)(hi & 0x7fffffffu) << 32) | lo;
+}
+LSH_HD double abs_bits(double x) {
+    uint32_t lo, hi;
+    halves(x, lo, hi);
+    return from_halves(lo, hi & 0x7fffffffu);
+}
 // |a| < |b|
-LSH_HD bool abs_lt(double a, double b) { return (bits_of(a) & kMag) < (bits_of(b) & kMag); }
+LSH_HD bool abs_lt(double a, double b) { return mag_bits(a) < mag_bits(b); }
 // a key ordered like the doubles, -0 and +0 both 0: the magnitude, negated
 // for a negative value
+// (through halves: on the plain bits the compiler finds |x| and materialises it
+// with an FP64 instruction)
 LSH_HD int64_t okey(double x) {
-    const int64_t k = (int64_t)bits_of(x);
-    return (k < 0) ? -(k & (int64_t)kMag) : k;
+    uint32_t lo, hi;
+    halves(x, lo, hi);
+    const int64_t k = (int64_t)(((uint64_t)hi << 32) | lo);
+    return ((int32_t)hi < 0) ? -(k & (int64_t)kMag) : k;
 }
 // a < b, any non-NaN a and b
 LSH_HD bool lt(double a, double b) { return okey(a) < okey(b); }

@@ -490,8 +490,8 @@ __global__ void __launch_bounds__(32 * kFluxWarps, LSH_FLUX_MINB)
     const int q = (int)((u0 + threadIdx.x / 32) % kFluxWarps), lane = threadIdx.x & 31;
     const int x = tx * kTileX + (lane & (kTileX - 1)), y = ty * kTileY + (q & 1) * 2 + lane / kTileX;
     const double dt = a.tm->dt;
-    if (q & 2) { if (x <= nx && y < ny) lsh::flux_edge<1, ORDER>(a, x, y, dt); }
-    else { if (x < nx && y <= ny) lsh::flux_edge<0, ORDER>(a, x, y, dt); }
+    const int dir = q >> 1;
+    if (dir ? (x <= nx && y < ny) : (x < nx && y <= ny)) lsh::flux_edge<ORDER>(a, dir, x, y, dt);
     tile_end(d, ty);
 }
 

@@ -15,7 +15,7 @@ namespace lsh {
 constexpr unsigned long long kRateInitBits = 0ULL;  // +0.0
 constexpr int kEdgeBlock = 128;
 constexpr int kCellBlock = 256;
-constexpr double kReconThin = 0.5;  // second order: least face depth / cell depth
+constexpr double kReconThin = 0.5;  // second order: least face depth / cell depth (half() of the depth)
 
 // Sticky error bit: an atomic OR on the device, a plain OR in host code.
 LSH_HD void err_or(int* word, int bit) {
@@ -23,24 +23,6 @@ LSH_HD void err_or(int* word, int bit) {
     atomicOr(word, bit);
 #else
     *word |= bit;
-#endif
-}
-
-// p on every active lane of the warp (the thread's own p in host code).
-LSH_HD bool warp_all(bool p) {
-#if defined(__CUDA_ARCH__)
-    return __all_sync(__activemask(), p);
-#else
-    return p;
-#endif
-}
-
-// p on some active lane of the warp (the thread's own p in host code).
-LSH_HD bool warp_any(bool p) {
-#if defined(__CUDA_ARCH__)
-    return __any_sync(__activemask(), p);
-#else
-    return p;
 #endif
 }
 
@@ -317,11 +299,15 @@ LSH_HD void do_edge(const KArgs& a, int x, int y, double dt) {
 // operands that are not NaN the same as the compares
 //   a > 0 && b > 0 ? (a < b ? a : b) : a < 0 && b < 0 ? (a > b ? a : b) : 0
 LSH_HD double minmod(double a, double b) {
-    const uint64_t ua = lshm::bits_of(a), ub = lshm::bits_of(b);
-    const bool nonzero = ((ua << 1) != 0) && ((ub << 1) != 0);
-    const bool same = ((ua ^ ub) >> 63) == 0;
+    // (through halves: on the plain bits the compiler finds a == 0 and b == 0)
+    uint32_t alo, ahi, blo, bhi;
+    lshm::halves(a, alo, ahi);
+    lshm::halves(b, blo, bhi);
+    const uint32_t am = ahi & 0x7fffffffu, bm = bhi & 0x7fffffffu;
+    const bool nonzero = (am | alo) != 0u && (bm | blo) != 0u;
+    const bool same = (int32_t)(ahi ^ bhi) >= 0;
     if (!(nonzero && same)) return 0.0;
-    return ((ua & lshm::kMag) < (ub & lshm::kMag)) ? a : b;
+    return ((((uint64_t)am << 32) | alo) < (((uint64_t)bm << 32) | blo)) ? a : b;
 }
 
 LSH_HD double recon_var(const KArgs& a, int id, int k) {
@@ -358,27 +344,21 @@ LSH_HD void recon_cell_from(const KArgs& a, int id, int i, int j, const Acc& w) 
             return;
         }
     }
-    // the reconstructed variables: eta1 = h1 + h2 - H, eta2 = h2 - H, the discharges, H
-    auto rv = [&](int k, int di, int dj) -> double {
-        if (k == 0) return (w(0, di, dj) + w(3, di, dj)) - w(6, di, dj);
-        if (k == 3) return w(3, di, dj) - w(6, di, dj);
-        return w(k, di, dj);
-    };
     const bool inx = (i > 0 && i < nx - 1), iny = (j > 0 && j < ny - 1);
-    auto slope_x = [&](int k) {
-        const double pc = rv(k, 0, 0);
-        return inx ? lsh::half(minmod(pc - rv(k, -1, 0), rv(k, 1, 0) - pc)) : 0.0;
-    };
-    auto slope_y = [&](int k) {
-        const double pc = rv(k, 0, 0);
-        return iny ? lsh::half(minmod(pc - rv(k, 0, -1), rv(k, 0, 1) - pc)) : 0.0;
+    // halved minmod slopes of a variable rv(di, dj)
+    auto slopes = [&](auto rv, double& x, double& y) {
+        const double pc = rv(0, 0);
+        x = inx ? lsh::half(minmod(pc - rv(-1, 0), rv(1, 0) - pc)) : 0.0;
+        y = iny ? lsh::half(minmod(pc - rv(0, -1), rv(0, 1) - pc)) : 0.0;
     };
     // No granular layer anywhere in the stencil (h2 = q2 = 0 at the cell and
-    // the neighbours it reads): eta2 = 0 - H, whose differences are exactly
-    // the negated differences of H, so its slope is the negated H slope, or
-    // +0 where minmod gives 0; the q2 slopes are minmod's 0, so +0; and the
-    // fallback's h2 tests, 0 +- 0 against 0.5 * 0, never fire.  A warp whose
-    // cells all qualify skips that FP64 work and gets the same bits.
+    // the neighbours it reads): eta1 = (h1 + 0) - H is h1 - H (but for the sign
+    // of a zero, which minmod does not see); eta2 = 0 - H, whose differences
+    // are exactly the negated differences of H, so its slope is the negated H
+    // slope, or +0 where minmod gives 0; the q2 slopes are minmod's 0, so +0;
+    // and the fallback's h2 tests, 0 +- 0 against 0.5 * 0, never fire.  A warp
+    // whose cells all qualify skips that FP64 work and gets the same bits: 23
+    // FP64 instructions instead of 56.
     bool one = true;
     {
         using lsh::is_zero;
@@ -392,32 +372,44 @@ LSH_HD void recon_cell_from(const KArgs& a, int id, int i, int j, const Acc& w) 
         if (one && j < ny - 1) one = nolayer(0, 1);
     }
     double sx[7], sy[7];
+    const double h1 = w(0, 0, 0);
+    bool bad = false;
+    slopes([&](int di, int dj) { return w(1, di, dj); }, sx[1], sy[1]);
+    slopes([&](int di, int dj) { return w(2, di, dj); }, sx[2], sy[2]);
+    slopes([&](int di, int dj) { return w(6, di, dj); }, sx[6], sy[6]);
     const bool fast = warp_all(one);
     if (fast) {
-        sx[0] = slope_x(0); sy[0] = slope_y(0);
-        sx[1] = slope_x(1); sy[1] = slope_y(1);
-        sx[2] = slope_x(2); sy[2] = slope_y(2);
-        sx[6] = slope_x(6); sy[6] = slope_y(6);
+        slopes([&](int di, int dj) { return w(0, di, dj) - w(6, di, dj); }, sx[0], sy[0]);
         sx[3] = lsh::is_zero(sx[6]) ? 0.0 : lshm::neg_if(sx[6], true);
         sy[3] = lsh::is_zero(sy[6]) ? 0.0 : lshm::neg_if(sy[6], true);
         sx[4] = sx[5] = sy[4] = sy[5] = 0.0;
     } else {
-#pragma unroll
-        for (int k = 0; k < 7; ++k) { sx[k] = slope_x(k); sy[k] = slope_y(k); }
+        lshm::rare();
+        slopes([&](int di, int dj) { return (w(0, di, dj) + w(3, di, dj)) - w(6, di, dj); }, sx[0], sy[0]);
+        slopes([&](int di, int dj) { return w(3, di, dj) - w(6, di, dj); }, sx[3], sy[3]);
+        slopes([&](int di, int dj) { return w(4, di, dj); }, sx[4], sy[4]);
+        slopes([&](int di, int dj) { return w(5, di, dj); }, sx[5], sy[5]);
     }
-    const double h1 = w(0, 0, 0), h2 = w(3, 0, 0);
-    const double dh1x = sx[0] - sx[3], dh1y = sy[0] - sy[3];
     // first order where a reconstructed depth would fall below kReconThin of
     // the cell's: a thin face with a finite discharge has an unbounded
-    // velocity, whose wave speed would collapse dt
-    // (the compares on the integer pipe)
-    const double g1 = kReconThin * h1;
+    // velocity, whose wave speed would collapse dt (the compares on the
+    // integer pipe).  Where every depth slope is at most a quarter of the
+    // depth (by the exponents) no face of layer 1 falls below it.
+    const double dh1x = sx[0] - sx[3], dh1y = sy[0] - sy[3];
     using lshm::okey;
-    const int64_t k1 = okey(g1);
-    bool bad = okey(h1 + dh1x) < k1 || okey(h1 - dh1x) < k1 || okey(h1 + dh1y) < k1 || okey(h1 - dh1y) < k1;
+    const int64_t quarter = (int64_t)lshm::bits_of(h1) - ((int64_t)2 << 52);
+    const bool deep = quarter > ((int64_t)1 << 52) && (int64_t)lshm::bits_of(lshm::abs_bits(dh1x)) <= quarter &&
+                      (int64_t)lshm::bits_of(lshm::abs_bits(dh1y)) <= quarter;
+    if (!warp_all(deep)) {
+        lshm::rare();
+        const int64_t k1 = okey(lsh::half(h1));  // kReconThin h1
+        bad = okey(h1 + dh1x) < k1 || okey(h1 - dh1x) < k1 || okey(h1 + dh1y) < k1 || okey(h1 - dh1y) < k1;
+    }
     if (!fast) {
+        lshm::rare();
+        const double h2 = w(3, 0, 0);
         const double dh2x = sx[3] + sx[6], dh2y = sy[3] + sy[6];
-        const int64_t k2 = okey(kReconThin * h2);
+        const int64_t k2 = okey(lsh::half(h2));
         bad = bad || okey(h2 + dh2x) < k2 || okey(h2 - dh2x) < k2 || okey(h2 + dh2y) < k2 || okey(h2 - dh2y) < k2;
     }
 #pragma unroll
@@ -468,7 +460,8 @@ __device__ __forceinline__ void block_max_bits(unsigned long long v, unsigned lo
 // MODE 0: order 1, in place.  MODE 1: order 2 stage 1 (W -> Wout).
 // MODE 2: order 2 stage 2, Wout = (Xavg + E(W)) / 2.
 // `busy` (may be null): set where the input or the output state is not all +0.
-template <int MODE>
+// PESO1: the caller knows that peso is 1.
+template <int MODE, bool PESO1 = false>
 LSH_HD unsigned long long volume_finish(const KArgs& a, int id, int j, double dt, const double wo[6], double acc[7],
                                         bool* busy = nullptr) {
     double w[6], rate;
@@ -499,8 +492,7 @@ LSH_HD unsigned long long volume_finish(const KArgs& a, int id, int j, double dt
         using lsh::is_zero;
         bool one = is_zero(wo[3]) && is_zero(wo[4]) && is_zero(wo[5]) && lshm::bits_of(acc[3]) == 0 &&
                    lshm::bits_of(acc[4]) == 0 && lshm::bits_of(acc[5]) == 0;
-        // times peso, whose usual value is 1
-        auto times_peso = [&](double v) { return (lshm::bits_of(a.c.peso) != lshm::bits_of(1.0)) ? a.c.peso * v : v; };
+        auto times_peso = [&](double v) { return PESO1 ? v : a.c.peso * v; };
         double s0x = 0.0, s3x = 0.0, s0y = 0.0, s3y = 0.0;
         if (a.c.order == 2) {
             s0x = a.sx[0][id]; s3x = a.sx[3][id]; s0y = a.sy[0][id]; s3y = a.sy[3][id];
@@ -546,20 +538,24 @@ LSH_HD unsigned long long volume_finish(const KArgs& a, int id, int j, double dt
         // takes the AND as a whole: a per-variable select is if-converted, and
         // its predicated-off FP64 instructions still hold the FP64 pipe.
         double x[6];
-        bool z = true;
+        bool z[2] = {true, true};  // per layer
         keep = still;
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
             x[k] = a.Xavg[k][id];
-            z &= lsh::is_zero(x[k]) && lsh::is_zero(w[k]);
+            z[k / 3] &= lsh::is_zero(x[k]) && lsh::is_zero(w[k]);
             keep &= (a.Wout[k] == a.Xavg[k]) && (lshm::bits_of(x[k]) == lshm::bits_of(w[k]));
         }
-        if (warp_all(z)) {
 #pragma unroll
-            for (int k = 0; k < 6; ++k) w[k] = lshm::from_bits(lshm::bits_of(x[k]) & lshm::bits_of(w[k]));
-        } else {
+        for (int l = 0; l < 2; ++l) {
+            if (warp_all(z[l])) {
 #pragma unroll
-            for (int k = 0; k < 6; ++k) w[k] = lsh::half(x[k] + w[k]);
+                for (int k = 3 * l; k < 3 * l + 3; ++k) w[k] = lshm::from_bits(lshm::bits_of(x[k]) & lshm::bits_of(w[k]));
+            } else {
+                lshm::rare();
+#pragma unroll
+                for (int k = 3 * l; k < 3 * l + 3; ++k) w[k] = lsh::half(x[k] + w[k]);
+            }
         }
     }
     if (busy) {
@@ -609,37 +605,116 @@ inline bool flux_fits(const lsh_params& p) { return p.peso == 1.0 && p.beta >= 1
 
 LSH_HD unsigned stage_mark(const KArgs& a) { return 2u * (unsigned)a.tm->steps + a.eb.stage + 1u; }
 
-// One edge of the flux pass.
+// x + y is exactly 0 (opposite values, or zeros), by the bits
+LSH_HD bool cancel(double x, double y) {
+    return lshm::bits_of(x) == (lshm::bits_of(y) ^ ~lshm::kMag) || (is_zero(x) && is_zero(y));
+}
+
+// No granular layer at cell `id` and its faces: h2, q2 and, at second order,
+// what their slopes add (eta2's and H's slopes cancel) are zeros.
+template <int ORDER>
+LSH_HD bool bare_cell(const KArgs& a, int id, const double* const* s) {
+    bool b = is_zero(a.W[3][id]) && is_zero(a.W[4][id]) && is_zero(a.W[5][id]);
+    if (ORDER == 2) b = b && is_zero(s[4][id]) && is_zero(s[5][id]) && cancel(s[3][id], s[6][id]);
+    return b;
+}
+
+// Layer 1 of a face (face_depths, face_rest) and zeros for layer 2.
 template <int DIR, int ORDER>
-LSH_HD void flux_edge(const KArgs& a, int x, int y, double dt) {
-    const EdgeSides s = edge_sides<DIR>(a, x, y);
-    const size_t e = (size_t)y * (a.c.nx + DIR) + x, np = a.eb.plane[DIR];
-    double* const q = a.eb.q[DIR];
-    if (DIR == 0 && a.eb.depth_out[0] && y < a.c.ny) {
+LSH_HD void bare_face(const KArgs& a, int id, int side, bool pos_normal, Face& f) {
+    using lshm::neg_if;
+    const bool neg = !(side & 1);
+    double qx = a.W[1][id], qy = a.W[2][id];
+    f.H = a.W[6][id];
+    if (ORDER == 2) {
+        const double* const* s = (side < 2) ? a.sx : a.sy;
+        qx = qx + neg_if(s[1][id], neg);
+        qy = qy + neg_if(s[2][id], neg);
+        f.H = f.H + neg_if(s[6][id], neg);
+    }
+    f.qn1 = neg_if(DIR == 1 ? qx : qy, !pos_normal);
+    f.qt1 = neg_if(DIR == 1 ? qy : qx, DIR == 1 ? !pos_normal : pos_normal);
+    f.h2 = f.qn2 = f.qt2 = 0.0;
+}
+template <int ORDER>
+LSH_HD double bare_depth(const KArgs& a, int id, int side) {
+    double h = a.W[0][id];
+    if (ORDER == 2) {
+        const double* const* s = (side < 2) ? a.sx : a.sy;
+        h = h + lshm::neg_if(s[0][id] - s[3][id], !(side & 1));
+    }
+    return h;
+}
+
+// The faces of an edge and its kind.  A warp whose edges all lie between cells
+// without a granular layer takes their layer-1 faces alone: 10 FP64
+// instructions instead of 24 at second order, none instead of 2 at first.
+template <int DIR, int ORDER>
+LSH_HD EdgeKind flux_faces(const KArgs& a, const EdgeSides& s, Face& A, Face& B) {
+    constexpr int side1 = (DIR == 0) ? 2 : 0;
+    const double* const* sl = (DIR == 0) ? a.sy : a.sx;
+    bool empty = is_zero(a.W[0][s.id0]) && is_zero(a.W[3][s.id0]) && (ORDER == 1 || a.szero[s.id0]);
+    if (empty && s.interior)
+        empty = is_zero(a.W[0][s.id1]) && is_zero(a.W[3][s.id1]) && (ORDER == 1 || a.szero[s.id1]);
+    if (empty) return kEdgeDry;
+    bool bare = bare_cell<ORDER>(a, s.id0, sl);
+    if (bare && s.interior) bare = bare_cell<ORDER>(a, s.id1, sl);
+    if (warp_all(bare)) {
+        A.h1 = bare_depth<ORDER>(a, s.id0, s.side0);
+        B.h1 = s.interior ? bare_depth<ORDER>(a, s.id1, side1) : A.h1;
+        if (lshm::lt_pos(half(A.h1 + B.h1), kEps)) return kEdgeDry;
+        bare_face<DIR, ORDER>(a, s.id0, s.side0, s.pos_normal, A);
+        if (s.interior) {
+            bare_face<DIR, ORDER>(a, s.id1, side1, s.pos_normal, B);
+        } else {
+            lshm::rare();
+            B = A;
+            B.qn1 = A.qn1 * s.bor;
+        }
+        return kEdgeSingle;
+    }
+    if (!edge_wet<DIR, ORDER>(a, s, A, B)) return kEdgeDry;
+    edge_faces<DIR, ORDER>(a, s, A, B);
+    return (is_zero(A.h2) && is_zero(B.h2) && is_zero(A.qn2) && is_zero(B.qn2)) ? kEdgeSingle : kEdgeBoth;
+}
+
+// One edge of the flux pass: dir 0 horizontal, 1 vertical.  The direction is a
+// value so that both share one copy of the flux's code (two filled the
+// instruction cache: 5.7 of 41 stall cycles per issue waited for it).
+template <int ORDER>
+LSH_HD void flux_edge(const KArgs& a, int dir, int x, int y, double dt) {
+    if (dir == 0 && a.eb.depth_out[0] && y < a.c.ny) {
         // order 1 updates in place: the limiter reads this copy, since a
         // neighbour may already hold its new depth
         const int id = y * a.c.nx + x;
         a.eb.depth_out[0][id] = a.W[0][id];
         a.eb.depth_out[1][id] = a.W[3][id];
     }
+    EdgeSides s;
     Face A, B;
-    if (!edge_wet<DIR, ORDER>(a, s, A, B)) {
-        a.eb.kind[DIR][e] = kEdgeDry;
-        return;
+    EdgeKind kind;
+    if (dir) {
+        s = edge_sides<1>(a, x, y);
+        kind = flux_faces<1, ORDER>(a, s, A, B);
+    } else {
+        s = edge_sides<0>(a, x, y);
+        kind = flux_faces<0, ORDER>(a, s, A, B);
     }
-    edge_faces<DIR, ORDER>(a, s, A, B);
-    const bool single = is_zero(A.h2) && is_zero(B.h2) && is_zero(A.qn2) && is_zero(B.qn2);
+    const size_t e = (size_t)y * (a.c.nx + dir) + x, np = dir ? a.eb.plane[1] : a.eb.plane[0];
+    (dir ? a.eb.kind[1] : a.eb.kind[0])[e] = kind;
+    if (kind == kEdgeDry) return;
+    const bool single = (kind == kEdgeSingle);
     EdgeRaw r;
-    if (single) edge_raw<false>(A, B, s.len, dt, a.c, r);
-    else edge_raw<true>(A, B, s.len, dt, a.c, r);
-    a.eb.kind[DIR][e] = single ? kEdgeSingle : kEdgeBoth;
-    q[e] = r.m[0]; q[e + np] = r.m[1]; q[e + 2 * np] = r.m[2];
-    q[e + 3 * np] = r.p[0]; q[e + 4 * np] = r.p[1]; q[e + 5 * np] = r.wave;
+    if (single) edge_raw1(A, B, s.len, a.c, r);
+    else edge_raw2(A, B, s.len, dt, a.c, r);
+    double* const q = (dir ? a.eb.q[1] : a.eb.q[0]) + e;
+    q[0] = r.m[0]; q[np] = r.m[1]; q[2 * np] = r.m[2];
+    q[3 * np] = r.p[0]; q[4 * np] = r.p[1]; q[5 * np] = r.wave;
     if (!single) {
-        q[e + 6 * np] = r.m[3]; q[e + 7 * np] = r.m[4]; q[e + 8 * np] = r.m[5];
-        q[e + 9 * np] = r.p[2]; q[e + 10 * np] = r.p[3];
+        q[6 * np] = r.m[3]; q[7 * np] = r.m[4]; q[8 * np] = r.m[5];
+        q[9 * np] = r.p[2]; q[10 * np] = r.p[3];
     }
-    const double scale = tmax(1.0, tmax(a.c.beta, a.c.peso));
+    const double scale = a.c.beta;  // >= peso = 1 (flux_fits)
 #pragma unroll
     for (int l = 0; l < 2; ++l) {
         if (l == 1 && single) break;
@@ -725,9 +800,9 @@ LSH_RECURSE double partial_mass(const KArgs& a, int i, int j, int layer, double 
 }
 
 // Subtracts the colour-C edge's terms from the cell's accumulators (the first
-// colour writes them), as do_edge's scatter does.  `f`: the limiter's factors
-// of the two layers' edges by colour (null: all 1).
-template <int C>
+// colour writes them), as do_edge's scatter does.  LIMIT: with the limiter's
+// factors f1, f2 of the layers' edges by colour (null: all 1).
+template <int C, bool LIMIT>
 LSH_HD void add_edge(const KArgs& a, int i, int j, int kind, const double* f1, const double* f2, double acc[7]) {
     constexpr int DIR = C / 2;
     if (kind == kEdgeDry) return;
@@ -737,7 +812,7 @@ LSH_HD void add_edge(const KArgs& a, int i, int j, int kind, const double* f1, c
     // back to x/y: DIR 1: (qx, qy) = sg (fn, ft); DIR 0: qx = -sg ft, qy = sg fn
     const bool neg = e.boundary;  // normal toward -x, -y
     auto take = [&](int l, const double* f, double v0, double v1, double v2) {
-        if (f && lshm::bits_of(f[C]) != lshm::bits_of(1.0)) { v0 = f[C] * v0; v1 = f[C] * v1; v2 = f[C] * v2; }
+        if (LIMIT && f && lshm::bits_of(f[C]) != lshm::bits_of(1.0)) { v0 = f[C] * v0; v1 = f[C] * v1; v2 = f[C] * v2; }
         const double dn = lshm::neg_if(v1, neg), dq = lshm::neg_if(v2, (DIR == 1) ? neg : !neg);
         const double dx = (DIR == 1) ? dn : dq, dy = (DIR == 1) ? dq : dn;
         const int k = 3 * l;
@@ -746,8 +821,10 @@ LSH_HD void add_edge(const KArgs& a, int i, int j, int kind, const double* f1, c
     };
     // the second cell's tangential momentum is the first's, negated
     take(0, f1, q[(e.second ? 3 : 0) * np], q[(e.second ? 4 : 1) * np], lshm::neg_if(q[2 * np], e.second));
-    if (kind == kEdgeBoth)
+    if (kind == kEdgeBoth) {
+        lshm::rare();
         take(1, f2, q[(e.second ? 9 : 6) * np], q[(e.second ? 10 : 7) * np], lshm::neg_if(q[8 * np], e.second));
+    }
     const double w = q[5 * np];
     acc[6] = (C == 0) ? plus0(w) : acc[6] + w;
 }
@@ -787,15 +864,22 @@ LSH_HD unsigned long long update_cell(const KArgs& a, int i, int j, double dt, b
 #pragma unroll
     for (int k = 0; k < 7; ++k) acc[k] = 0.0;
     if (any) {
-        const bool je = !(j & 1), ie = !(i & 1);
-        const double* f1 = limit[0] ? f : nullptr;
-        const double* f2 = limit[1] ? f + 4 : nullptr;
-        add_edge<0>(a, i, j, je ? kb : kt, f1, f2, acc);
-        add_edge<1>(a, i, j, je ? kt : kb, f1, f2, acc);
-        add_edge<2>(a, i, j, ie ? kl : kr, f1, f2, acc);
-        add_edge<3>(a, i, j, ie ? kr : kl, f1, f2, acc);
+        const int k0 = (j & 1) ? kt : kb, k1 = (j & 1) ? kb : kt, k2 = (i & 1) ? kr : kl, k3 = (i & 1) ? kl : kr;
+        if (warp_any(limit[0] || limit[1])) {
+            const double* f1 = limit[0] ? f : nullptr;
+            const double* f2 = limit[1] ? f + 4 : nullptr;
+            add_edge<0, true>(a, i, j, k0, f1, f2, acc);
+            add_edge<1, true>(a, i, j, k1, f1, f2, acc);
+            add_edge<2, true>(a, i, j, k2, f1, f2, acc);
+            add_edge<3, true>(a, i, j, k3, f1, f2, acc);
+        } else {
+            add_edge<0, false>(a, i, j, k0, nullptr, nullptr, acc);
+            add_edge<1, false>(a, i, j, k1, nullptr, nullptr, acc);
+            add_edge<2, false>(a, i, j, k2, nullptr, nullptr, acc);
+            add_edge<3, false>(a, i, j, k3, nullptr, nullptr, acc);
+        }
     }
-    return volume_finish<MODE>(a, id, j, dt, wo, acc, &busy);
+    return volume_finish<MODE, true>(a, id, j, dt, wo, acc, &busy);
 }
 
 // dt from the largest acc_w / area: 2 CFL / max rate, 1e30 when no cell has a wave speed

@@ -74,6 +74,24 @@ struct TimeRec {
 
 struct V4 { double x, y, z, w; };
 
+// p on every active lane of the warp (the thread's own p in host code).
+LSH_HD bool warp_all(bool p) {
+#if defined(__CUDA_ARCH__)
+    return __all_sync(__activemask(), p);
+#else
+    return p;
+#endif
+}
+
+// p on some active lane of the warp (the thread's own p in host code).
+LSH_HD bool warp_any(bool p) {
+#if defined(__CUDA_ARCH__)
+    return __any_sync(__activemask(), p);
+#else
+    return p;
+#endif
+}
+
 // Compares run on the integer pipe (lsh_fpmath.h: exact for non-NaN
 // operands): lt_pos / gt_pos against the positive thresholds EPSILON, eps_h,
 // vmax, lt / okey for operands of either sign.
@@ -106,25 +124,33 @@ LSH_HD double vfac(double h, double eps_h) {
     return div(kSqrt2 * h, root(fmad(h2, h2, m2 * m2)));
 }
 
-// x / 2 and 2 x on the exponent field (integer pipe), the FP64 multiply only
-// where the result or x is not a normal number or zero
+// x / 2 and 2 x on the integer pipe (no FP64 instruction even for special
+// values: a rarely taken one would be predicated into every warp's stream, and
+// one predicated off still holds the FP64 unit).  Subnormal results round to
+// even; infinities and NaN stay.
 LSH_HD double half(double x) {
     uint32_t lo, hi;
     lshm::halves(x, lo, hi);
-    if (((hi >> 20) & 0x7ffu) - 2u < 2045u) return lshm::from_halves(lo, hi - 0x00100000u);
-    if (((hi << 1) | lo) == 0u) return x;
-    return 0.5 * x;
+    const uint32_t e = (hi >> 20) & 0x7ffu;
+    if (e - 2u < 2045u) return lshm::from_halves(lo, hi - 0x00100000u);
+    if (e >= 2u) return x;
+    // the magnitude is m 2^-1074 (exponent 1 included): m / 2, ties to even
+    const uint64_t m = ((uint64_t)(hi & 0x7fffffffu) << 32) | lo;
+    const uint64_t h = (m >> 1) + (m & (m >> 1) & 1u);
+    return lshm::from_halves((uint32_t)h, (uint32_t)(h >> 32) | (hi & 0x80000000u));
 }
 LSH_HD double twice(double x) {
     uint32_t lo, hi;
     lshm::halves(x, lo, hi);
-    if (((hi >> 20) & 0x7ffu) - 1u < 2045u) return lshm::from_halves(lo, hi + 0x00100000u);
-    if (((hi << 1) | lo) == 0u) return x;
-    return 2.0 * x;
+    const uint32_t e = (hi >> 20) & 0x7ffu;
+    if (e - 1u < 2045u) return lshm::from_halves(lo, hi + 0x00100000u);
+    if (e == 0x7ffu) return x;
+    if (e != 0u) return lshm::from_halves(0u, (hi & 0x80000000u) | 0x7ff00000u);
+    return lshm::from_halves(lo << 1, (hi & 0x80000000u) | (hi << 1) | (lo >> 31));
 }
 
 // 0 + x and 0 - x on the integer pipe: x and -x, with +0 for either zero (NaN
-// takes the FP64 operation: its sign steers the limiter's integer compares)
+// keeps its sign, which steers integer compares)
 LSH_HD double plus0(double x) {
     uint32_t lo, hi;
     lshm::halves(x, lo, hi);
@@ -133,8 +159,9 @@ LSH_HD double plus0(double x) {
 LSH_HD double minus0(double x) {
     uint32_t lo, hi;
     lshm::halves(x, lo, hi);
-    if ((hi & 0x7ff00000u) == 0x7ff00000u) return 0.0 - x;
-    return lshm::from_halves(lo, (((hi << 1) | lo) == 0u) ? 0u : (hi ^ 0x80000000u));
+    const uint32_t mag = hi & 0x7fffffffu;
+    const bool nan = mag > 0x7ff00000u || (mag == 0x7ff00000u && lo != 0u);
+    return lshm::from_halves(lo, ((mag | lo) == 0u) ? 0u : (nan ? hi : (hi ^ 0x80000000u)));
 }
 
 // log2 x of a positive normal x in units of 2^-20, low by at most 0.0861
@@ -197,36 +224,22 @@ LSH_HD EigBounds eig_bounds(double a, double b, double c, double d, int full) {
     return e;
 }
 
-// aproximarAutovalores1D (Arista_kernel.cu:152-237).  L2 == false: the
-// granular layer is absent (h2 = 0, u2 = 0), so the internal pair is exactly
-// zero and its square root is skipped.
-template <bool L2>
-LSH_HD EigBounds eig_edge(double h1, double h2, double u1, double u2, double q, const Consts& c,
-                                  double Fknown = -1.0, double sqrt_h = -1.0, bool mean_u = false) {
-    const double h = L2 ? h1 + h2 : h1;
+// aproximarAutovalores1D (Arista_kernel.cu:152-237), both layers.
+LSH_HD EigBounds eig_edge(double h1, double h2, double u1, double u2, double q, const Consts& c, double sqrt_h = -1.0,
+                          bool mean_u = false) {
+    const double h = h1 + h2;
+    const double F = vfac(h, c.eps_h);
     // mean_u (the edge average, q = h1 u1 + h2 u2): with no granular layer and
     // h > eps_h, u = q vfac(h) = (h1 u1) / h1 is u1 itself -- an exact
-    // restatement the CPU oracle makes too; the single-layer edge then skips
-    // the division
-    const bool direct = mean_u && is_zero(h2) && gt_pos(h, c.eps_h);
-    double F = 0.0;
-    // single layer: vfac(h1 + 0) is vfac(h1), which the caller may already hold
-    if (L2 || !direct) F = (!L2 && !lt0(Fknown)) ? Fknown : vfac(h, c.eps_h);
-    const double u = direct ? u1 : q * F;
+    // restatement the CPU oracle makes too
+    const double u = (mean_u && is_zero(h2) && gt_pos(h, c.eps_h)) ? u1 : q * F;
     // sqrt_h >= 0: sqrt(h1) is known and h2 == 0, so sqrt(g h) = sqrt(g) sqrt(h1)
     const double cg = !lt0(sqrt_h) ? c.sqrt_g * sqrt_h : root(c.g * h);
-    const double a = u - cg, d = u + cg;
-    if (!L2) {
-        // the internal pair is 0, 0: both sorts leave min(a, 0), max(d, 0) and
-        // between them 0 and the external value on the other side of 0, if any
-        const bool up = gt0(a), down = lt0(d);
-        return EigBounds{up ? 0.0 : a, down ? 0.0 : d, up ? a : (down ? abs_bits(d) : 0.0)};
-    }
     const double uu = fmad(u1, h2, u2 * h1) * F;
     const double du = u1 - u2;
     const double aux = fmad(-((du * du) * F), c.inv_gp, 1.0);
     const double ci = root((((c.gp * h1) * h2) * F) * abs_bits(aux));
-    return eig_bounds(a, uu - ci, uu + ci, d, c.eig_sort);
+    return eig_bounds(u - cg, uu - ci, uu + ci, u + cg, c.eig_sort);
 }
 
 // defTerminoFriccion (Arista_kernel.cu:11-58)
@@ -289,97 +302,158 @@ struct EdgeInPos {
 // tangential momentum is -m[3 l + 2]), and the wave term.
 struct EdgeRaw { double m[6], p[4], wave; };
 
-// procesarArista (Arista_kernel.cu:324-645) up to the limiter, the depths
-// already known to be wet (the caller skips dry edges, :397).  L2 == false:
-// both faces have no granular layer (h2 = qn2 = 0); every layer-1 value is
-// then the same as in the general path and every layer-2 output is zero, so
-// that work is skipped.
+// A single-layer edge: edge_raw where both faces have no granular layer (h2 =
+// qn2 = 0; tangential terms of layer 2 unused), whose layer-1 values are the
+// same as in the general path, and its layer-2 outputs zeros.
 //
-// The FP64 unit bounds this (16 cycles per instruction and SM, 55 cycles of
-// latency), so what gives the same bits off it runs on the integer pipe:
-// divisions and roots (lsh_ieee.h), halvings, sums with zero, compares, the
-// eigenvalue bounds' order (eig_bounds), and the differences of eigenvalues
-// with an aut2 of zero.
-template <bool L2>
-LSH_HD void edge_raw(const Face& A, const Face& B, double len, double dt, const Consts& c, EdgeRaw& o) {
+// The FP64 unit bounds every pass (16 cycles per instruction and SM, 55 of
+// latency), so what gives the same bits off it runs on the integer pipe, and
+// what only some edges need sits in blocks that a warp votes on: an
+// instruction predicated off still holds the unit.  63 FP64 instructions of
+// the 200 that the plain statement takes (10 of them the second-order faces').
+LSH_HD void edge_raw1(const Face& A, const Face& B, double len, const Consts& c, EdgeRaw& o) {
     const double eps = c.eps_h;
-    double Aq1 = A.qn1, Aq2 = L2 ? A.qn2 : 0.0, Bq1 = B.qn1, Bq2 = L2 ? B.qn2 : 0.0;
+    double Aq = A.qn1, Bq = B.qn1;
+    const double h = half(A.h1 + B.h1);
+    const double tA = A.h1 - A.H, tB = B.h1 - B.H;
+    // tratamientoSecoMojado (Arista_kernel.cu:301-321); H - h is -(h - H)
+    if (lt_pos(A.h1, eps) && lt(A.H, lshm::neg_if(tB, true))) Bq = 0.0;
+    if (lt_pos(B.h1, eps) && lt(B.H, lshm::neg_if(tA, true))) Aq = 0.0;
+    const double fA = vfac(A.h1, eps), fB = vfac(B.h1, eps);
+    const double sA = root(A.h1), sB = root(B.h1);
+    const double uA = fA * Aq, uB = fB * Bq;
+    const double u = div(fmad(sA, uA, sB * uB), sA + sB + kEps);
+
+    const double Hm = tmin(A.H, B.H);
+    const double deta = max0(tB + Hm) - max0(tA + Hm);
+    const double gh = c.g * h;
+
+    // eigenvalue bounds (eig_edge, its single-layer form): min(u - c, 0) and
+    // max(u + c, 0) of the average and of both faces
+    double ue = u;
+    if (!gt_pos(h, eps)) ue = (h * u) * vfac(h, eps);  // else q vfac(h) = (h u) / h restated as u
+    const double cg = root(gh);
+    const double lo = ue - cg, hi = ue + cg;
+    const double cA = c.sqrt_g * sA, cB = c.sqrt_g * sB;
+    const double eA = uA - cA, wA = uA + cA, eB = uB - cB, wB = uB + cB;
+    // (least of values <= 0 and greatest of values >= 0: by their magnitudes)
+    auto larger = [](double x, double y) { return abs_lt(x, y) ? y : x; };
+    const double aut1 = larger(gt0(lo) ? 0.0 : lo, larger(gt0(eA) ? 0.0 : eA, gt0(eB) ? 0.0 : eB));
+    const double aut3 = larger(lt0(hi) ? 0.0 : hi, larger(lt0(wA) ? 0.0 : wA, lt0(wB) ? 0.0 : wB));
+    const double b1 = abs_bits(aut1), b3 = abs_bits(aut3);
+    double lmax = lt_pos(b3, b1) ? b1 : b3;
+    if (lt_pos(lmax, abs_bits(u))) lmax = abs_bits(u);
+    const double d13 = aut1 - aut3;
+    // IFCP coefficients.  Subcritical average (its middle eigenvalues 0), waves
+    // to both sides: aut3 |aut1| - aut1 |aut3| is -2 p for the rounded product p
+    // = aut1 aut3 (the fma's sum -2 p + (p - exact) is within half an ulp of
+    // -2 p), and the middle gaps are aut1 and -aut3.
+    double n0, n1;
+    bool wide;
+    const bool sub = !gt0(lo) && !lt0(hi) && lt0(aut1) && gt0(aut3) && !lt_pos(b1, 0x1p-400) && !lt_pos(b3, 0x1p-400);
+    if (warp_all(sub)) {
+        lshm::rare();
+        n0 = lshm::neg_if(twice(aut1 * aut3), true);
+        n1 = aut3 + aut1;
+        wide = !lt_pos(b1, kEps) && !lt_pos(b3, kEps);
+    } else {
+        lshm::rare();
+        double aut2 = gt0(lo) ? lo : (lt0(hi) ? abs_bits(hi) : 0.0);
+        aut2 = lshm::neg_if(aut2, sgn(aut1 + aut3) < 0);
+        n0 = fmad(aut3, b1, -(aut1 * b3));
+        n1 = b3 - b1;
+        wide = !abs_lt(aut1 - aut2, kEps) && !abs_lt(aut2 - aut3, kEps);
+    }
+    double a0 = lmax, a1 = 0.0;
+    if (wide && !abs_lt(d13, kEps)) {
+        const double inv = rcp(lshm::neg_if(d13, true));  // 1 / (aut3 - aut1)
+        a0 = n0 * inv;
+        a1 = n1 * inv;
+    }
+
+    const double FA = lt_pos(A.h1, kEps) ? 0.0 : uA * Aq, FB = lt_pos(B.h1, kEps) ? 0.0 : uB * Bq;
+    const double dF = Bq - Aq;
+    const double tx = plus0(dF), ty = gh * deta + (FB - FA);
+    const double half_x = half(tx), half_y = half(ty);
+    const double Qx = half(fmad(a0, deta, a1 * tx));
+    const double Qy = half(fmad(a0, dF, a1 * ty));
+    const double Fm = half_x + (Aq - Qx);
+    const bool out = gt0(Fm);
+    const double ut = abs_lt(Fm, kEps) ? 0.0 : (out ? fA : fB) * (out ? A.qt1 : B.qt1);
+    o.m[0] = len * Fm;
+    o.m[1] = len * (half_y + (FA - Qy));
+    o.m[2] = len * (Fm * ut);
+    o.p[0] = len * (half_x + (Qx - Bq));
+    o.p[1] = len * (half_y + (Qy - FB));
+    o.m[3] = o.m[4] = o.m[5] = o.p[2] = o.p[3] = 0.0;
+    if (lt_pos(lmax, eps)) { lshm::rare(); lmax = lmax + eps; }
+    o.wave = len * lmax;
+}
+
+// procesarArista (Arista_kernel.cu:324-645) up to the limiter, the depths
+// already known to be wet (the caller skips dry edges, :397): both layers.
+LSH_HD void edge_raw2(const Face& A, const Face& B, double len, double dt, const Consts& c, EdgeRaw& o) {
+    const double eps = c.eps_h;
+    double Aq1 = A.qn1, Aq2 = A.qn2, Bq1 = B.qn1, Bq2 = B.qn2;
     const double Ah1 = A.h1, Bh1 = B.h1;
-    const double Ah2 = L2 ? A.h2 : 0.0, Bh2 = L2 ? B.h2 : 0.0;
+    const double Ah2 = A.h2, Bh2 = B.h2;
     const double H0 = A.H, H1 = B.H;
     const double h1ij = half(Ah1 + Bh1);
-    const double h2ij = L2 ? half(Ah2 + Bh2) : 0.0;
+    const double h2ij = half(Ah2 + Bh2);
 
     // tratamientoSecoMojado (Arista_kernel.cu:301-321): the conditions on
     // layer 1 need its depth below eps_h on one side (or a negative h2)
-    if (L2) {
+    if (lt_pos(Ah2, eps) || lt_pos(Bh2, eps)) {
+        lshm::rare();
         if (lt_pos(Ah2, eps) && lt(H0, H1 - Bh2)) Bq2 = 0.0;
         if (lt_pos(Bh2, eps) && lt(H1, H0 - Ah2)) Aq2 = 0.0;
-        if (lt_pos(Ah1, eps) || lt_pos(Bh1, eps) || lt0(Ah2) || lt0(Bh2)) {
-            if (lt_pos(Ah1, eps) && lt(H0 - Ah2, H1 - Bh1 - Bh2)) Bq1 = 0.0;
-            if (lt_pos(Bh1, eps) && lt(H1 - Bh2, H0 - Ah1 - Ah2)) Aq1 = 0.0;
-            if (lt_pos(Ah2 + Ah1, eps) && lt(H0, H1 - Bh1 - Bh2)) { Bq1 = 0.0; Bq2 = 0.0; }
-            if (lt_pos(Bh2 + Bh1, eps) && lt(H1, H0 - Ah1 - Ah2)) { Aq1 = 0.0; Aq2 = 0.0; }
-        }
-    } else if (lt_pos(Ah1, eps) || lt_pos(Bh1, eps)) {
-        if (lt_pos(Ah1, eps) && lt(H0, H1 - Bh1)) Bq1 = 0.0;
-        if (lt_pos(Bh1, eps) && lt(H1, H0 - Ah1)) Aq1 = 0.0;
+    }
+    if (lt_pos(Ah1, eps) || lt_pos(Bh1, eps) || lt0(Ah2) || lt0(Bh2)) {
+        lshm::rare();
+        if (lt_pos(Ah1, eps) && lt(H0 - Ah2, H1 - Bh1 - Bh2)) Bq1 = 0.0;
+        if (lt_pos(Bh1, eps) && lt(H1 - Bh2, H0 - Ah1 - Ah2)) Aq1 = 0.0;
+        if (lt_pos(Ah2 + Ah1, eps) && lt(H0, H1 - Bh1 - Bh2)) { Bq1 = 0.0; Bq2 = 0.0; }
+        if (lt_pos(Bh2 + Bh1, eps) && lt(H1, H0 - Ah1 - Ah2)) { Aq1 = 0.0; Aq2 = 0.0; }
     }
 
     const double fA1 = vfac(Ah1, eps), fB1 = vfac(Bh1, eps);
     const double sa1 = root(Ah1), sb1 = root(Bh1);
     const double uA1 = fA1 * Aq1, uB1 = fB1 * Bq1;
     const double u1ij = div(fmad(sa1, uA1, sb1 * uB1), sa1 + sb1 + kEps);
-    double u2ij = 0.0, uA2 = 0.0, uB2 = 0.0, fA2 = 0.0, fB2 = 0.0;
-    if (L2) {
-        fA2 = vfac(Ah2, eps);
-        fB2 = vfac(Bh2, eps);
-        const double sa2 = root(Ah2), sb2 = root(Bh2);
-        uA2 = fA2 * Aq2;
-        uB2 = fB2 * Bq2;
-        u2ij = div(fmad(sa2, uA2, sb2 * uB2), sa2 + sb2 + kEps);
-    }
+    const double fA2 = vfac(Ah2, eps), fB2 = vfac(Bh2, eps);
+    const double sa2 = root(Ah2), sb2 = root(Bh2);
+    const double uA2 = fA2 * Aq2, uB2 = fB2 * Bq2;
+    const double u2ij = div(fmad(sa2, uA2, sb2 * uB2), sa2 + sb2 + kEps);
     // a face's celerity sqrt(g h) is sqrt(g) sqrt(h1) when its granular layer is empty
-    const bool oneA = !L2 || is_zero(Ah2), oneB = !L2 || is_zero(Bh2);
+    const bool oneA = is_zero(Ah2), oneB = is_zero(Bh2);
 
     const double Hm = tmin(H0, H1);
-    const double deta1 = L2 ? max0(Bh1 + Bh2 - H1 + Hm) - max0(Ah1 + Ah2 - H0 + Hm)
-                            : max0(Bh1 - H1 + Hm) - max0(Ah1 - H0 + Hm);
-    const double deta2 = L2 ? max0(Bh2 - H1 + Hm) - max0(Ah2 - H0 + Hm) : 0.0;
-    const double gh1 = c.g * h1ij, gh2 = L2 ? c.g * h2ij : 0.0;
-    const double p1 = gh1 * deta1;                                            // pressure terms
-    const double p2 = L2 ? gh2 * fmad(c.omr, deta2, c.r * deta1) : 0.0;
+    const double deta1 = max0(Bh1 + Bh2 - H1 + Hm) - max0(Ah1 + Ah2 - H0 + Hm);
+    const double deta2 = max0(Bh2 - H1 + Hm) - max0(Ah2 - H0 + Hm);
+    const double gh1 = c.g * h1ij, gh2 = c.g * h2ij;
+    // pressure terms, and layer 2's below the Coulomb threshold
+    const double p1 = gh1 * deta1;
+    const double p2 = gh2 * fmad(c.omr, deta2, c.r * deta1);
+    const double mu = friction_mu(h1ij, u1ij, h2ij, u2ij, c);
+    const double sc = ((fsc_of(h1ij, c) * mu) * c.g) * h2ij;
+    const bool coul = lt_pos(abs_bits(h2ij * u2ij), (c.peso * sc) * dt);
+    const double p2c = coul ? (gh2 * c.r) * deta1 : p2;
 
-    bool coul = false;
-    double p2c = p2;
-    if (L2) {
-        const double mu = friction_mu(h1ij, u1ij, h2ij, u2ij, c);
-        const double sc = ((fsc_of(h1ij, c) * mu) * c.g) * h2ij;
-        coul = lt(abs_bits(h2ij * u2ij), (c.peso * sc) * dt);
-        if (coul) p2c = (gh2 * c.r) * deta1;
-    }
-
-    const EigBounds D = eig_edge<L2>(h1ij, h2ij, u1ij, u2ij, L2 ? fmad(h1ij, u1ij, h2ij * u2ij) : h1ij * u1ij, c, -1.0, -1.0, true);
-    const EigBounds E0 = eig_edge<L2>(Ah1, Ah2, uA1, uA2, L2 ? Aq1 + Aq2 : Aq1, c, fA1, oneA ? sa1 : -1.0);
-    const EigBounds E1 = eig_edge<L2>(Bh1, Bh2, uB1, uB2, L2 ? Bq1 + Bq2 : Bq1, c, fB1, oneB ? sb1 : -1.0);
+    const EigBounds D = eig_edge(h1ij, h2ij, u1ij, u2ij, fmad(h1ij, u1ij, h2ij * u2ij), c, -1.0, true);
+    const EigBounds E0 = eig_edge(Ah1, Ah2, uA1, uA2, Aq1 + Aq2, c, oneA ? sa1 : -1.0);
+    const EigBounds E1 = eig_edge(Bh1, Bh2, uB1, uB2, Bq1 + Bq2, c, oneB ? sb1 : -1.0);
     const double aut1 = tmin(D.lo, tmin(E0.lo, E1.lo));
     const double aut3 = tmax(D.hi, tmax(E0.hi, E1.hi));
     const double b1 = abs_bits(aut1), b3 = abs_bits(aut3);
-    double lmax = tmax(b3, b1);
-    const double umax = L2 ? tmax(abs_bits(u1ij), abs_bits(u2ij)) : abs_bits(u1ij);
-    if (lt(lmax, umax)) lmax = umax;
-    double aut2 = D.mid;
-    double d12 = aut1, d23 = minus0(aut3);  // aut1 - aut2, aut2 - aut3 with aut2 = 0
-    if (L2 || !is_zero(aut2)) {
-        aut2 = lshm::neg_if(aut2, sgn(aut1 + aut3) < 0);
-        d12 = aut1 - aut2;
-        d23 = aut2 - aut3;
-    }
-    const double d13 = aut1 - aut3;
+    double lmax = lt_pos(b3, b1) ? b1 : b3;
+    if (lt_pos(lmax, abs_bits(u1ij))) lmax = abs_bits(u1ij);
+    if (lt_pos(lmax, abs_bits(u2ij))) lmax = abs_bits(u2ij);
+    const double aut2 = lshm::neg_if(D.mid, sgn(aut1 + aut3) < 0);
+    const double d12 = aut1 - aut2, d13 = aut1 - aut3, d23 = aut2 - aut3;
 
     double a0, a1, a2 = 0.0;
     if (!abs_lt(d13, kEps) && !abs_lt(d12, kEps) && !abs_lt(d23, kEps)) {
-        if (L2 && !lt_pos(h1ij, eps) && !lt_pos(h2ij, eps)) {
+        if (!lt_pos(h1ij, eps) && !lt_pos(h2ij, eps)) {
             const double inv = rcp((d12 * d13) * d23);
             const double a = (b1 * d23) * inv;
             const double b = -((abs_bits(aut2) * d13) * inv);
@@ -401,43 +475,31 @@ LSH_HD void edge_raw(const Face& A, const Face& B, double len, double dt, const 
     const double tx = plus0(dFx), ty = p1 + dFy;
     const double half_x = half(tx), half_y = half(ty);  // dF + pressure is ty with the terms exchanged
 
-    double Ix = deta1;
-    if (L2 && !coul && gt_pos(Ah1, eps) && gt_pos(Bh1, eps)) Ix = Ix - deta2;
-    // deta2 is 0 without a granular layer: x - 0 is x
-
-    double Qx, Qy;
-    if (L2) {
-        const double dFz = Bq2 - Aq2;
-        const double tz = plus0(dFz);
-        const double FAw = lt_pos(Ah2, kEps) ? 0.0 : uA2 * Aq2, FBw = lt_pos(Bh2, kEps) ? 0.0 : uB2 * Bq2;
-        const double dFw = FBw - FAw;
-        const double tw = p2c + dFw;
-        const double Atx = ty;
-        const double Aty = fmad(gh1, tz, fmad(u1ij + u1ij, ty, fmad(-u1ij, u1ij, gh1) * tx));
-        Qx = half(fmad(a0, Ix, fmad(a1, tx, a2 * Atx)));
-        Qy = half(fmad(a0, dFx, fmad(a1, ty, a2 * Aty)));
-        const double Iz = coul ? 0.0 : deta2;
-        const double Atz = tw;
-        const double Atw = fmad(c.r * gh2, tx, fmad(fmad(-u2ij, u2ij, gh2), tz, (u2ij + u2ij) * tw));
-        const double Qz = half(fmad(a0, Iz, fmad(a1, tz, a2 * Atz)));
-        const double Qw = half(fmad(a0, dFz, fmad(a1, tw, a2 * Atw)));
-        const double half_z = half(tz), half_w = half(dFw + p2);
-        const double Fmz = half_z + (Aq2 - Qz), Fmw = half_w + (FAw - Qw);
-        const double Fpz = half_z + (Qz - Bq2), Fpw = half_w + (Qw - FBw);
-        const double u2t = abs_lt(Fmz, kEps) ? 0.0 : (gt0(Fmz) ? fA2 * A.qt2 : fB2 * B.qt2);
-        o.m[3] = len * Fmz; o.m[4] = len * Fmw; o.m[5] = len * (Fmz * u2t);
-        o.p[2] = len * Fpz; o.p[3] = len * Fpw;
-    } else {
-        Qx = half(fmad(a0, Ix, a1 * tx));
-        Qy = half(fmad(a0, dFx, a1 * ty));
-        o.m[3] = o.m[4] = o.m[5] = o.p[2] = o.p[3] = 0.0;
-    }
+    const double Ix = (!coul && gt_pos(Ah1, eps) && gt_pos(Bh1, eps)) ? deta1 - deta2 : deta1;
+    const double dFz = Bq2 - Aq2;
+    const double tz = plus0(dFz);
+    const double FAw = lt_pos(Ah2, kEps) ? 0.0 : uA2 * Aq2, FBw = lt_pos(Bh2, kEps) ? 0.0 : uB2 * Bq2;
+    const double dFw = FBw - FAw;
+    const double tw = p2c + dFw;
+    const double Aty = fmad(gh1, tz, fmad(u1ij + u1ij, ty, fmad(-u1ij, u1ij, gh1) * tx));
+    const double Qx = half(fmad(a0, Ix, fmad(a1, tx, a2 * ty)));
+    const double Qy = half(fmad(a0, dFx, fmad(a1, ty, a2 * Aty)));
+    const double Iz = coul ? 0.0 : deta2;
+    const double Atw = fmad(c.r * gh2, tx, fmad(fmad(-u2ij, u2ij, gh2), tz, (u2ij + u2ij) * tw));
+    const double Qz = half(fmad(a0, Iz, fmad(a1, tz, a2 * tw)));
+    const double Qw = half(fmad(a0, dFz, fmad(a1, tw, a2 * Atw)));
+    const double half_z = half(tz), half_w = half(dFw + p2);
+    const double Fmz = half_z + (Aq2 - Qz), Fmw = half_w + (FAw - Qw);
+    const double Fpz = half_z + (Qz - Bq2), Fpw = half_w + (Qw - FBw);
+    const double u2t = abs_lt(Fmz, kEps) ? 0.0 : (gt0(Fmz) ? fA2 * A.qt2 : fB2 * B.qt2);
+    o.m[3] = len * Fmz; o.m[4] = len * Fmw; o.m[5] = len * (Fmz * u2t);
+    o.p[2] = len * Fpz; o.p[3] = len * Fpw;
     const double Fmx = half_x + (Aq1 - Qx), Fmy = half_y + (FAy - Qy);
     const double Fpx = half_x + (Qx - Bq1), Fpy = half_y + (Qy - FBy);
     const double u1t = abs_lt(Fmx, kEps) ? 0.0 : (gt0(Fmx) ? fA1 * A.qt1 : fB1 * B.qt1);
     o.m[0] = len * Fmx; o.m[1] = len * Fmy; o.m[2] = len * (Fmx * u1t);
     o.p[0] = len * Fpx; o.p[1] = len * Fpy;
-    if (lt_pos(lmax, eps)) lmax = lmax + eps;
+    if (lt_pos(lmax, eps)) { lshm::rare(); lmax = lmax + eps; }
     o.wave = len * lmax;
 }
 
@@ -489,7 +551,8 @@ LSH_HD bool far_from_empty(double out, double h, double area, double dt, double 
 template <bool L2, class Pos>
 LSH_HD void edge_flux(const EdgeIn& e, double dt, const Consts& c, EdgeOut& o, const Pos& pos) {
     EdgeRaw w;
-    edge_raw<L2>(e.A, e.B, e.len, dt, c, w);
+    if (L2) edge_raw2(e.A, e.B, e.len, dt, c, w);
+    else edge_raw1(e.A, e.B, e.len, c, w);
     o.wave = w.wave;
 #pragma unroll
     for (int l = 0; l < 2; ++l) {
@@ -531,7 +594,7 @@ LSH_HD double edge_initial_wave(const Face& A, const Face& B, double len, const 
     const double fA2 = vfac(A.h2, eps), fB2 = vfac(B.h2, eps);
     sa = root(A.h2); sb = root(B.h2);
     const double u2ij = div(fmad(sa, fA2 * A.qn2, sb * (fB2 * B.qn2)), sa + sb + kEps);
-    const EigBounds D = eig_edge<true>(h1ij, h2ij, u1ij, u2ij, fmad(h1ij, u1ij, h2ij * u2ij), c);
+    const EigBounds D = eig_edge(h1ij, h2ij, u1ij, u2ij, fmad(h1ij, u1ij, h2ij * u2ij), c);
     double lmax = tmax(D.lo, D.hi);
     const double b = tmax(abs_bits(u1ij), abs_bits(u2ij));
     if (lt(lmax, b)) lmax = b;

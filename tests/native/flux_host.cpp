@@ -80,8 +80,8 @@ unsigned long long stage(Grid& g, int st, bool flux, double dt, long long* marke
     if (ORDER == 2) for (size_t id = 0; id < g.N; ++id) recon_cell(a, int(id));
     unsigned long long r = 0;
     if (flux) {
-        for (int y = 0; y <= ny; ++y) for (int x = 0; x < nx; ++x) flux_edge<0, ORDER>(a, x, y, dt);
-        for (int y = 0; y < ny; ++y) for (int x = 0; x <= nx; ++x) flux_edge<1, ORDER>(a, x, y, dt);
+        for (int y = 0; y <= ny; ++y) for (int x = 0; x < nx; ++x) flux_edge<ORDER>(a, 0, x, y, dt);
+        for (int y = 0; y < ny; ++y) for (int x = 0; x <= nx; ++x) flux_edge<ORDER>(a, 1, x, y, dt);
         for (size_t id = 0; id < g.N; ++id) *marked += (g.mark[id] == stage_mark(a)) + (g.mark2[id] == stage_mark(a));
         for (int j = 0; j < ny; ++j) for (int i = 0; i < nx; ++i) { bool busy = false; const unsigned long long b = update_cell<MODE>(a, i, j, dt, busy); r = b > r ? b : r; }
     } else {
