@@ -36,9 +36,12 @@
 
 namespace lshm {
 
+// (a PTX move, as halves below: opaque to the compiler)
 LSH_HD uint64_t bits_of(double x) {
 #if defined(__CUDA_ARCH__)
-    return (uint64_t)__double_as_longlong(x);
+    uint64_t u;
+    asm("mov.b64 %0, %1;" : "=l"(u) : "d"(x));
+    return u;
 #else
     uint64_t u;
     std::memcpy(&u, &x, sizeof(u));

@@ -285,16 +285,18 @@ __global__ void LSH_CELL_BOUNDS k_volume(KArgs a, Dep d = Dep{}) {
 
 
 // Advance the device clock: t += dt, dt = min per-cell dt (ShallowWater.cu:436-442).
+// One read and one write of the record: its loads do not wait for each other.
 __device__ __forceinline__ void advance_clock(TimeRec* tm, double two_cfl) {
-    if (tm->done) return;
-    tm->t += tm->dt;
-    tm->steps += 1;
-    const double nd = lsh::dt_of(tm->rmax_bits, two_cfl);
-    tm->dt = nd;
-    tm->rmax_bits = kRateInitBits;
-    if (tm->t >= tm->t_end) tm->done = 1;
-    if (tm->dt_min > 0.0 && nd < tm->dt_min) { tm->err |= 1 << LSH_ERR_STALL; tm->done = 1; }
-    if (tm->err) tm->done = 1;
+    TimeRec r = *tm;
+    if (r.done) return;
+    r.t += r.dt;
+    r.steps += 1;
+    r.dt = lsh::dt_of(r.rmax_bits, two_cfl);
+    r.rmax_bits = kRateInitBits;
+    if (r.t >= r.t_end) r.done = 1;
+    if (r.dt_min > 0.0 && r.dt < r.dt_min) { r.err |= 1 << LSH_ERR_STALL; r.done = 1; }
+    if (r.err) r.done = 1;
+    *tm = r;
 }
 
 // The clock of a step of colour passes.  With `ctr`, its threads also zero the
@@ -393,15 +395,22 @@ __global__ void __launch_bounds__(kCellBlock) k_init_eta(KArgs a) {
 // and depths up to two cells away, the stencil one cell).
 constexpr int kTileX = 16, kTileY = 4;
 constexpr int kCellWarps = 2, kFluxWarps = 4, kFluxParts = 4;  // warps per tile, and launches of the flux pass
-#ifndef LSH_FLUX_MINB
-#define LSH_FLUX_MINB 8
+// Resident blocks per SM that the kernels are compiled for, [large grid, small
+// grid].  A large grid wants the warps: flux pass in blocks of 128 threads, 4 /
+// 6 / 8 / 10 (128 / 80 / 64 / 48 registers) ran the 1024^2 wet shelf's step in
+// 916 / 852 / 872 / 975 us; the update in blocks of 64, 8 / 12 / 16 / 20: 975 /
+// 902 / 876 / 886; the reconstruction 24 / 32: no difference.  A small one has
+// one or two warps per SM, and wants no spills: 2, 4 and 8 blocks took the 64^2
+// fjord's step from 179 to 160 us, the 200^2 shelf's from 72 to 66.
+constexpr int kFluxBlocks[2] = {6, 2}, kUpdateBlocks[2] = {16, 4}, kSlopesBlocks[2] = {32, 8};
+// Tiles up to which a grid is small.  All-wet shelves, large against small
+// kernels, us per step: 400^2 (2626 tiles) 232 / 206 at second order, 96 / 96 at
+// first; 512^2 (4257) 271 / 283 and 113 / 120.  Grids with dry land gain longer
+// (fjord 523^2 234 / 219, 800^2 263 / 247), but only the step knows how much is dry.
+#ifndef LSH_SMALL_TILES
+#define LSH_SMALL_TILES 4000
 #endif
-#ifndef LSH_UPDATE_MINB
-#define LSH_UPDATE_MINB 20
-#endif
-#ifndef LSH_SLOPES_MINB
-#define LSH_SLOPES_MINB 32
-#endif
+constexpr unsigned kSmallTiles = LSH_SMALL_TILES;
 
 inline __host__ __device__ int tiles_x(int nx) { return (nx + 1 + kTileX - 1) / kTileX; }
 inline __host__ __device__ int tiles_y(int ny) { return (ny + 1 + kTileY - 1) / kTileY; }
@@ -478,8 +487,8 @@ __device__ __forceinline__ void warp_max_bits(unsigned long long v, unsigned lon
 }
 
 // Blocks first, first + 1, ... of the flux pass: one to four warps of a tile each.
-template <int ORDER>
-__global__ void __launch_bounds__(32 * kFluxWarps, LSH_FLUX_MINB)
+template <int ORDER, bool SMALL>
+__global__ void __launch_bounds__(32 * kFluxWarps, kFluxBlocks[SMALL])
     k_flux(const __grid_constant__ KArgs a, const __grid_constant__ TileMap m, TileDep d, unsigned first) {
     if (a.tm->done) return;
     const unsigned bw = blockDim.x / 32, u0 = (first + blockIdx.x) * bw;
@@ -504,8 +513,8 @@ __device__ __forceinline__ bool tile_cell(const KArgs& a, int tx, int ty, unsign
     return i < a.c.nx && j < a.c.ny;
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(32 * kCellWarps, LSH_UPDATE_MINB)
+template <int MODE, bool SMALL>
+__global__ void __launch_bounds__(32 * kCellWarps, kUpdateBlocks[SMALL])
     k_update(const __grid_constant__ KArgs a, const __grid_constant__ TileMap m, TileDep d) {
     if (a.tm->done) return;
     const unsigned u0 = blockIdx.x * (blockDim.x / 32);
@@ -524,7 +533,8 @@ __global__ void __launch_bounds__(32 * kCellWarps, LSH_UPDATE_MINB)
     tile_end(d, ty);
 }
 
-__global__ void __launch_bounds__(32 * kCellWarps, LSH_SLOPES_MINB)
+template <bool SMALL>
+__global__ void __launch_bounds__(32 * kCellWarps, kSlopesBlocks[SMALL])
     k_slopes(const __grid_constant__ KArgs a, const __grid_constant__ TileMap m, TileDep d) {
     if (a.tm->done) return;
     const unsigned u0 = blockIdx.x * (blockDim.x / 32);
@@ -546,13 +556,17 @@ __global__ void __launch_bounds__(256) k_clock(TimeRec* tm, double two_cfl, unsi
         for (int c0 = 0; c0 < m.ntx; c0 += 32) {
             const int c = c0 + lane;
             unsigned v = 0;
-            if (c < m.ntx) {
-                for (int y = max(r - 2, 0); y <= min(r + 2, m.nty - 1); ++y)
-                    for (int x = max(c - 2, 0); x <= min(c + 2, m.ntx - 1); ++x) {
-                        const size_t t = (size_t)y * m.ntx + x;
-                        v |= m.busy[0][t] | m.busy[1][t];
-                    }
-            }
+            // the window's 50 loads at once (a loop over its part inside the
+            // grid waited for each: 6 us on any grid)
+#pragma unroll
+            for (int dy = -2; dy <= 2; ++dy)
+#pragma unroll
+                for (int dx = -2; dx <= 2; ++dx) {
+                    const int y = min(max(r + dy, 0), m.nty - 1), x = min(max(c + dx, 0), m.ntx - 1);
+                    const size_t t = (size_t)y * m.ntx + x;
+                    v |= (unsigned)m.busy[0][t] | (unsigned)m.busy[1][t];
+                }
+            if (c >= m.ntx) v = 0;
             const unsigned on = __ballot_sync(0xffffffffu, v != 0);
             if (v) m.list[(size_t)r * m.ntx + n + __popc(on & ((1u << lane) - 1u))] = c;
             n += __popc(on);
@@ -714,15 +728,14 @@ inline int flux_dep_stride(int ny) { return (tiles_y(ny) + 63) & ~63; }
 // (with their edge buffers).  `c` (may be null: full-grid launches one after
 // the other): flux_dep_stride counters for each pass, which the clock kernel
 // zeroes.  `mark` is called after each launch.  Returns the kernels launched.
-// A grid of few tiles takes blocks of one warp, so that every SM's FP64 unit
-// has work; a large one a tile per block.
-template <class Mark>
-inline int enqueue_flux_step(const KArgs& a1, const KArgs& a2, const TileMap& m, unsigned* c, double two_cfl,
-                             cudaStream_t s, Mark&& mark) {
+// A small grid takes blocks of one warp, so that every SM's FP64 unit has
+// work; a large one a tile per block.
+template <bool SMALL, class Mark>
+inline int enqueue_flux_step_as(const KArgs& a1, const KArgs& a2, const TileMap& m, unsigned* c, double two_cfl,
+                                cudaStream_t s, Mark&& mark) {
     const int order = a1.c.order, st = flux_dep_stride(a1.c.ny), last = flux_step_passes(order) - 1;
     const unsigned tiles = unsigned(m.ntx) * unsigned(m.nty);
-    const bool spread = tiles <= 2048;
-    const unsigned cw = spread ? 1 : kCellWarps, fw = spread ? 1 : kFluxWarps;  // warps per block
+    constexpr unsigned cw = SMALL ? 1 : kCellWarps, fw = SMALL ? 1 : kFluxWarps;  // warps per block
     const unsigned nf = tiles * (kFluxWarps / fw), nc = tiles * (kCellWarps / cw);
     TileDep d;  // the pass before as producer, this pass's own counters
     int pass = 0;
@@ -748,20 +761,27 @@ inline int enqueue_flux_step(const KArgs& a1, const KArgs& a2, const TileMap& m,
         end(kFluxWarps / fw);
     };
     if (order == 1) {
-        flux(k_flux<1>, a1);
-        cells(k_update<0>, a1);
+        flux(k_flux<1, SMALL>, a1);
+        cells(k_update<0, SMALL>, a1);
     } else {
-        cells(k_slopes, a1);
-        flux(k_flux<2>, a1);
-        cells(k_update<1>, a1);
-        cells(k_slopes, a2);
-        flux(k_flux<2>, a2);
-        cells(k_update<2>, a2);
+        cells(k_slopes<SMALL>, a1);
+        flux(k_flux<2, SMALL>, a1);
+        cells(k_update<1, SMALL>, a1);
+        cells(k_slopes<SMALL>, a2);
+        flux(k_flux<2, SMALL>, a2);
+        cells(k_update<2, SMALL>, a2);
     }
     // a plain launch: waits for the whole step, then zeroes the counters
     k_clock<<<clock_blocks(m), 256, 0, s>>>(a1.tm, two_cfl, c, c ? pass * st : 0, m);
     mark();
     return (order == 1) ? 6 : 13;
+}
+template <class Mark>
+inline int enqueue_flux_step(const KArgs& a1, const KArgs& a2, const TileMap& m, unsigned* c, double two_cfl,
+                             cudaStream_t s, Mark&& mark) {
+    return (unsigned(m.ntx) * unsigned(m.nty) <= kSmallTiles)
+               ? enqueue_flux_step_as<true>(a1, a2, m, c, two_cfl, s, mark)
+               : enqueue_flux_step_as<false>(a1, a2, m, c, two_cfl, s, mark);
 }
 
 }  // namespace

@@ -610,62 +610,87 @@ LSH_HD bool cancel(double x, double y) {
     return lshm::bits_of(x) == (lshm::bits_of(y) ^ ~lshm::kMag) || (is_zero(x) && is_zero(y));
 }
 
-// No granular layer at cell `id` and its faces: h2, q2 and, at second order,
+// A cell's state and, at second order, its slopes across an edge.
+template <int ORDER>
+struct CellSide { double w[7], s[ORDER == 2 ? 7 : 1]; bool zero; };
+template <int DIR, int ORDER>
+LSH_HD void load_side(const KArgs& a, int id, CellSide<ORDER>& c) {
+#pragma unroll
+    for (int k = 0; k < 7; ++k) c.w[k] = a.W[k][id];
+    c.zero = true;
+    if constexpr (ORDER == 2) {
+        c.zero = a.szero[id] != 0;
+#pragma unroll
+        for (int k = 0; k < 7; ++k) c.s[k] = (DIR == 0 ? a.sy : a.sx)[k][id];
+    }
+}
+
+// The face of a cell toward its +slope side (`neg`: the other one) in the edge
+// frame (face_depths, face_rest).  BARE: layer 1 alone, zeros for layer 2.
+template <int DIR, int ORDER, bool BARE>
+LSH_HD double side_depth(const CellSide<ORDER>& c, bool neg, int layer) {
+    double h = c.w[3 * layer];
+    if constexpr (ORDER == 2) h = h + lshm::neg_if(layer ? c.s[3] + c.s[6] : c.s[0] - c.s[3], neg);
+    return h;
+}
+template <int DIR, int ORDER, bool BARE>
+LSH_HD void side_rest(const CellSide<ORDER>& c, bool neg, bool pos_normal, Face& f) {
+    using lshm::neg_if;
+    double q[4] = {c.w[1], c.w[2], c.w[4], c.w[5]};
+    f.H = c.w[6];
+    if constexpr (ORDER == 2) {
+        q[0] = q[0] + neg_if(c.s[1], neg);
+        q[1] = q[1] + neg_if(c.s[2], neg);
+        if (!BARE) {
+            q[2] = q[2] + neg_if(c.s[4], neg);
+            q[3] = q[3] + neg_if(c.s[5], neg);
+        }
+        f.H = f.H + neg_if(c.s[6], neg);
+    }
+    f.qn1 = neg_if(q[1 - DIR], !pos_normal);
+    f.qt1 = neg_if(q[DIR], DIR == 1 ? !pos_normal : pos_normal);
+    if (BARE) {
+        f.h2 = f.qn2 = f.qt2 = 0.0;
+    } else {
+        f.qn2 = neg_if(q[3 - DIR], !pos_normal);
+        f.qt2 = neg_if(q[2 + DIR], DIR == 1 ? !pos_normal : pos_normal);
+    }
+}
+
+// No granular layer at the cell and its faces: h2, q2 and, at second order,
 // what their slopes add (eta2's and H's slopes cancel) are zeros.
 template <int ORDER>
-LSH_HD bool bare_cell(const KArgs& a, int id, const double* const* s) {
-    bool b = is_zero(a.W[3][id]) && is_zero(a.W[4][id]) && is_zero(a.W[5][id]);
-    if (ORDER == 2) b = b && is_zero(s[4][id]) && is_zero(s[5][id]) && cancel(s[3][id], s[6][id]);
+LSH_HD bool bare_side(const CellSide<ORDER>& c) {
+    bool b = is_zero(c.w[3]) & is_zero(c.w[4]) & is_zero(c.w[5]);
+    if constexpr (ORDER == 2) b = b & is_zero(c.s[4]) & is_zero(c.s[5]) & cancel(c.s[3], c.s[6]);
     return b;
 }
 
-// Layer 1 of a face (face_depths, face_rest) and zeros for layer 2.
-template <int DIR, int ORDER>
-LSH_HD void bare_face(const KArgs& a, int id, int side, bool pos_normal, Face& f) {
-    using lshm::neg_if;
-    const bool neg = !(side & 1);
-    double qx = a.W[1][id], qy = a.W[2][id];
-    f.H = a.W[6][id];
-    if (ORDER == 2) {
-        const double* const* s = (side < 2) ? a.sx : a.sy;
-        qx = qx + neg_if(s[1][id], neg);
-        qy = qy + neg_if(s[2][id], neg);
-        f.H = f.H + neg_if(s[6][id], neg);
-    }
-    f.qn1 = neg_if(DIR == 1 ? qx : qy, !pos_normal);
-    f.qt1 = neg_if(DIR == 1 ? qy : qx, DIR == 1 ? !pos_normal : pos_normal);
-    f.h2 = f.qn2 = f.qt2 = 0.0;
-}
-template <int ORDER>
-LSH_HD double bare_depth(const KArgs& a, int id, int side) {
-    double h = a.W[0][id];
-    if (ORDER == 2) {
-        const double* const* s = (side < 2) ? a.sx : a.sy;
-        h = h + lshm::neg_if(s[0][id] - s[3][id], !(side & 1));
-    }
-    return h;
-}
-
-// The faces of an edge and its kind.  A warp whose edges all lie between cells
+// The faces of an edge and its kind, as edge_wet and edge_faces give them.
+// Both cells' values are loaded at once, whatever the edge turns out to be: a
+// load behind a test of another costs an L2 round trip (700 cycles), which a
+// small grid's lone warps cannot hide.  A warp whose edges all lie between cells
 // without a granular layer takes their layer-1 faces alone: 10 FP64
-// instructions instead of 24 at second order, none instead of 2 at first.
+// instructions instead of 24 at second order.
 template <int DIR, int ORDER>
 LSH_HD EdgeKind flux_faces(const KArgs& a, const EdgeSides& s, Face& A, Face& B) {
-    constexpr int side1 = (DIR == 0) ? 2 : 0;
-    const double* const* sl = (DIR == 0) ? a.sy : a.sx;
-    bool empty = is_zero(a.W[0][s.id0]) && is_zero(a.W[3][s.id0]) && (ORDER == 1 || a.szero[s.id0]);
-    if (empty && s.interior)
-        empty = is_zero(a.W[0][s.id1]) && is_zero(a.W[3][s.id1]) && (ORDER == 1 || a.szero[s.id1]);
+    CellSide<ORDER> ca, cb;
+    load_side<DIR, ORDER>(a, s.id0, ca);
+    load_side<DIR, ORDER>(a, s.interior ? s.id1 : s.id0, cb);
+    // both cells empty with zero slopes (edge_wet)
+    const bool empty = is_zero(ca.w[0]) & is_zero(ca.w[3]) & ca.zero & is_zero(cb.w[0]) & is_zero(cb.w[3]) & cb.zero;
     if (empty) return kEdgeDry;
-    bool bare = bare_cell<ORDER>(a, s.id0, sl);
-    if (bare && s.interior) bare = bare_cell<ORDER>(a, s.id1, sl);
+    const bool na = !(s.side0 & 1);
+    const bool bare = bare_side<ORDER>(ca) & bare_side<ORDER>(cb);
     if (warp_all(bare)) {
-        A.h1 = bare_depth<ORDER>(a, s.id0, s.side0);
-        B.h1 = s.interior ? bare_depth<ORDER>(a, s.id1, side1) : A.h1;
+        A.h1 = side_depth<DIR, ORDER, true>(ca, na, 0);
+        B.h1 = A.h1;
+        if (s.interior) { lshm::rare(); B.h1 = side_depth<DIR, ORDER, true>(cb, true, 0); }
         if (lshm::lt_pos(half(A.h1 + B.h1), kEps)) return kEdgeDry;
-        bare_face<DIR, ORDER>(a, s.id0, s.side0, s.pos_normal, A);
+        side_rest<DIR, ORDER, true>(ca, na, s.pos_normal, A);
         if (s.interior) {
-            bare_face<DIR, ORDER>(a, s.id1, side1, s.pos_normal, B);
+            lshm::rare();
+            side_rest<DIR, ORDER, true>(cb, true, s.pos_normal, B);
         } else {
             lshm::rare();
             B = A;
@@ -673,8 +698,21 @@ LSH_HD EdgeKind flux_faces(const KArgs& a, const EdgeSides& s, Face& A, Face& B)
         }
         return kEdgeSingle;
     }
-    if (!edge_wet<DIR, ORDER>(a, s, A, B)) return kEdgeDry;
-    edge_faces<DIR, ORDER>(a, s, A, B);
+    A.h1 = side_depth<DIR, ORDER, false>(ca, na, 0);
+    A.h2 = side_depth<DIR, ORDER, false>(ca, na, 1);
+    B.h1 = s.interior ? side_depth<DIR, ORDER, false>(cb, true, 0) : A.h1;
+    B.h2 = s.interior ? side_depth<DIR, ORDER, false>(cb, true, 1) : A.h2;
+    // dry edge (Arista_kernel.cu:397)
+    if (lshm::lt_pos(half(A.h1 + B.h1), kEps) && lshm::lt_pos(half(A.h2 + B.h2), kEps)) return kEdgeDry;
+    side_rest<DIR, ORDER, false>(ca, na, s.pos_normal, A);
+    if (s.interior) {
+        side_rest<DIR, ORDER, false>(cb, true, s.pos_normal, B);
+    } else {
+        // ghost: the cell's face with the normal discharges times the boundary factor
+        B = A;
+        B.qn1 = A.qn1 * s.bor;
+        B.qn2 = A.qn2 * s.bor;
+    }
     return (is_zero(A.h2) && is_zero(B.h2) && is_zero(A.qn2) && is_zero(B.qn2)) ? kEdgeSingle : kEdgeBoth;
 }
 
@@ -752,6 +790,41 @@ LSH_HD CellEdge cell_edge(int i, int j) {
     return e;
 }
 
+// Whether all that the four edges take from layer `layer` of cell (i, j) in dt,
+// with the limiter's beta and eps, is less than its content: then, as for an
+// unmarked cell, the limiter's test is false on each of its sides.
+LSH_HD bool holds_all(const KArgs& a, int i, int j, int layer, double dt) {
+    double out = 0.0;
+    auto edge = [&](int dir, size_t at, bool second) {
+        const double v = a.eb.q[dir][at + (layer ? (second ? 9 : 6) : (second ? 3 : 0)) * a.eb.plane[dir]];
+        const bool loses = a.eb.kind[dir][at] > layer && gt0(v);
+        out = out + (loses ? v : 0.0);
+    };
+    const int nx = a.c.nx;
+    edge(0, (size_t)j * nx + i, j > 0);
+    edge(0, (size_t)(j + 1) * nx + i, false);
+    edge(1, (size_t)j * (nx + 1) + i, i > 0);
+    edge(1, (size_t)j * (nx + 1) + i + 1, false);
+    const double need = dt * fmad(a.c.beta, out, 4.0 * kEps);
+    return lt_pos(need, (a.eb.depth[layer][(size_t)j * nx + i] * a.geo.area[j]) * (1.0 - 0x1p-30));
+}
+
+// Whether the limiter may act on an edge of cell (i, j): one of the edges' cells
+// is marked and may be emptied.
+LSH_RECURSE bool limit_near(const KArgs& a, int i, int j, int layer, double dt) {
+    const unsigned now = stage_mark(a);
+    const unsigned* mk = a.eb.mark[layer];
+    const int nx = a.c.nx, ny = a.c.ny;
+    bool near = false;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const int ci = i + (k == 1) - (k == 2), cj = j + (k == 3) - (k == 4);
+        if (ci < 0 || ci >= nx || cj < 0 || cj >= ny) continue;
+        if (mk[(size_t)cj * nx + ci] == now && !holds_all(a, ci, cj, layer, dt)) near = true;
+    }
+    return near;
+}
+
 // The limiter's factors on the edges of cell (i, j) before colour C, in colour
 // order (factors[0 .. C), may be null), and the mass terms that those edges
 // leave in the cell's accumulator of `layer` -- what the colour passes' limiter
@@ -779,8 +852,9 @@ LSH_HD double limited_mass(const KArgs& a, int i, int j, int layer, double dt, d
     const unsigned* mark = a.eb.mark[layer];
     if (!(mark[s.id0] == now || (s.interior && mark[s.id1] == now))) return own;
     if (!gt0(m) && !(s.interior && gt0(p))) return own;
+    // the limiter reads the partial sum of a cell that loses: mostly one of the two
     double other = 0.0;
-    if (s.interior) {
+    if (s.interior && gt0(e.second ? m : p)) {
         const int io = e.second ? s.id0 - s.row0 * a.c.nx : s.id1 - s.row1 * a.c.nx;
         other = partial_mass<P>(a, io, e.second ? s.row0 : s.row1, layer, dt, nullptr);
     }
@@ -800,12 +874,14 @@ LSH_RECURSE double partial_mass(const KArgs& a, int i, int j, int layer, double 
 }
 
 // Subtracts the colour-C edge's terms from the cell's accumulators (the first
-// colour writes them), as do_edge's scatter does.  LIMIT: with the limiter's
-// factors f1, f2 of the layers' edges by colour (null: all 1).
+// colour writes them), as do_edge's scatter does.  A dry edge's planes are
+// loaded like the others', so that no load waits for the kinds, and taken as
+// +0: an accumulator never holds -0, so subtracting zeros leaves its bits.
+// LIMIT: with the limiter's factors f1, f2 of the layers' edges by colour (null:
+// all 1).
 template <int C, bool LIMIT>
 LSH_HD void add_edge(const KArgs& a, int i, int j, int kind, const double* f1, const double* f2, double acc[7]) {
     constexpr int DIR = C / 2;
-    if (kind == kEdgeDry) return;
     const CellEdge e = cell_edge<C>(i, j);
     const size_t at = (size_t)e.y * (a.c.nx + DIR) + e.x, np = a.eb.plane[DIR];
     const double* q = a.eb.q[DIR] + at;
@@ -819,14 +895,15 @@ LSH_HD void add_edge(const KArgs& a, int i, int j, int kind, const double* f1, c
         if (C == 0) { acc[k] = minus0(v0); acc[k + 1] = minus0(dx); acc[k + 2] = minus0(dy); }
         else { acc[k] = acc[k] - v0; acc[k + 1] = acc[k + 1] - dx; acc[k + 2] = acc[k + 2] - dy; }
     };
+    const bool wet = (kind != kEdgeDry);
+    const double q0 = q[(e.second ? 3 : 0) * np], q1 = q[(e.second ? 4 : 1) * np], q2 = q[2 * np], w = q[5 * np];
     // the second cell's tangential momentum is the first's, negated
-    take(0, f1, q[(e.second ? 3 : 0) * np], q[(e.second ? 4 : 1) * np], lshm::neg_if(q[2 * np], e.second));
+    take(0, f1, wet ? q0 : 0.0, wet ? q1 : 0.0, wet ? lshm::neg_if(q2, e.second) : 0.0);
     if (kind == kEdgeBoth) {
         lshm::rare();
         take(1, f2, q[(e.second ? 9 : 6) * np], q[(e.second ? 10 : 7) * np], lshm::neg_if(q[8 * np], e.second));
     }
-    const double w = q[5 * np];
-    acc[6] = (C == 0) ? plus0(w) : acc[6] + w;
+    acc[6] = (C == 0) ? (wet ? plus0(w) : 0.0) : acc[6] + (wet ? w : 0.0);
 }
 
 // One cell of the Euler-stage update after the flux pass (MODE as volume_finish).
@@ -838,46 +915,43 @@ LSH_HD unsigned long long update_cell(const KArgs& a, int i, int j, double dt, b
     const unsigned char* kh = a.eb.kind[0] + id;
     const unsigned char* kv = a.eb.kind[1] + (size_t)j * (nx + 1) + i;
     const int kb = kh[0], kt = kh[nx], kl = kv[0], kr = kv[1], any = kb | kt | kl | kr;
+    const int k0 = (j & 1) ? kt : kb, k1 = (j & 1) ? kb : kt, k2 = (i & 1) ? kr : kl, k3 = (i & 1) ? kl : kr;
     busy |= (any != 0);
-    // an edge is limited only where one of its two cells is marked
-    bool limit[2] = {false, false};
-    double f[8];
-    if (any) {
-        const unsigned now = stage_mark(a);
-#pragma unroll
-        for (int l = 0; l < 2; ++l) {
-            if (l == 1 && !(any & kEdgeBoth)) break;
-            const unsigned* mk = a.eb.mark[l] + id;
-            bool m = (mk[0] == now);
-            if (j > 0) m |= (mk[-nx] == now);
-            if (j < ny - 1) m |= (mk[nx] == now);
-            if (i > 0) m |= (mk[-1] == now);
-            if (i < nx - 1) m |= (mk[1] == now);
-            limit[l] = m;
-        }
-        if (limit[0]) partial_mass<4>(a, i, j, 0, dt, f);
-        if (limit[1]) partial_mass<4>(a, i, j, 1, dt, f + 4);
-    }
     double wo[6], acc[7];
 #pragma unroll
     for (int k = 0; k < 6; ++k) wo[k] = a.W[k][id];
 #pragma unroll
-    for (int k = 0; k < 7; ++k) acc[k] = 0.0;
-    if (any) {
-        const int k0 = (j & 1) ? kt : kb, k1 = (j & 1) ? kb : kt, k2 = (i & 1) ? kr : kl, k3 = (i & 1) ? kl : kr;
-        if (warp_any(limit[0] || limit[1])) {
-            const double* f1 = limit[0] ? f : nullptr;
-            const double* f2 = limit[1] ? f + 4 : nullptr;
-            add_edge<0, true>(a, i, j, k0, f1, f2, acc);
-            add_edge<1, true>(a, i, j, k1, f1, f2, acc);
-            add_edge<2, true>(a, i, j, k2, f1, f2, acc);
-            add_edge<3, true>(a, i, j, k3, f1, f2, acc);
-        } else {
-            add_edge<0, false>(a, i, j, k0, nullptr, nullptr, acc);
-            add_edge<1, false>(a, i, j, k1, nullptr, nullptr, acc);
-            add_edge<2, false>(a, i, j, k2, nullptr, nullptr, acc);
-            add_edge<3, false>(a, i, j, k3, nullptr, nullptr, acc);
-        }
+    for (int k = 3; k < 6; ++k) acc[k] = 0.0;
+    // an edge is limited only where one of its two cells is marked
+    bool limit[2];
+    const unsigned now = stage_mark(a);
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+        const unsigned* mk = a.eb.mark[l] + id;
+        limit[l] = (mk[0] == now) | (mk[j > 0 ? -nx : 0] == now) | (mk[j < ny - 1 ? nx : 0] == now) |
+                   (mk[i > 0 ? -1 : 0] == now) | (mk[i < nx - 1 ? 1 : 0] == now);
+        if (l == 1) limit[l] = limit[l] && (any & kEdgeBoth);
+    }
+    if (warp_any(any && (limit[0] || limit[1]))) {
+        lshm::rare();
+        limit[0] = any && limit[0] && limit_near(a, i, j, 0, dt);
+        limit[1] = any && limit[1] && limit_near(a, i, j, 1, dt);
+    }
+    if (warp_any(any && (limit[0] || limit[1]))) {
+        double f[8];
+        if (limit[0]) partial_mass<4>(a, i, j, 0, dt, f);
+        if (limit[1]) partial_mass<4>(a, i, j, 1, dt, f + 4);
+        const double* f1 = limit[0] ? f : nullptr;
+        const double* f2 = limit[1] ? f + 4 : nullptr;
+        add_edge<0, true>(a, i, j, k0, f1, f2, acc);
+        add_edge<1, true>(a, i, j, k1, f1, f2, acc);
+        add_edge<2, true>(a, i, j, k2, f1, f2, acc);
+        add_edge<3, true>(a, i, j, k3, f1, f2, acc);
+    } else {
+        add_edge<0, false>(a, i, j, k0, nullptr, nullptr, acc);
+        add_edge<1, false>(a, i, j, k1, nullptr, nullptr, acc);
+        add_edge<2, false>(a, i, j, k2, nullptr, nullptr, acc);
+        add_edge<3, false>(a, i, j, k3, nullptr, nullptr, acc);
     }
     return volume_finish<MODE, true>(a, id, j, dt, wo, acc, &busy);
 }
@@ -885,7 +959,7 @@ LSH_HD unsigned long long update_cell(const KArgs& a, int i, int j, double dt, b
 // dt from the largest acc_w / area: 2 CFL / max rate, 1e30 when no cell has a wave speed
 LSH_HD double dt_of(unsigned long long rmax_bits, double two_cfl) {
     const double m = lshm::from_bits(rmax_bits);
-    return (m > 0.0) ? two_cfl / m : lsh::kBig;
+    return (m > 0.0) ? lsh::div(two_cfl, m) : lsh::kBig;
 }
 
 // One edge of the initial-dt pass (procesarAristasDeltaTInicialGPU,

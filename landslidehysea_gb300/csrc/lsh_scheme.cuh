@@ -117,9 +117,17 @@ LSH_HD double max0(double a) { return gt0(a) ? a : 0.0; }
 LSH_HD double fmad(double a, double b, double c) { return lshm::fmad(a, b, c); }
 LSH_HD double exp_neg(double x) { return lshm::exp_neg(x); }
 
+// x == +0 or -0, by bit pattern (integer pipe)
+LSH_HD bool is_zero(double x) {
+    uint32_t lo, hi;
+    lshm::halves(x, lo, hi);
+    return ((hi << 1) | lo) == 0u;
+}
+
 // sqrt(2) h / sqrt(h^4 + max(h, eps_h)^4); exactly 1/h for h > eps_h
 LSH_HD double vfac(double h, double eps_h) {
     if (gt_pos(h, eps_h)) return rcp(h);
+    if (is_zero(h)) return h;  // an empty layer: the quotient below is that zero
     const double h2 = h * h, m2 = eps_h * eps_h;
     return div(kSqrt2 * h, root(fmad(h2, h2, m2 * m2)));
 }
@@ -176,13 +184,6 @@ constexpr int32_t kLog2One = 1 << 20;
 LSH_HD double pow43(double h) { return h * lshm::cbrt_pos(h); }
 
 LSH_HD int sgn(double x) { return abs_lt(x, kEps) ? 0 : (gt0(x) ? 1 : -1); }
-
-// x == +0 or -0, by bit pattern (integer pipe)
-LSH_HD bool is_zero(double x) {
-    uint32_t lo, hi;
-    lshm::halves(x, lo, hi);
-    return ((hi << 1) | lo) == 0u;
-}
 
 // NaN or Inf, by the exponent bits (integer pipe)
 LSH_HD bool is_bad(double x) {
@@ -684,15 +685,20 @@ LSH_HD void dis_implicita(const double wo[6], double w[6], double dt, const Cons
     double u2x = f2 * w[4], u2y = f2 * w[5];
     const double fo2 = vfac(wo[3], eps);
     const double uo2x = fo2 * wo[4], uo2y = fo2 * wo[5];
-    const double dx = uo1x - uo2x, dy = uo1y - uo2y;
-    const double du = root(fmad(dx, dx, dy * dy));
     const double u2 = root(fmad(uo2x, uo2x, uo2y * uo2y));
     if (gt0(h1) && gt0(h2)) {
-        const double hmod = fmad(c.r, h1, h2);
-        const double m = gt_pos(hmod, c.eps_1r) ? hmod : c.eps_1r;
-        const double hm2 = hmod * hmod, m2 = m * m;
-        const double hh = div(hmod, root(fmad(hm2, hm2, m2 * m2)));
-        const double k12 = ((dt * kSqrt2) * hh) * (c.mfc * du);
+        // interlayer friction; without it (mfc = 0) its coefficient is +0 for
+        // any finite depths and velocities
+        double k12 = 0.0;
+        if (lshm::bits_of(c.mfc) != 0) {
+            const double dx = uo1x - uo2x, dy = uo1y - uo2y;
+            const double du = root(fmad(dx, dx, dy * dy));
+            const double hmod = fmad(c.r, h1, h2);
+            const double m = gt_pos(hmod, c.eps_1r) ? hmod : c.eps_1r;
+            const double hm2 = hmod * hmod, m2 = m * m;
+            const double hh = div(hmod, root(fmad(hm2, hm2, m2 * m2)));
+            k12 = ((dt * kSqrt2) * hh) * (c.mfc * du);
+        }
         const double c1 = k12 * h2;
         const double c2 = (k12 * c.r) * h1;
         const double c3 = div((dt * c.g_mfs2) * u2, pow43(h2) + kEps);
