@@ -271,9 +271,9 @@ int read_time(lsh_ctx* ctx) {
     return LSH_OK;
 }
 
-int set_t_end(lsh_ctx* ctx, double t_end) {
-    // update t_end and recompute `done` on the device stream (small H2D copy of two fields)
-    if (int s = read_time(ctx)) return s;
+// t_end and `done` into the device record, from the host copy that read_time
+// has just filled (a small H2D copy on the stream).
+int put_t_end(lsh_ctx* ctx, double t_end) {
     ctx->tm_host->t_end = t_end;
     ctx->tm_host->done = (ctx->tm_host->t >= t_end || ctx->tm_host->err) ? 1 : 0;
     LSH_CUDA(cudaMemcpyAsync(ctx->tm, ctx->tm_host, sizeof(TimeRec), cudaMemcpyHostToDevice, ctx->stream));
@@ -498,21 +498,26 @@ int lsh_synchronize(lsh_ctx* ctx) {
 int lsh_run_until(lsh_ctx* ctx, double t_end, long long max_steps, long long* steps_done) {
     if (!ctx) return LSH_ERR_INVALID;
     if (!ctx->has_state) { g_last_error = "lsh_set_state has not been called"; return LSH_ERR_INVALID; }
-    if (int s = set_t_end(ctx, t_end)) return s;
     if (int s = read_time(ctx)) return s;
+    if (int s = put_t_end(ctx, t_end)) return s;
     const long long start = ctx->tm_host->steps;
     int status = LSH_OK;
     while (!ctx->tm_host->done) {
         long long left = (max_steps > 0) ? max_steps - (ctx->tm_host->steps - start) : (1LL << 40);
         if (left <= 0) break;
-        const int batch = (int)std::min<long long>(left, 8 * kGraphChunk);
+        // Steps past t_end find the record done and do nothing, but are launched
+        // all the same: as many as the next step's dt needs to get there (6
+        // readings 8 steps apart on a 512^2 fjord: 47 ms with batches of 128).
+        const double need = std::ceil((t_end - ctx->tm_host->t) / ctx->tm_host->dt);
+        int batch = (int)std::min<long long>(left, 8 * kGraphChunk);
+        if (need < batch) batch = std::max(1, (int)need);
         if ((status = lsh_step(ctx, batch))) break;
         if ((status = read_time(ctx))) break;
     }
-    if (status == LSH_OK) status = err_bits_to_status(ctx->tm_host->err);
     if (steps_done) *steps_done = ctx->tm_host->steps - start;
+    if (status == LSH_OK) status = err_bits_to_status(ctx->tm_host->err);
     // step-count mode again for later lsh_step calls
-    int s2 = set_t_end(ctx, INFINITY);
+    int s2 = put_t_end(ctx, INFINITY);
     if (status == LSH_OK) status = s2;
     return status;
 }
