@@ -177,15 +177,15 @@ int lsh_get_launch_count(lsh_ctx* ctx, long long* launches);
  * *dt_io: the dt of the first step; <= 0 means "run the initial-dt pass
  * first".  On return *t_io and *dt_io hold the time and the next step's dt.
  * eta1 max is not tracked.
- * Its accumulators, per-row geometry and time record live in one file-scope
- * __device__ array sized for LSH_NOALLOC_MAX_CELLS cells and
- * LSH_NOALLOC_MAX_ROWS rows (about 3.9 MB), which every GPU that loads the
+ * Its scratch (edge fluxes or accumulators, per-row geometry, time record)
+ * lives in one file-scope __device__ array sized for LSH_NOALLOC_MAX_CELLS cells and
+ * LSH_NOALLOC_MAX_ROWS rows (about 15 MB), which every GPU that loads the
  * library holds until the process exits.  Larger grids are rejected with
  * LSH_ERR_INVALID.  The first call on a device looks that array's device
  * address up (cudaGetSymbolAddress, with that device current); make that
- * first call before any stream capture.  The accumulators are written, not
- * added to, by the step's first edge pass, and the time record is rewritten
- * by every call, so nothing left by an earlier call is read.  All calls of
+ * first call before any stream capture.  A step writes its scratch before it
+ * reads it, and the time record is rewritten by every call, so no value left by
+ * an earlier call enters a result.  All calls of
  * one process share the one array (each process has its own copy), so calls
  * that overlap on the GPU (on other streams, or from other host threads)
  * race: serialise them. */

@@ -663,28 +663,38 @@ int lsh_get_launch_count(lsh_ctx* ctx, long long* launches) {
 // ------------------------------------------------------------------ allocation-free stepping
 //
 // lsh_step_noalloc (include/lsh.h) runs the first-order step with all of its
-// scratch in the file-scope array below instead of allocated memory.  Layout
-// (doubles): 7 accumulators of LSH_NOALLOC_MAX_CELLS, then 6 per-row geometry
-// arrays of LSH_NOALLOC_MAX_ROWS + 1, then the 64-byte time record.  Host code
-// must not use the array's name as an address: the device address is looked
-// up once per device with cudaGetSymbolAddress (with that device current) and
-// passed to the kernels.
+// scratch in the file-scope array below instead of allocated memory.  Layout:
+// the 64-byte time record and the per-row geometry (7 arrays of ny + 1, written
+// by one copy per call), the wave accumulator, then either the flux pass's
+// buffers with its copy of the depths, or, for grids whose edges do not fit
+// there (more than LSH_NOALLOC_MAX_ROWS columns) and parameters the flux pass
+// does not take, the colour passes' six other accumulators.  Host code must not
+// use the array's name as an address: the device address is looked up once per
+// device with cudaGetSymbolAddress (with that device current) and passed to
+// the kernels.
 
 namespace {
 
-constexpr size_t kNaAccStride = LSH_NOALLOC_MAX_CELLS;
-constexpr size_t kNaGeoStride = LSH_NOALLOC_MAX_ROWS + 1;
-constexpr size_t kNaGeoOffset = 7 * kNaAccStride;
-constexpr size_t kNaTimeOffset = (kNaGeoOffset + 7 * kNaGeoStride + 31) & ~size_t(31);
-constexpr size_t kNaDoubles = kNaTimeOffset + sizeof(TimeRec) / sizeof(double);
+constexpr size_t kNaCells = LSH_NOALLOC_MAX_CELLS, kNaRows = LSH_NOALLOC_MAX_ROWS;
+constexpr size_t kNaHead = (sizeof(TimeRec) + 7 * (kNaRows + 1) * sizeof(double) + 255) & ~size_t(255);
+constexpr size_t kNaAccBytes = kNaCells * sizeof(double);
+// two edges per cell and one more line each way, planes and kinds; two marks
+// per cell; tile lists of the smallest tiles (unused here) and alignment; the
+// pass counters; the copy of the depths
+constexpr size_t kNaFluxBytes = 2 * (kNaCells + kNaRows) * (lsh::kEdgePlanes * sizeof(double) + 1) +
+                                kNaCells * 2 * sizeof(unsigned) + (size_t(1) << 19);
+constexpr size_t kNaCtrBytes = 2 * (kNaRows / kTileY + 64) * sizeof(unsigned);
+constexpr size_t kNaBytes = kNaHead + kNaAccBytes + kNaFluxBytes + kNaCtrBytes + 2 * kNaAccBytes + 1024;
+static_assert(kNaFluxBytes + 2 * kNaAccBytes >= 6 * kNaAccBytes, "room for the colour passes' accumulators");
 
-__device__ __align__(256) double g_noalloc_scratch[kNaDoubles];
+__device__ __align__(256) unsigned char g_noalloc_scratch[kNaBytes];
 
 constexpr int kNaMaxDevices = 64;
-double* g_noalloc_base[kNaMaxDevices] = {};
+unsigned char* g_noalloc_base[kNaMaxDevices] = {};
 std::mutex g_noalloc_mu;
-// host-side geometry staging for the upload (no heap allocation per call)
-double g_noalloc_geo_host[7 * kNaGeoStride];
+// host-side staging of the time record and the geometry (no heap allocation per call)
+alignas(64) unsigned char g_noalloc_head_host[kNaHead];
+unsigned g_noalloc_stage = 0;  // the calls' steps so far, as the marks count them (EdgeBuf::stage)
 
 // Move the running min of per-cell dt into dt (initial-dt pass of a no-alloc call).
 __global__ void k_noalloc_take_dt(TimeRec* tm, double two_cfl) {
@@ -711,42 +721,45 @@ extern "C" int lsh_step_noalloc(const lsh_params* p, double* const dev_state[LSH
     LSH_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kNaMaxDevices) { g_last_error = "lsh_step_noalloc: device index out of range"; return LSH_ERR_INVALID; }
     if (!g_noalloc_base[dev]) {
-        double* base = nullptr;
+        unsigned char* base = nullptr;
         cudaError_t e = cudaGetSymbolAddress(reinterpret_cast<void**>(&base), g_noalloc_scratch);
         if (e != cudaSuccess) return fail_cuda(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
         g_noalloc_base[dev] = base;
     }
-    double* base = g_noalloc_base[dev];
+    unsigned char* base = g_noalloc_base[dev];
 
-    lsh::fill_geo(*p, g_noalloc_geo_host, kNaGeoStride);
-    LSH_CUDA(cudaMemcpyAsync(base + kNaGeoOffset, g_noalloc_geo_host, 7 * kNaGeoStride * sizeof(double),
-                             cudaMemcpyHostToDevice, s));
-    TimeRec* tm = reinterpret_cast<TimeRec*>(base + kNaTimeOffset);
+    const int nx = p->nx, ny = p->ny;
+    const size_t rows = size_t(ny) + 1;
     TimeRec init{};
     init.t = *t_io;
     init.dt = *dt_io;
     init.t_end = INFINITY;
     init.dt_min = p->dt_min;
     init.rmax_bits = kRateInitBits;
-    LSH_CUDA(cudaMemcpyAsync(tm, &init, sizeof(TimeRec), cudaMemcpyHostToDevice, s));
+    std::memcpy(g_noalloc_head_host, &init, sizeof(init));
+    lsh::fill_geo(*p, reinterpret_cast<double*>(g_noalloc_head_host + sizeof(TimeRec)), rows);
+    LSH_CUDA(cudaMemcpyAsync(base, g_noalloc_head_host, sizeof(TimeRec) + 7 * rows * sizeof(double),
+                             cudaMemcpyHostToDevice, s));
+    TimeRec* tm = reinterpret_cast<TimeRec*>(base);
 
     KArgs a;
     std::memset(&a, 0, sizeof(a));
     a.c = lsh::make_consts(*p);
     a.c.track_eta = 0;
-    const double* g = base + kNaGeoOffset;
+    const double* g = reinterpret_cast<const double*>(base + sizeof(TimeRec));
     a.geo.area = g;
-    a.geo.len_v = g + kNaGeoStride;
-    a.geo.len_h = g + 2 * kNaGeoStride;
-    a.geo.tanR = g + 3 * kNaGeoStride;
-    a.geo.wx = g + 4 * kNaGeoStride;
-    a.geo.wy = g + 5 * kNaGeoStride;
-    a.geo.inv_area = g + 6 * kNaGeoStride;
-    for (int k = 0; k < 7; ++k) { a.W[k] = dev_state[k]; a.acc[k] = base + k * kNaAccStride; }
-    for (int k = 0; k < 6; ++k) a.Wout[k] = dev_state[k];
+    a.geo.len_v = g + rows;
+    a.geo.len_h = g + 2 * rows;
+    a.geo.tanR = g + 3 * rows;
+    a.geo.wx = g + 4 * rows;
+    a.geo.wy = g + 5 * rows;
+    a.geo.inv_area = g + 6 * rows;
+    double* acc = reinterpret_cast<double*>(base + kNaHead);
+    for (int k = 0; k < 7; ++k) a.W[k] = dev_state[k];
+    a.acc[6] = acc;
+    for (int k = 0; k < 6; ++k) { a.acc[k] = acc + (k + 1) * kNaCells; a.Wout[k] = dev_state[k]; }
     a.tm = tm;
 
-    const int nx = p->nx, ny = p->ny;
     const dim3 nbc = cell_grid(nx, ny);
     if (!(*dt_io > 0.0)) {
         // initial dt (ShallowWater.cu:236-257) into the time record
@@ -754,15 +767,31 @@ extern "C" int lsh_step_noalloc(const lsh_params* p, double* const dev_state[LSH
         k_cell_dt<<<nbc, cell_block(), 0, s>>>(a);
         k_noalloc_take_dt<<<1, 1, 0, s>>>(tm, 2.0 * p->cfl);
     }
-    const dim3 gh0 = edge_grid_h(nx, ny, 0), gh1 = edge_grid_h(nx, ny, 1);
-    const dim3 gv0 = edge_grid_v(nx, ny, 0), gv1 = edge_grid_v(nx, ny, 1);
-    for (int i = 0; i < nsteps; ++i) {
-        k_edges_h<true, 1><<<gh0, edge_block_h(), 0, s>>>(a, 0);
-        k_edges_h<false, 1><<<gh1, edge_block_h(), 0, s>>>(a, 1);
-        k_edges_v<1><<<gv0, edge_block_v(), 0, s>>>(a, 0);
-        k_edges_v<1><<<gv1, edge_block_v(), 0, s>>>(a, 1);
-        k_volume<0><<<nbc, cell_block(), 0, s>>>(a);
-        k_advance<<<1, 1, 0, s>>>(tm, 2.0 * p->cfl);
+    FluxMem fm;
+    if (lsh::flux_fits(*p) && fm.layout(nullptr, nx, ny) <= kNaFluxBytes) {
+        // every tile, with the passes overlapped; the counters are zero at load
+        // and after each step
+        unsigned char* mem = base + kNaHead + kNaAccBytes;
+        fm.layout(mem, nx, ny);
+        fm.map.count = nullptr;
+        unsigned* ctr = reinterpret_cast<unsigned*>(mem + kNaFluxBytes);
+        double* depth = reinterpret_cast<double*>(mem + kNaFluxBytes + ((kNaCtrBytes + 255) & ~size_t(255)));
+        a.eb = fm.eb;
+        a.eb.stage = g_noalloc_stage;
+        g_noalloc_stage += 2u * (unsigned)nsteps;
+        for (int l = 0; l < 2; ++l) a.eb.depth[l] = a.eb.depth_out[l] = depth + l * kNaCells;
+        for (int i = 0; i < nsteps; ++i) enqueue_flux_step(a, a, fm.map, ctr, 2.0 * p->cfl, s, [] {});
+    } else {
+        const dim3 gh0 = edge_grid_h(nx, ny, 0), gh1 = edge_grid_h(nx, ny, 1);
+        const dim3 gv0 = edge_grid_v(nx, ny, 0), gv1 = edge_grid_v(nx, ny, 1);
+        for (int i = 0; i < nsteps; ++i) {
+            k_edges_h<true, 1><<<gh0, edge_block_h(), 0, s>>>(a, 0);
+            k_edges_h<false, 1><<<gh1, edge_block_h(), 0, s>>>(a, 1);
+            k_edges_v<1><<<gv0, edge_block_v(), 0, s>>>(a, 0);
+            k_edges_v<1><<<gv1, edge_block_v(), 0, s>>>(a, 1);
+            k_volume<0><<<nbc, cell_block(), 0, s>>>(a);
+            k_advance<<<1, 1, 0, s>>>(tm, 2.0 * p->cfl);
+        }
     }
     LSH_CUDA(cudaGetLastError());
     TimeRec out{};

@@ -418,7 +418,7 @@ inline __host__ __device__ int tiles_y(int ny) { return (ny + 1 + kTileY - 1) / 
 struct TileMap {
     int ntx, nty;
     int* list;               // per tile row: the listed tiles' columns, ascending
-    int* count;              // per tile row: how many
+    int* count;              // per tile row: how many (null: every tile, and no busy flags)
     // per stage and tile, one byte for each of its warps of the cell passes
     unsigned short* busy[2];
 };
@@ -435,7 +435,10 @@ __device__ __forceinline__ bool tile_of(const TileMap& m, unsigned u, int warps,
     const unsigned t = u / (unsigned)warps;
     ty = (int)(t / (unsigned)m.ntx);
     const int k = (int)(t - (unsigned)ty * (unsigned)m.ntx);
-    if (ty >= m.nty || k >= m.count[ty]) return false;
+    tx = k;
+    if (ty >= m.nty) return false;
+    if (!m.count) return true;
+    if (k >= m.count[ty]) return false;
     tx = m.list[(size_t)ty * m.ntx + k];
     return true;
 }
@@ -448,7 +451,7 @@ __device__ __forceinline__ void tile_begin(const TileDep& d, const TileMap& m, T
     if (!d.wait) return;
     const int r = max(t - 1, 0) + (int)threadIdx.x;
     if (r <= min(t + after, m.nty - 1)) {
-        const unsigned target = d.per * (unsigned)m.count[r];
+        const unsigned target = d.per * (unsigned)(m.count ? m.count[r] : m.ntx);
         const int tbit = 1 << LSH_ERR_TIMEOUT;
         volatile int* err = &tm->err;
         unsigned long long start = 0;
@@ -527,7 +530,7 @@ __global__ void __launch_bounds__(32 * kCellWarps, kUpdateBlocks[SMALL])
     if (in) bits = lsh::update_cell<MODE>(a, i, j, a.tm->dt, busy);
     __syncwarp();
     busy = __any_sync(0xffffffffu, busy);
-    if ((threadIdx.x & 31) == 0)
+    if (m.count && (threadIdx.x & 31) == 0)
         reinterpret_cast<unsigned char*>(m.busy[MODE == 1 ? 1 : 0] + (size_t)ty * m.ntx + tx)[half] = busy;
     if (MODE != 2) warp_max_bits(bits, &a.tm->rmax_bits);
     tile_end(d, ty);
@@ -772,7 +775,8 @@ inline int enqueue_flux_step_as(const KArgs& a1, const KArgs& a2, const TileMap&
         cells(k_update<2, SMALL>, a2);
     }
     // a plain launch: waits for the whole step, then zeroes the counters
-    k_clock<<<clock_blocks(m), 256, 0, s>>>(a1.tm, two_cfl, c, c ? pass * st : 0, m);
+    if (m.count) k_clock<<<clock_blocks(m), 256, 0, s>>>(a1.tm, two_cfl, c, c ? pass * st : 0, m);
+    else k_advance<<<1, 256, 0, s>>>(a1.tm, two_cfl, c, c ? pass * st : 0);
     mark();
     return (order == 1) ? 6 : 13;
 }
