@@ -216,6 +216,55 @@ __global__ void __launch_bounds__(kCellBlock, 8) k_recon_tape(KArgs a, unsigned*
     dep_end(d);
 }
 
+// The flux pass's kernels for the recomputation (lsh_kernels.cuh): the slopes
+// with their branch tape, and the cell update that keeps the accumulators and
+// their partial sums (all of the grid's tiles: the reverse sweep reads them
+// everywhere).
+template <bool SMALL>
+__global__ void __launch_bounds__(32 * kCellWarps, kSlopesBlocks[SMALL])
+    k_slopes_tape(const __grid_constant__ KArgs a, const __grid_constant__ TileMap m, TileDep d) {
+    const unsigned u0 = blockIdx.x * (blockDim.x / 32);
+    int tx, ty, half, i, j;
+    if (!tile_of(m, u0, kCellWarps, tx, ty)) return;
+    tile_begin(d, m, a.tm, ty, 1);
+    if (tile_cell(a, tx, ty, u0, half, i, j)) {
+        const int id = j * a.c.nx + i;
+        a.tape[id] = lsh::recon_cell(a, id);
+    }
+    tile_end(d, ty);
+}
+
+template <int MODE, bool SMALL>
+__global__ void __launch_bounds__(32 * kCellWarps, kUpdateBlocks[SMALL])
+    k_update_keep(const __grid_constant__ KArgs a, const __grid_constant__ TileMap m, TileDep d) {
+    const unsigned u0 = blockIdx.x * (blockDim.x / 32);
+    int tx, ty, half, i, j;
+    if (!tile_of(m, u0, kCellWarps, tx, ty)) return;
+    tile_begin(d, m, a.tm, ty, 1);
+    bool busy = false;
+    if (tile_cell(a, tx, ty, u0, half, i, j)) lsh::update_cell<MODE, true>(a, i, j, a.tm->dt, busy);
+    tile_end(d, ty);
+}
+
+// The recomputation of one step: order 1 from a1, order 2 stage 1 from a1 (X to
+// Y) and stage 2's accumulators from a2.
+template <bool SMALL>
+void enqueue_recompute(const KArgs& a1, const KArgs& a2, const TileMap& m, unsigned* c, cudaStream_t s) {
+    auto none = [] {};
+    FluxPasses<SMALL, decltype(none)> p(m, c, a1.c, s, none);
+    if (a1.c.order == 1) {
+        p.flux(k_flux<1, SMALL>, a1);
+        p.cells(k_update_keep<-1, SMALL>, a1);
+    } else {
+        p.cells(k_slopes_tape<SMALL>, a1);
+        p.flux(k_flux<2, SMALL>, a1);
+        p.cells(k_update_keep<1, SMALL>, a1);
+        p.cells(k_slopes_tape<SMALL>, a2);
+        p.flux(k_flux<2, SMALL>, a2);
+        p.cells(k_update_keep<-1, SMALL>, a2);
+    }
+}
+
 // Max and arg-max (lowest cell on ties) of acc_w / area (0 below EPSILON).
 __global__ void __launch_bounds__(kCellBlock) k_adj_rate_max(const double* acc6, Geo geo, int nx, long long N,
                                                              unsigned long long* rmax) {
@@ -358,6 +407,7 @@ __global__ void __launch_bounds__(32 * kRed) k_adj_reduce_rows(const double* par
 // stays (the host reads it after the run, and later waits give up at once).
 __device__ __forceinline__ void set_dt_body(lsh::TimeRec* tm, const double* dt) {
     tm->dt = *dt;
+    tm->steps += 1;  // the flux pass's marks of an earlier replay are not this one's
     tm->rmax_bits = kRateInitBits;
     tm->done = 0;
     tm->err &= 1 << LSH_ERR_TIMEOUT;
@@ -414,7 +464,11 @@ struct lsh_adjoint {
     double* eta_dummy = nullptr;
     unsigned* tape1 = nullptr, *tape2 = nullptr;
     unsigned char* szero1 = nullptr, *szero2 = nullptr;  // slope-zero flags of s1x/s1y and s2x/s2y
-    unsigned* dep_ctr = nullptr;    // pass-overlap counters of one step (13 segments of dep_stride)
+    FluxMem flux;                   // the flux pass's arrays, in place of Yb, sxb, syb and accb (flux_on)
+    bool flux_on = false;           // false: the colour passes (flux_fits)
+    bool listed = false;            // flux.map lists the tiles that X's next step has to visit
+    unsigned* dep_ctr = nullptr;    // pass-overlap counters of one step
+    size_t n_ctr = 0;
     int dep_stride = 0;             // 0: the passes run fully ordered
     bool ordered = false;           // lsh_adjoint_set_ordered: no pass overlap
     double* geo_buf = nullptr;
@@ -500,19 +554,50 @@ void fwd_passes(const lsh_adjoint* A, const KArgs& a, double* snaps[3][2], doubl
     k_edges_v<ORDER><<<grid_v(A, 1), edge_block_v(), 0, s>>>(a, 1);
 }
 
+// The stages' arguments of a step X -> X, or of its recomputation (`replay`),
+// which leaves X as it is.
+void step_args(const lsh_adjoint* A, bool replay, KArgs& a1, KArgs& a2) {
+    double* const* X = A->X;
+    double* Y7[7];
+    for (int k = 0; k < 6; ++k) Y7[k] = A->Y[k];
+    Y7[6] = A->X[6];
+    double* const* out = replay ? nullptr : X;
+    if (A->order == 1) {
+        a1 = a2 = fwd_args(A, X, out, nullptr, A->acc1, nullptr, nullptr);
+    } else {
+        a1 = fwd_args(A, X, A->Y, nullptr, A->acc1, A->s1x, A->s1y);
+        a2 = fwd_args(A, Y7, out, out, A->acc2, A->s2x, A->s2y);
+        if (replay) { a1.tape = A->tape1; a2.tape = A->tape2; }
+    }
+    std::memcpy(a1.part, A->snap1, sizeof(a1.part));
+    std::memcpy(a2.part, A->snap2, sizeof(a2.part));
+    if (!A->flux_on) return;
+    a1.eb = a2.eb = A->flux.eb;
+    a2.eb.stage = 1;
+    for (int l = 0; l < 2; ++l) {
+        a1.eb.depth[l] = a1.W[3 * l];
+        a2.eb.depth[l] = a2.W[3 * l];
+        if (A->order == 1 && !replay) a1.eb.depth[l] = a1.eb.depth_out[l] = A->Y[3 * l];  // in place
+    }
+}
+
 // One forward step X -> X (the product's step: the same kernels and order),
-// with the time record's dt; k_advance leaves the next dt in the record.
-void fwd_step(const lsh_adjoint* A, cudaStream_t s) {
+// with the time record's dt; the clock leaves the next dt in the record.
+void fwd_step(lsh_adjoint* A, cudaStream_t s) {
     const dim3 nbc = cell_grid(A->p.nx, A->p.ny);
     double* const* X = A->X;
+    if (A->flux_on) {
+        KArgs a1, a2;
+        step_args(A, false, a1, a2);
+        if (!A->listed) launch_all_busy(A->flux.map, s);
+        A->listed = true;
+        enqueue_flux_step(a1, a2, A->flux.map, overlap_ctr(A), 2.0 * A->c.cfl, s, [] {});
+        return;
+    }
     if (overlap_ctr(A)) {
         // the product's overlapped step (lsh_kernels.cuh)
-        double* Y7[7];
-        for (int k = 0; k < 6; ++k) Y7[k] = A->Y[k];
-        Y7[6] = A->X[6];
-        const KArgs a1 = (A->order == 1) ? fwd_args(A, X, X, nullptr, A->acc1, nullptr, nullptr)
-                                         : fwd_args(A, X, A->Y, nullptr, A->acc1, A->s1x, A->s1y);
-        const KArgs a2 = (A->order == 1) ? a1 : fwd_args(A, Y7, X, X, A->acc2, A->s2x, A->s2y);
+        KArgs a1, a2;
+        step_args(A, false, a1, a2);
         enqueue_step_overlap(A->p.nx, A->p.ny, A->order, a1, a2, A->dep_ctr, A->dep_stride, A->tm, 2.0 * A->c.cfl, s);
         return;
     }
@@ -685,6 +770,7 @@ struct Ops : lsh::RevolveOps {
         return 0;
     }
     int restore(int k, int) override {
+        A->listed = false;
         for (int v = 0; v < 6; ++v)
             A_CUDA(cudaMemcpyAsync(A->X[v], slot(k, v), A->N * sizeof(double), cudaMemcpyDeviceToDevice, A->stream));
         return 0;
@@ -705,7 +791,17 @@ int Ops::reverse_step(int n) {
     k_set_dt<<<1, 1, 0, s>>>(A->tm, A->d_dts + n);
     double* const* X = A->X;
     const double dt = A->h_dts[n];
-    if (overlap_ctr(A)) {
+    A->listed = false;
+    if (A->flux_on) {
+        KArgs a1, a2;
+        step_args(A, true, a1, a2);
+        TileMap m = A->flux.map;
+        m.count = nullptr;
+        unsigned* c = overlap_ctr(A);
+        const bool small = (unsigned(m.ntx) * unsigned(m.nty) <= kSmallTiles);
+        (small ? enqueue_recompute<true> : enqueue_recompute<false>)(a1, a2, m, c, s);
+        if (c) cudaMemsetAsync(c, 0, A->n_ctr * sizeof(unsigned), s);
+    } else if (overlap_ctr(A)) {
         // overlapped passes; the edge passes take the accumulator snapshots
         // themselves, at the cells the reverse sweep reads them
         unsigned* c = A->dep_ctr;
@@ -733,7 +829,7 @@ int Ops::reverse_step(int n) {
             enqueue_stage_overlap<2, -1>(nx, ny, a2, s, pr2, c + 7 * st, st, true, A->snap2);
         }
         // ordered after the passes (a stream operation waits for them all)
-        cudaMemsetAsync(c, 0, size_t(13) * st * sizeof(unsigned), s);
+        cudaMemsetAsync(c, 0, A->n_ctr * sizeof(unsigned), s);
     } else if (A->order == 1) {
         const KArgs a = fwd_args(A, X, nullptr, nullptr, A->acc1, nullptr, nullptr);
         fwd_passes<1>(A, a, A->snap1, A->acc1, s);
@@ -783,7 +879,7 @@ int Ops::reverse_step(int n) {
         }
     }
     // ordered after the chain: its counters back to zero
-    if (overlap_ctr(A)) cudaMemsetAsync(A->dep_ctr, 0, size_t(13) * A->dep_stride * sizeof(unsigned), s);
+    if (overlap_ctr(A)) cudaMemsetAsync(A->dep_ctr, 0, A->n_ctr * sizeof(unsigned), s);
     {
         const long long chunk = (nparts + kReduceRows - 1) / kReduceRows;
         k_adj_reduce_rows<<<kReduceRows, 32 * kRed, 0, s>>>(A->part, nparts, chunk, A->part2);
@@ -858,6 +954,7 @@ int fwd_begin(lsh_adjoint* A, const double* const host_state[LSH_NVARS], const d
     A->have_forward = false;
     A->spine_stored = false;
     A->cur_step = -1;
+    A->listed = false;
     A->have_target = (target != nullptr) && A->ng > 0;
     if (A->have_target)
         A_CUDA(cudaMemcpyAsync(A->d_tgt, target, sizeof(double) * (size_t)A->nsteps * A->ng, cudaMemcpyHostToDevice, s));
@@ -952,6 +1049,7 @@ int grad_begin(lsh_adjoint* A, double misfit_weight, const double* const bar_fin
     A->stats.reversed_steps = 0;
     A->spine_stored = false;  // the sweep reuses the slots
     A->cur_step = -1;
+    A->listed = false;
     A_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1024,11 +1122,6 @@ void grad_params_of(const lsh_adjoint* A, double gp[4]) {
 // own.  An item waits only for the rows of its member that it reads or
 // overwrites in the pass it depends on, with bounded waits as in the queue.
 
-struct ReconTape {
-    static constexpr bool kOn = true;
-    __device__ static unsigned run(const KArgs& a, int id) { return lsh::recon_cell_tape(a, id); }
-};
-
 constexpr int kRThreads = kAdjCellBlock;  // the adjoint kernels' block size
 constexpr int kRMaxPasses = 16;
 // CTAs per SM of the reverse queue (its register budget: 40 at 12) and the
@@ -1040,7 +1133,7 @@ constexpr int kRMaxPasses = 16;
 // 6/4 5.33, 7/4 5.15, 8/4 4.96, 10/4 4.75, 12/4 4.63, 12/8 4.67, 14/4 4.60,
 // 16/2 4.56, 16/4 4.74, 16/8 4.95.
 #ifndef LSH_ADJB_MINB
-#define LSH_ADJB_MINB 12
+#define LSH_ADJB_MINB 8
 #endif
 #ifndef LSH_ADJB_FETCH
 #define LSH_ADJB_FETCH 4
@@ -1390,8 +1483,9 @@ __global__ void __launch_bounds__(kCellBlock) k_adjb_project(const RMis* t) {
 // The members of one order, with their queues and tables.
 struct AdjGroup {
     int order = 1;
+    bool flux = true;          // every member's step takes the flux pass
     std::vector<lsh_adjoint*> m;
-    KArgs* d_kargs = nullptr;  // [2][n] the forward step, then [8][n] the recomputation
+    KArgs* d_kargs = nullptr;  // [2][n] the forward step, then [2 or 8][n] the recomputation
     void* qmem_fwd = nullptr;
     void* qmem_rec = nullptr;
     void* rmem = nullptr;      // the reverse plan's tables and counters
@@ -1516,34 +1610,21 @@ int build_group(AdjGroup& g) {
     const int n = (int)g.m.size();
     std::vector<int> nx(n), ny(n);
     std::vector<KArgs> ka(size_t(10) * n);
+    for (const lsh_adjoint* A : g.m) g.flux = g.flux && A->flux_on;
     for (int s = 0; s < n; ++s) {
         lsh_adjoint* A = g.m[s];
         nx[s] = A->p.nx;
         ny[s] = A->p.ny;
-        double* const* X = A->X;
-        double* Y7[7];
-        for (int k = 0; k < 6; ++k) Y7[k] = A->Y[k];
-        Y7[6] = A->X[6];
-        // the forward step: stage 1 (X -> Y, or X -> X), stage 2 (Y -> X, averaged with X)
-        const KArgs a1 = (g.order == 1) ? fwd_args(A, X, X, nullptr, A->acc1, nullptr, nullptr)
-                                        : fwd_args(A, X, A->Y, nullptr, A->acc1, A->s1x, A->s1y);
-        ka[s] = a1;
-        ka[n + s] = (g.order == 1) ? a1 : fwd_args(A, Y7, X, X, A->acc2, A->s2x, A->s2y);
-        // the recomputation: per stage the plain arguments (with the branch
-        // tape), then the three snapshot-taking edge passes
-        KArgs r1 = (g.order == 1) ? fwd_args(A, X, nullptr, nullptr, A->acc1, nullptr, nullptr)
-                                  : fwd_args(A, X, A->Y, nullptr, A->acc1, A->s1x, A->s1y);
-        r1.tape = A->tape1;
-        KArgs r2 = r1;
-        if (g.order == 2) {
-            r2 = fwd_args(A, Y7, nullptr, nullptr, A->acc2, A->s2x, A->s2y);
-            r2.tape = A->tape2;
-        }
+        // the forward step's two stages, then the recomputation's: each stage's
+        // plain arguments, then those of the three snapshot-taking colour passes
+        step_args(A, false, ka[s], ka[n + s]);
+        KArgs r1, r2;
+        step_args(A, true, r1, r2);
         for (int st = 0; st < 2; ++st) {
             const KArgs& base = st ? r2 : r1;
             double* const (*snaps)[2] = st ? A->snap2 : A->snap1;
-            ka[size_t(2 + 4 * st) * n + s] = base;
-            for (int k = 0; k < 3; ++k) {
+            ka[size_t(2 + (g.flux ? st : 4 * st)) * n + s] = base;
+            for (int k = 0; k < 3 && !g.flux; ++k) {
                 KArgs v = base;
                 v.snap[0] = snaps[k][0];
                 v.snap[1] = snaps[k][1];
@@ -1568,21 +1649,14 @@ int build_group(AdjGroup& g) {
     g.d_mis = reinterpret_cast<RMis*>(tb + o_mis);
     g.d_red = reinterpret_cast<RRed*>(tb + o_r);
     // the forward step's queue
-    std::vector<QPassSpec> fp, rp;
-    const int stages = (g.order == 2) ? 2 : 1;
-    for (int st = 0; st < stages; ++st) {
-        if (g.order == 2) fp.push_back({kOpRecon, kBCell, st});
-        fp.push_back({kOpH0, kBH0, st});
-        fp.push_back({kOpH1, kBH1, st});
-        fp.push_back({kOpV0, kBV0, st});
-        fp.push_back({kOpV1, kBV1, st});
-        fp.push_back({(g.order == 1) ? kOpVol0 : (st == 0 ? kOpVol1 : kOpVol2), kBCell, st});
-    }
+    const std::vector<QPassSpec> fp = g.flux ? flux_queue_passes(g.order, false) : colour_queue_passes(g.order);
     if (int st = build_queue_plan(nx, ny, fp, g.d_kargs, &g.qmem_fwd, g.fwd, g.nctr_fwd)) return st;
     // the recomputation's queue (variables 0..7 of its table)
-    for (int st = 0; st < stages; ++st) {
+    std::vector<QPassSpec> rp;
+    if (g.flux) rp = flux_queue_passes(g.order, true);
+    for (int st = 0; st < g.order && !g.flux; ++st) {
         const int v = 4 * st;
-        if (g.order == 2) rp.push_back({kOpReconTape, kBCell, v});
+        if (g.order == 2) rp.push_back({kOpRecon, kBCell, v});
         rp.push_back({kOpH0, kBH0, v});
         rp.push_back({kOpH1, kBH1, v + 1});
         rp.push_back({kOpV0, kBV0, v + 2});
@@ -1673,9 +1747,7 @@ constexpr int kAdjbFwdFetch = LSH_ADJB_FWD_FETCH;
 void group_forward(AdjGroup& g, int sms, int n, bool record, cudaStream_t s) {
     const int nm = (int)g.m.size();
     if (!record) k_adjb_pre<<<(nm + 127) / 128, 128, 0, s>>>(g.d_mem, nm, n);
-    const int grid = sms * kAdjbFwdCtas;
-    if (g.order == 1) k_batch_step<1><<<grid, kBThreads, 0, s>>>(g.fwd, kAdjbFwdFetch);
-    else k_batch_step<2><<<grid, kBThreads, 0, s>>>(g.fwd, kAdjbFwdFetch);
+    (g.flux ? launch_queue<kQFlux> : launch_queue<kQColour>)(g.fwd, g.order, sms, kAdjbFwdCtas, kAdjbFwdFetch, s);
     const int adv = std::max(1, std::min((std::max(g.nctr_fwd, nm) + 255) / 256, 2 * sms));
     k_batch_advance<<<adv, 256, 0, s>>>(g.d_kargs, nm, g.fwd.ctr, g.nctr_fwd, g.fwd.head);
     if (record) k_adjb_record<<<nm, 128, 0, s>>>(g.d_fmem, n);
@@ -1685,9 +1757,7 @@ void group_forward(AdjGroup& g, int sms, int n, bool record, cudaStream_t s) {
 void group_reverse(AdjGroup& g, int sms, int n, cudaStream_t s) {
     const int nm = (int)g.m.size();
     k_adjb_pre<<<(nm + 127) / 128, 128, 0, s>>>(g.d_mem, nm, n);
-    const int grid = sms * kAdjbFwdCtas;
-    if (g.order == 1) k_batch_step<1, ReconTape><<<grid, kBThreads, 0, s>>>(g.rec, kAdjbFwdFetch);
-    else k_batch_step<2, ReconTape><<<grid, kBThreads, 0, s>>>(g.rec, kAdjbFwdFetch);
+    (g.flux ? launch_queue<kQFluxKeep> : launch_queue<kQColour>)(g.rec, g.order, sms, kAdjbFwdCtas, kAdjbFwdFetch, s);
     const int rgrid = sms * LSH_ADJB_MINB;
     if (g.order == 1) k_adjb_reverse<1><<<rgrid, kRThreads, 0, s>>>(g.rev, g.parity, n);
     else k_adjb_reverse<2><<<rgrid, kRThreads, 0, s>>>(g.rev, g.parity, n);
@@ -1791,8 +1861,19 @@ int lsh_adjoint_create(const lsh_params* params, int device, int n_gauges, const
     const int narr = 7 + 6 + 28 + 14 + 12 + 18 + 21 + 1 + 2;
     const size_t geo_n = 7 * size_t(params->ny + 1);
     A->dep_stride = dep_stride_for(params->nx, params->ny);
-    const size_t bytes = (size_t(narr) * A->npad + ((geo_n + 31) & ~size_t(31))) * sizeof(double) +
-                         2 * A->npad * sizeof(unsigned) + 2 * A->npad + size_t(13) * A->dep_stride * sizeof(unsigned);
+    A->flux_on = lsh::flux_fits(A->p);
+    if (A->dep_stride)
+        A->n_ctr = std::max(size_t(13) * A->dep_stride,
+                            size_t(flux_step_passes(A->order)) * flux_dep_stride(params->ny));
+    // The flux pass's arrays hold nothing between passes, and the reverse
+    // sweep's stage and slope adjoints (each stage's volume adjoint writes them
+    // anew) nothing outside a reversed step's adjoint passes: one place for both,
+    // so the adjoint needs no more memory.  Only a narrow grid's edges outgrow it.
+    const size_t shared = size_t(6 + 21) * A->npad * sizeof(double);
+    const size_t flux_bytes = A->flux_on ? A->flux.layout(nullptr, params->nx, params->ny) : 0;
+    const size_t extra = (flux_bytes > shared) ? (flux_bytes - shared + 255) & ~size_t(255) : 0;
+    const size_t bytes = (size_t(narr) * A->npad + ((geo_n + 31) & ~size_t(31))) * sizeof(double) + extra +
+                         2 * A->npad * sizeof(unsigned) + 2 * A->npad + A->n_ctr * sizeof(unsigned);
     { cudaError_t e = cudaMalloc(&A->slab, bytes); if (e != cudaSuccess) return bail(afail(e, "cudaMalloc adjoint work arrays")); }
     {
         // zero the work arrays and wait: the geometry and gauge copies below go
@@ -1809,8 +1890,11 @@ int lsh_adjoint_create(const lsh_params* params, int device, int n_gauges, const
     for (int k = 0; k < 7; ++k) { take(A->s1x[k]); take(A->s1y[k]); take(A->s2x[k]); take(A->s2y[k]); }
     for (int k = 0; k < 7; ++k) { take(A->acc1[k]); take(A->acc2[k]); }
     for (int q = 0; q < 3; ++q) for (int v = 0; v < 2; ++v) { take(A->snap1[q][v]); take(A->snap2[q][v]); }
-    for (int k = 0; k < 6; ++k) { take(A->Xb[k]); take(A->Xbn[k]); take(A->Yb[k]); }
+    for (int k = 0; k < 6; ++k) { take(A->Xb[k]); take(A->Xbn[k]); }
+    if (A->flux_on) A->flux.layout(reinterpret_cast<unsigned char*>(cur), params->nx, params->ny);
+    for (int k = 0; k < 6; ++k) take(A->Yb[k]);
     for (int k = 0; k < 7; ++k) { take(A->sxb[k]); take(A->syb[k]); take(A->accb[k]); }
+    cur += extra / sizeof(double);
     take(A->eta_dummy);
     take(A->hN[0]);
     take(A->hN[1]);

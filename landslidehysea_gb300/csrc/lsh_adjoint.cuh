@@ -1335,11 +1335,8 @@ LSH_HD void volume_adj_body(const AdjArgs& a, int id, double& dtb, ConstBar& cb)
     for (int k = 0; k < 7; ++k) a.accb[k][id] = accb[k];
 }
 
-// Branch tape of one cell's reconstruction (recon_cell): for variable k and
-// direction d (0 x, 1 y) bits 2 (7 d + k) .. +1 hold the minmod choice (0
-// zero, 1 the backward difference, 2 the forward one); bit 28: slopes zeroed
-// (a reconstructed depth below kReconThin of the cell's, or the dry shortcut).
-// Without bit 28, sx and sy hold the cell's slopes (recon_cell's values).
+// The branch tape of one cell's reconstruction restated plainly, and without
+// kTapeFlat its slopes: what recon_cell is compared with.
 LSH_HD unsigned recon_tape_slopes(const double* const* W, int nx, int ny, int id, double sx[7], double sy[7]) {
     const int j = id / nx, i = id - j * nx;
     {
@@ -1391,28 +1388,8 @@ LSH_HD unsigned recon_tape_cell(const double* const* W, int nx, int ny, int id) 
     return recon_tape_slopes(W, nx, ny, id, sx, sy);
 }
 
-// The reconstruction of recon_cell (lsh_passes.cuh) writing its slopes and
-// returning the branch tape of recon_tape_cell in one pass: the slopes are
-// the halved minmod choices, the operations recon_cell performs, so they are
-// bit-identical to recon_cell's.
-LSH_HD unsigned recon_cell_tape(const KArgs& a, int id) {
-    double sx[7], sy[7];
-    const unsigned t = recon_tape_slopes(a.W, a.c.nx, a.c.ny, id, sx, sy);
-    if (t & (1u << 28)) {
-        // zero slopes; with slope-zero flags (as recon_cell keeps them) a cell
-        // whose stored slopes are already zero skips the stores
-        if (a.szero && a.szero[id]) return t;
-        for (int k = 0; k < 7; ++k) { a.sxw[k][id] = 0.0; a.syw[k][id] = 0.0; }
-        if (a.szero) a.szero[id] = 1;
-        return t;
-    }
-    if (a.szero) a.szero[id] = 0;
-    for (int k = 0; k < 7; ++k) {
-        a.sxw[k][id] = sx[k];
-        a.syw[k][id] = sy[k];
-    }
-    return t;
-}
+// The recomputation's reconstruction: recon_cell's slopes and branch tape.
+LSH_HD unsigned recon_cell_tape(const KArgs& a, int id) { return recon_cell(a, id); }
 
 // Reconstruction adjoint, gathered at cell id: Wbar[id] += sum over the
 // slopes that read cell id of d(slope)/d(W[id]) * slope adjoint.

@@ -103,6 +103,7 @@ struct lsh_batch {
     std::vector<size_t> base;       // first cell of each scenario in the slab arrays
     size_t total = 0;
     void* slab = nullptr;
+    void* edge_mem = nullptr;       // the flux pass's arrays (null: the colour passes)
     KArgs* d_args = nullptr;        // [n] (stage 1), [n, 2n) (stage 2)
     std::vector<KArgs> h_args;
     lsh::TimeRec* d_tm = nullptr;   // [n]
@@ -118,29 +119,15 @@ namespace {
 
 constexpr int kernels_per_step = 2;  // the step kernel and the clock kernel
 
-// The step's passes: reconstruction (second order), the four colour edge
-// passes and the Euler stage, per stage.
 int build_plan(lsh_batch* b) {
     std::vector<int> nx(b->n), ny(b->n);
     for (int s = 0; s < b->n; ++s) { nx[s] = b->params[s].nx; ny[s] = b->params[s].ny; }
-    std::vector<QPassSpec> passes;
-    const int stages = (b->order == 2) ? 2 : 1;
-    for (int st = 0; st < stages; ++st) {
-        if (b->order == 2) passes.push_back({kOpRecon, kBCell, st});
-        passes.push_back({kOpH0, kBH0, st});
-        passes.push_back({kOpH1, kBH1, st});
-        passes.push_back({kOpV0, kBV0, st});
-        passes.push_back({kOpV1, kBV1, st});
-        passes.push_back({(b->order == 1) ? kOpVol0 : (st == 0 ? kOpVol1 : kOpVol2), kBCell, st});
-    }
-    return build_queue_plan(nx, ny, passes, b->d_args, &b->d_plan_mem, b->plan, b->n_ctr);
+    return build_queue_plan(nx, ny, b->edge_mem ? flux_queue_passes(b->order, false) : colour_queue_passes(b->order), b->d_args, &b->d_plan_mem, b->plan, b->n_ctr);
 }
 
 void enqueue_batch_step(lsh_batch* b, cudaStream_t s) {
-    const int grid = std::max(1, b->sms * std::min(std::max(b->tune.ctas_per_sm, 1), kBMaxCtas));
-    const int fetch = std::max(1, b->tune.items_per_fetch);
-    if (b->order == 1) k_batch_step<1><<<grid, kBThreads, 0, s>>>(b->plan, fetch);
-    else k_batch_step<2><<<grid, kBThreads, 0, s>>>(b->plan, fetch);
+    (b->edge_mem ? launch_queue<kQFlux> : launch_queue<kQColour>)(b->plan, b->order, b->sms, b->tune.ctas_per_sm,
+                                                                  std::max(1, b->tune.items_per_fetch), s);
     const int adv = std::max(1, std::min((std::max(b->n_ctr, b->n) + 255) / 256, 2 * b->sms));
     k_batch_advance<<<adv, 256, 0, s>>>(b->d_args, b->n, b->plan.ctr, b->n_ctr, b->plan.head);
 }
@@ -204,6 +191,27 @@ int lsh_batch_create(const lsh_params* params, int n, int device, lsh_batch** ou
     const size_t flag_bytes = (b->order == 2) ? ((cells + 7) & ~size_t(7)) : 0;
     const size_t bytes = (size_t(arrays) * cells + geo) * sizeof(double) + flag_bytes;
     { cudaError_t e = cudaMalloc(&b->slab, bytes); if (e != cudaSuccess) return bail(bfail(e, "cudaMalloc batch slab")); }
+    // The flux pass's arrays: 23 doubles a cell beside the slab's 36 (22 at order
+    // 1).  Without room for them, or with a scenario that flux_fits refuses, the
+    // batch takes the colour passes, which need none.
+    std::vector<size_t> edge_off(n);
+    {
+        size_t edge_bytes = 0;
+        bool fits = true;
+        lsh::EdgeBuf eb{};
+        for (int s = 0; s < n; ++s) {
+            edge_off[s] = edge_bytes;
+            edge_bytes += lsh::edge_layout(eb, nullptr, params[s].nx, params[s].ny);
+            fits = fits && lsh::flux_fits(params[s]);
+        }
+        if (fits && cudaMalloc(&b->edge_mem, edge_bytes) == cudaSuccess) {
+            cudaError_t e = cudaMemset(b->edge_mem, 0, edge_bytes);
+            if (e != cudaSuccess) return bail(bfail(e, "edge arrays"));
+        } else {
+            b->edge_mem = nullptr;
+            (void)cudaGetLastError();
+        }
+    }
     { cudaError_t e = cudaMalloc(&b->d_tm, sizeof(lsh::TimeRec) * n); if (e != cudaSuccess) return bail(bfail(e, "cudaMalloc")); }
     const int nargs = (b->order == 2) ? 2 * n : n;
     { cudaError_t e = cudaMalloc(&b->d_args, sizeof(KArgs) * nargs); if (e != cudaSuccess) return bail(bfail(e, "cudaMalloc")); }
@@ -241,11 +249,20 @@ int lsh_batch_create(const lsh_params* params, int n, int device, lsh_batch** ou
             a.szero = flags + o;  // both stages share the slopes and their flags
         }
         a.tm = b->d_tm + s;
+        if (b->edge_mem) {
+            lsh::edge_layout(a.eb, static_cast<unsigned char*>(b->edge_mem) + edge_off[s], p.nx, p.ny);
+            for (int l = 0; l < 2; ++l) {
+                a.eb.depth[l] = a.W[3 * l];
+                if (b->order == 1) a.eb.depth[l] = a.eb.depth_out[l] = arr(7 + 3 * l) + o;  // in place: a copy in Y
+            }
+        }
         b->h_args[s] = a;
         if (b->order == 2) {
             KArgs a2 = a;  // stage 2: Y -> X, average with X
             for (int k = 0; k < 6; ++k) { a2.W[k] = arr(7 + k) + o; a2.Wout[k] = arr(k) + o; a2.Xavg[k] = arr(k) + o; }
             a2.W[6] = arr(6) + o;
+            a2.eb.stage = 1;
+            for (int l = 0; l < 2; ++l) a2.eb.depth[l] = a2.W[3 * l];
             b->h_args[n + s] = a2;
         }
     }
@@ -267,6 +284,7 @@ int lsh_batch_destroy(lsh_batch* b) {
     if (b->d_args) cudaFree(b->d_args);
     if (b->d_tm) cudaFree(b->d_tm);
     if (b->slab) cudaFree(b->slab);
+    if (b->edge_mem) cudaFree(b->edge_mem);
     if (b->stream) cudaStreamDestroy(b->stream);
     (void)cudaGetLastError();
     delete b;

@@ -691,21 +691,15 @@ struct FluxMem {
     unsigned char* clear = nullptr;
     size_t clear_bytes = 0;
     size_t layout(unsigned char* mem, int nx, int ny) {
-        const size_t N = size_t(nx) * ny, tiles = size_t(tiles_x(nx)) * tiles_y(ny);
+        const size_t tiles = size_t(tiles_x(nx)) * tiles_y(ny);
         size_t at = 0;
         auto take = [&](size_t bytes) { unsigned char* q = mem + at; at += (bytes + 255) & ~size_t(255); return q; };
-        const size_t n[2] = {(N + nx + 31) & ~size_t(31), (N + ny + 31) & ~size_t(31)};
-        for (int d = 0; d < 2; ++d) {
-            eb.plane[d] = n[d];
-            eb.q[d] = reinterpret_cast<double*>(take(lsh::kEdgePlanes * n[d] * sizeof(double)));
-            eb.kind[d] = take(n[d]);
-        }
         map.ntx = tiles_x(nx);
         map.nty = tiles_y(ny);
         map.list = reinterpret_cast<int*>(take(tiles * sizeof(int)));
         map.count = reinterpret_cast<int*>(take(map.nty * sizeof(int)));
-        clear = mem + at;
-        for (int l = 0; l < 2; ++l) eb.mark[l] = reinterpret_cast<unsigned*>(take(N * sizeof(unsigned)));
+        at += lsh::edge_layout(eb, mem + at, nx, ny);
+        clear = reinterpret_cast<unsigned char*>(eb.mark[0]);
         for (int l = 0; l < 2; ++l) map.busy[l] = reinterpret_cast<unsigned short*>(take(tiles * sizeof(unsigned short)));
         clear_bytes = size_t(mem + at - clear);
         return at;
@@ -727,6 +721,50 @@ inline void launch_all_busy(const TileMap& m, cudaStream_t s) {
 inline int flux_step_passes(int order) { return (order == 1) ? 2 : 6; }
 inline int flux_dep_stride(int ny) { return (tiles_y(ny) + 63) & ~63; }
 
+// Launches a step's passes in order, each behind the one before through the
+// counters `c` (null: one after the other); `mark` is called after each launch.
+template <bool SMALL, class Mark>
+struct FluxPasses {
+    static constexpr unsigned cw = SMALL ? 1 : kCellWarps, fw = SMALL ? 1 : kFluxWarps;  // warps per block
+    const TileMap& m;
+    unsigned* c;
+    const int st, last;
+    const unsigned tiles;
+    cudaStream_t s;
+    Mark& mark;
+    TileDep d;  // the pass before as producer, this pass's own counters
+    int pass = 0;
+    FluxPasses(const TileMap& map, unsigned* ctr, const lsh::Consts& k, cudaStream_t stream, Mark& mk)
+        : m(map), c(ctr), st(flux_dep_stride(k.ny)), last(flux_step_passes(k.order) - 1),
+          tiles(unsigned(map.ntx) * unsigned(map.nty)), s(stream), mark(mk) {}
+    int counters() const { return c ? pass * st : 0; }
+    template <class Kernel, class... X>
+    void cells(Kernel kernel, const KArgs& a, const X&... x) {
+        begin();
+        launch_pass(d.wait != nullptr, dim3(tiles * (kCellWarps / cw)), dim3(32 * cw), s, kernel, a, m, d, x...);
+        mark();
+        end(kCellWarps / cw);
+    }
+    template <class Kernel>
+    void flux(Kernel kernel, const KArgs& a) {
+        begin();
+        const unsigned n = tiles * (kFluxWarps / fw);
+        for (int q = 0; q < kFluxParts; ++q) {
+            const unsigned b0 = unsigned((unsigned long long)n * q / kFluxParts);
+            const unsigned b1 = unsigned((unsigned long long)n * (q + 1) / kFluxParts);
+            launch_pass(c && (q > 0 || d.wait), dim3(b1 - b0), dim3(32 * fw), s, kernel, a, m, d, b0);
+            mark();
+        }
+        end(kFluxWarps / fw);
+    }
+private:
+    void begin() { if (c) d.done = (pass < last) ? c + pass * st : nullptr; }
+    void end(unsigned per) {
+        if (c) { d.wait = d.done; d.per = per; }
+        ++pass;
+    }
+};
+
 // One time step: a1 the stage 1 arguments (order 1: in place), a2 stage 2's
 // (with their edge buffers).  `c` (may be null: full-grid launches one after
 // the other): flux_dep_stride counters for each pass, which the clock kernel
@@ -736,47 +774,22 @@ inline int flux_dep_stride(int ny) { return (tiles_y(ny) + 63) & ~63; }
 template <bool SMALL, class Mark>
 inline int enqueue_flux_step_as(const KArgs& a1, const KArgs& a2, const TileMap& m, unsigned* c, double two_cfl,
                                 cudaStream_t s, Mark&& mark) {
-    const int order = a1.c.order, st = flux_dep_stride(a1.c.ny), last = flux_step_passes(order) - 1;
-    const unsigned tiles = unsigned(m.ntx) * unsigned(m.nty);
-    constexpr unsigned cw = SMALL ? 1 : kCellWarps, fw = SMALL ? 1 : kFluxWarps;  // warps per block
-    const unsigned nf = tiles * (kFluxWarps / fw), nc = tiles * (kCellWarps / cw);
-    TileDep d;  // the pass before as producer, this pass's own counters
-    int pass = 0;
-    auto begin = [&] { if (c) d.done = (pass < last) ? c + pass * st : nullptr; };
-    auto end = [&](unsigned per) {
-        if (c) { d.wait = d.done; d.per = per; }
-        ++pass;
-    };
-    auto cells = [&](auto kernel, const KArgs& a) {
-        begin();
-        launch_pass(d.wait != nullptr, dim3(nc), dim3(32 * cw), s, kernel, a, m, d);
-        mark();
-        end(kCellWarps / cw);
-    };
-    auto flux = [&](auto kernel, const KArgs& a) {
-        begin();
-        for (int q = 0; q < kFluxParts; ++q) {
-            const unsigned b0 = unsigned((unsigned long long)nf * q / kFluxParts);
-            const unsigned b1 = unsigned((unsigned long long)nf * (q + 1) / kFluxParts);
-            launch_pass(c && (q > 0 || d.wait), dim3(b1 - b0), dim3(32 * fw), s, kernel, a, m, d, b0);
-            mark();
-        }
-        end(kFluxWarps / fw);
-    };
+    const int order = a1.c.order;
+    FluxPasses<SMALL, Mark> p(m, c, a1.c, s, mark);
     if (order == 1) {
-        flux(k_flux<1, SMALL>, a1);
-        cells(k_update<0, SMALL>, a1);
+        p.flux(k_flux<1, SMALL>, a1);
+        p.cells(k_update<0, SMALL>, a1);
     } else {
-        cells(k_slopes<SMALL>, a1);
-        flux(k_flux<2, SMALL>, a1);
-        cells(k_update<1, SMALL>, a1);
-        cells(k_slopes<SMALL>, a2);
-        flux(k_flux<2, SMALL>, a2);
-        cells(k_update<2, SMALL>, a2);
+        p.cells(k_slopes<SMALL>, a1);
+        p.flux(k_flux<2, SMALL>, a1);
+        p.cells(k_update<1, SMALL>, a1);
+        p.cells(k_slopes<SMALL>, a2);
+        p.flux(k_flux<2, SMALL>, a2);
+        p.cells(k_update<2, SMALL>, a2);
     }
     // a plain launch: waits for the whole step, then zeroes the counters
-    if (m.count) k_clock<<<clock_blocks(m), 256, 0, s>>>(a1.tm, two_cfl, c, c ? pass * st : 0, m);
-    else k_advance<<<1, 256, 0, s>>>(a1.tm, two_cfl, c, c ? pass * st : 0);
+    if (m.count) k_clock<<<clock_blocks(m), 256, 0, s>>>(a1.tm, two_cfl, c, p.counters(), m);
+    else k_advance<<<1, 256, 0, s>>>(a1.tm, two_cfl, c, p.counters());
     mark();
     return (order == 1) ? 6 : 13;
 }

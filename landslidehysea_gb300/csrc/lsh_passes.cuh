@@ -66,7 +66,10 @@ struct KArgs {
     // before left them, to snap[0], snap[1] -- the partial sums its limiter
     // reads, which the reverse sweep needs at exactly those cells
     double* snap[2];
-    unsigned* tape;       // the recomputation's reconstruction branch tape (kOpReconTape; null otherwise)
+    // and the cell update copies the partial sums of each cell with a wet edge
+    // after the first three colours to part[colour]
+    double* part[3][2];
+    unsigned* tape;       // the recomputation's reconstruction branch tape (null otherwise)
     EdgeBuf eb;           // the flux pass's results (q[0] null: the colour passes run instead)
 };
 
@@ -298,7 +301,8 @@ LSH_HD void do_edge(const KArgs& a, int x, int y, double dt) {
 // sign (b on a tie), else 0 -- on the bit patterns (integer pipe); for
 // operands that are not NaN the same as the compares
 //   a > 0 && b > 0 ? (a < b ? a : b) : a < 0 && b < 0 ? (a > b ? a : b) : 0
-LSH_HD double minmod(double a, double b) {
+// `choice`: 0 for neither, 1 for a, 2 for b.
+LSH_HD double minmod_choice(double a, double b, unsigned& choice) {
     // (through halves: on the plain bits the compiler finds a == 0 and b == 0)
     uint32_t alo, ahi, blo, bhi;
     lshm::halves(a, alo, ahi);
@@ -306,22 +310,28 @@ LSH_HD double minmod(double a, double b) {
     const uint32_t am = ahi & 0x7fffffffu, bm = bhi & 0x7fffffffu;
     const bool nonzero = (am | alo) != 0u && (bm | blo) != 0u;
     const bool same = (int32_t)(ahi ^ bhi) >= 0;
+    const bool first = (((uint64_t)am << 32) | alo) < (((uint64_t)bm << 32) | blo);
+    choice = (nonzero && same) ? (first ? 1u : 2u) : 0u;
     if (!(nonzero && same)) return 0.0;
-    return ((((uint64_t)am << 32) | alo) < (((uint64_t)bm << 32) | blo)) ? a : b;
+    return first ? a : b;
+}
+LSH_HD double minmod(double a, double b) {
+    unsigned choice;
+    return minmod_choice(a, b, choice);
 }
 
-LSH_HD double recon_var(const KArgs& a, int id, int k) {
-    if (k == 0) return (a.W[0][id] + a.W[3][id]) - a.W[6][id];
-    if (k == 3) return a.W[3][id] - a.W[6][id];
-    return a.W[k][id];
-}
+// The branch tape of one cell's reconstruction, which its adjoint replays: for
+// variable k and direction d (0 x, 1 y) bits 2 (7 d + k) .. +1 hold the minmod
+// choice; kTapeFlat: zero slopes (a reconstructed depth below kReconThin of the
+// cell's, or the dry shortcut).
+constexpr unsigned kTapeFlat = 1u << 28;
 
 // One cell of the second-order reconstruction, its inputs read through an
 // accessor w(k, di, dj) = W[k] at cell (i + di, j + dj): global memory
 // (recon_cell) or a shared-memory tile (k_recon).  Neighbours are read only
-// inside the grid.
+// inside the grid.  Returns the cell's branch tape.
 template <class Acc>
-LSH_HD void recon_cell_from(const KArgs& a, int id, int i, int j, const Acc& w) {
+LSH_HD unsigned recon_cell_from(const KArgs& a, int id, int i, int j, const Acc& w) {
     const int nx = a.c.nx, ny = a.c.ny;
     // A cell whose own and 4 neighbours' depths are all zero only meets dry
     // edges (a dry cell's faces always have zero depth: any nonzero depth
@@ -337,19 +347,22 @@ LSH_HD void recon_cell_from(const KArgs& a, int id, int i, int j, const Acc& w) 
         if (dry) {
             // zero slopes; a cell whose stored slopes are already zero (and stays
             // dry, the common case far from the flow) skips the 14 stores
-            if (a.szero && a.szero[id]) return;
+            if (a.szero && a.szero[id]) return kTapeFlat;
 #pragma unroll
             for (int k = 0; k < 7; ++k) { a.sxw[k][id] = 0.0; a.syw[k][id] = 0.0; }
             if (a.szero) a.szero[id] = 1;
-            return;
+            return kTapeFlat;
         }
     }
     const bool inx = (i > 0 && i < nx - 1), iny = (j > 0 && j < ny - 1);
-    // halved minmod slopes of a variable rv(di, dj)
-    auto slopes = [&](auto rv, double& x, double& y) {
+    // halved minmod slopes of variable k, rv(di, dj)
+    unsigned tape = 0;
+    auto slopes = [&](int k, auto rv, double& x, double& y) {
         const double pc = rv(0, 0);
-        x = inx ? lsh::half(minmod(pc - rv(-1, 0), rv(1, 0) - pc)) : 0.0;
-        y = iny ? lsh::half(minmod(pc - rv(0, -1), rv(0, 1) - pc)) : 0.0;
+        unsigned cx = 0, cy = 0;
+        x = inx ? lsh::half(minmod_choice(pc - rv(-1, 0), rv(1, 0) - pc, cx)) : 0.0;
+        y = iny ? lsh::half(minmod_choice(pc - rv(0, -1), rv(0, 1) - pc, cy)) : 0.0;
+        tape |= (cx << (2 * k)) | (cy << (2 * (7 + k)));
     };
     // No granular layer anywhere in the stencil (h2 = q2 = 0 at the cell and
     // the neighbours it reads): eta1 = (h1 + 0) - H is h1 - H (but for the sign
@@ -374,21 +387,22 @@ LSH_HD void recon_cell_from(const KArgs& a, int id, int i, int j, const Acc& w) 
     double sx[7], sy[7];
     const double h1 = w(0, 0, 0);
     bool bad = false;
-    slopes([&](int di, int dj) { return w(1, di, dj); }, sx[1], sy[1]);
-    slopes([&](int di, int dj) { return w(2, di, dj); }, sx[2], sy[2]);
-    slopes([&](int di, int dj) { return w(6, di, dj); }, sx[6], sy[6]);
+    slopes(1, [&](int di, int dj) { return w(1, di, dj); }, sx[1], sy[1]);
+    slopes(2, [&](int di, int dj) { return w(2, di, dj); }, sx[2], sy[2]);
+    slopes(6, [&](int di, int dj) { return w(6, di, dj); }, sx[6], sy[6]);
     const bool fast = warp_all(one);
     if (fast) {
-        slopes([&](int di, int dj) { return w(0, di, dj) - w(6, di, dj); }, sx[0], sy[0]);
+        slopes(0, [&](int di, int dj) { return w(0, di, dj) - w(6, di, dj); }, sx[0], sy[0]);
         sx[3] = lsh::is_zero(sx[6]) ? 0.0 : lshm::neg_if(sx[6], true);
         sy[3] = lsh::is_zero(sy[6]) ? 0.0 : lshm::neg_if(sy[6], true);
         sx[4] = sx[5] = sy[4] = sy[5] = 0.0;
+        tape |= ((tape >> 12) & 3u) << 6 | ((tape >> 26) & 3u) << 20;  // eta2's choices are H's
     } else {
         lshm::rare();
-        slopes([&](int di, int dj) { return (w(0, di, dj) + w(3, di, dj)) - w(6, di, dj); }, sx[0], sy[0]);
-        slopes([&](int di, int dj) { return w(3, di, dj) - w(6, di, dj); }, sx[3], sy[3]);
-        slopes([&](int di, int dj) { return w(4, di, dj); }, sx[4], sy[4]);
-        slopes([&](int di, int dj) { return w(5, di, dj); }, sx[5], sy[5]);
+        slopes(0, [&](int di, int dj) { return (w(0, di, dj) + w(3, di, dj)) - w(6, di, dj); }, sx[0], sy[0]);
+        slopes(3, [&](int di, int dj) { return w(3, di, dj) - w(6, di, dj); }, sx[3], sy[3]);
+        slopes(4, [&](int di, int dj) { return w(4, di, dj); }, sx[4], sy[4]);
+        slopes(5, [&](int di, int dj) { return w(5, di, dj); }, sx[5], sy[5]);
     }
     // first order where a reconstructed depth would fall below kReconThin of
     // the cell's: a thin face with a finite discharge has an unbounded
@@ -418,13 +432,14 @@ LSH_HD void recon_cell_from(const KArgs& a, int id, int i, int j, const Acc& w) 
         a.syw[k][id] = bad ? 0.0 : sy[k];
     }
     if (a.szero) a.szero[id] = 0;  // conservative: only the dry path marks zeros
+    return bad ? kTapeFlat : tape;
 }
 
 // One cell of the second-order reconstruction from global memory.
-LSH_HD void recon_cell(const KArgs& a, int id) {
+LSH_HD unsigned recon_cell(const KArgs& a, int id) {
     const int nx = a.c.nx;
     const int j = id / nx, i = id - j * nx;
-    recon_cell_from(a, id, i, j, [&](int k, int di, int dj) -> double { return a.W[k][id + di + dj * nx]; });
+    return recon_cell_from(a, id, i, j, [&](int k, int di, int dj) -> double { return a.W[k][id + di + dj * nx]; });
 }
 
 #if defined(__CUDACC__)
@@ -598,6 +613,22 @@ LSH_HD unsigned long long volume_cell(const KArgs& a, int id, double dt) {
 // That an unmarked cell is never limited needs its partial sums not to fall
 // below what its own edges take, so the limiter's factors must not be
 // negative: a limited edge takes at most peso / beta of a cell's content, and
+// Its arrays placed in `mem` (256-byte aligned; null: the size alone), the marks
+// last; the bytes they take.
+inline size_t edge_layout(EdgeBuf& eb, unsigned char* mem, int nx, int ny) {
+    const size_t N = size_t(nx) * ny;
+    size_t at = 0;
+    auto take = [&](size_t bytes) { unsigned char* q = mem + at; at += (bytes + 255) & ~size_t(255); return q; };
+    const size_t n[2] = {(N + nx + 31) & ~size_t(31), (N + ny + 31) & ~size_t(31)};
+    for (int d = 0; d < 2; ++d) {
+        eb.plane[d] = n[d];
+        eb.q[d] = reinterpret_cast<double*>(take(kEdgePlanes * n[d] * sizeof(double)));
+        eb.kind[d] = take(n[d]);
+    }
+    for (int l = 0; l < 2; ++l) eb.mark[l] = reinterpret_cast<unsigned*>(take(N * sizeof(unsigned)));
+    return at;
+}
+
 // flux_fits asks for peso = 1 and beta >= 1 (the reference's values, both 1).
 // The colour passes take the other parameters.
 
@@ -909,7 +940,10 @@ LSH_HD void add_edge(const KArgs& a, int i, int j, int kind, const double* f1, c
 // One cell of the Euler-stage update after the flux pass (MODE as volume_finish).
 // `busy` is set where the cell's input or output state is not all +0 or one of
 // its edges is not dry.
-template <int MODE>
+// KEEP (the adjoint's recomputation): the accumulators go to a.acc and, at cells
+// with a wet edge, the partial sums acc[0], acc[3] after the first three colours
+// to a.part; MODE < 0 ends there.
+template <int MODE, bool KEEP = false>
 LSH_HD unsigned long long update_cell(const KArgs& a, int i, int j, double dt, bool& busy) {
     const int nx = a.c.nx, ny = a.c.ny, id = j * nx + i;
     const unsigned char* kh = a.eb.kind[0] + id;
@@ -937,6 +971,11 @@ LSH_HD unsigned long long update_cell(const KArgs& a, int i, int j, double dt, b
         limit[0] = any && limit[0] && limit_near(a, i, j, 0, dt);
         limit[1] = any && limit[1] && limit_near(a, i, j, 1, dt);
     }
+    auto partial = [&](int c) {
+        if (!KEEP || !any) return;
+        a.part[c][0][id] = acc[0];
+        a.part[c][1][id] = acc[3];
+    };
     if (warp_any(any && (limit[0] || limit[1]))) {
         double f[8];
         if (limit[0]) partial_mass<4>(a, i, j, 0, dt, f);
@@ -944,16 +983,27 @@ LSH_HD unsigned long long update_cell(const KArgs& a, int i, int j, double dt, b
         const double* f1 = limit[0] ? f : nullptr;
         const double* f2 = limit[1] ? f + 4 : nullptr;
         add_edge<0, true>(a, i, j, k0, f1, f2, acc);
+        partial(0);
         add_edge<1, true>(a, i, j, k1, f1, f2, acc);
+        partial(1);
         add_edge<2, true>(a, i, j, k2, f1, f2, acc);
+        partial(2);
         add_edge<3, true>(a, i, j, k3, f1, f2, acc);
     } else {
         add_edge<0, false>(a, i, j, k0, nullptr, nullptr, acc);
+        partial(0);
         add_edge<1, false>(a, i, j, k1, nullptr, nullptr, acc);
+        partial(1);
         add_edge<2, false>(a, i, j, k2, nullptr, nullptr, acc);
+        partial(2);
         add_edge<3, false>(a, i, j, k3, nullptr, nullptr, acc);
     }
-    return volume_finish<MODE, true>(a, id, j, dt, wo, acc, &busy);
+    if (KEEP) {
+#pragma unroll
+        for (int k = 0; k < 7; ++k) a.acc[k][id] = acc[k];
+    }
+    if constexpr (MODE < 0) return 0;
+    else return volume_finish<MODE, true>(a, id, j, dt, wo, acc, &busy);
 }
 
 // dt from the largest acc_w / area: 2 CFL / max rate, 1e30 when no cell has a wave speed

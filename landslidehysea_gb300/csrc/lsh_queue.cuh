@@ -1,6 +1,7 @@
 // lsh_queue.cuh -- the device work queue of the batched paths: one
-// persistent launch runs a sequence of passes (reconstruction, the four
-// colour edge passes, the Euler stage) over many scenarios of uneven grids.
+// persistent launch runs a sequence of passes (reconstruction, flux pass and
+// cell update, or the four colour edge passes and the Euler stage) over many
+// scenarios of uneven grids.
 //
 // CTAs of 64 threads pull items -- (pass, scenario, 2-D tile of the
 // single-grid shapes) -- from one queue, in pass order.  An item waits only
@@ -12,12 +13,13 @@
 // item, and when, changes no bit: every scenario is bit-identical to its
 // single-grid run.  The ensemble (lsh_batch.cu) runs a time step this way;
 // the batched adjoint (lsh_adjoint.cu) runs its forward steps and the
-// recomputation of a reversed step (reconstruction with its branch tape,
-// edge passes with their snapshots) this way too.
+// recomputation of a reversed step (with the branch tape, accumulators and
+// partial sums that the reverse sweep reads) this way too.
 #pragma once
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -32,30 +34,32 @@ namespace {
 using lsh::KArgs;
 using lsh::kRateInitBits;
 
-// No branch tape: the forward step's kernels.
-struct NoTape {
-    static constexpr bool kOn = false;
-    __device__ static unsigned run(const KArgs&, int) { return 0u; }
-};
-
 constexpr int kBThreads = 64;    // threads per persistent CTA
-// CTAs per SM the step kernel is compiled for (its register budget: 48 at 20)
+// What the queue's kernel runs.
+enum QueueKind : int { kQColour = 0, kQFlux = 1, kQFluxKeep = 2 };
+// CTAs per SM the step kernel is compiled for: the colour passes 20 (a register
+// budget of 48), the flux pass fewer, since its edges need more registers.
 #ifndef LSH_BATCH_MAXCTAS
 #define LSH_BATCH_MAXCTAS 20
 #endif
-constexpr int kBMaxCtas = LSH_BATCH_MAXCTAS;
+#ifndef LSH_BATCH_FLUX_CTAS
+#define LSH_BATCH_FLUX_CTAS 12
+#endif
+constexpr int kBMaxCtas = LSH_BATCH_MAXCTAS, kBFluxCtas = LSH_BATCH_FLUX_CTAS;
 constexpr int kMaxPasses = 12;
 
 // Tilings of a scenario's passes, 64-thread tiles of the single-grid shapes:
 // horizontal edges of parity 0 / 1 (16 columns x 4 edge lines), vertical
-// edges of parity 0 / 1 (8 edge columns x 8 rows), cells (16 x 4).
-enum BKind : int { kBH0 = 0, kBH1 = 1, kBV0 = 2, kBV1 = 3, kBCell = 4, kBKinds = 5 };
+// edges of parity 0 / 1 (8 edge columns x 8 rows), cells (16 x 4), and for the
+// flux pass the horizontal and the vertical edges of 16 x 4 places.
+enum BKind : int { kBH0 = 0, kBH1 = 1, kBV0 = 2, kBV1 = 3, kBCell = 4, kBFlux = 5, kBKinds = 6 };
 constexpr int kTileHX = 16, kTileHY = 4, kTileVX = 8, kTileVY = 8, kTileCX = 16, kTileCY = 4;
-// What a pass does.
-// kOpReconTape: the reconstruction that also stores the adjoint's branch
-// tape (a.tape); only a kernel instantiated with a tape policy runs it.
+// What a pass does: the colour passes and the Euler stage by MODE, the
+// reconstruction (with its branch tape where a.tape is set), the flux pass and
+// the cell update (kOpUpd<m>: MODE m; kOpUpdEnd: the accumulators alone).
 enum BOp : int {
-    kOpH0 = 0, kOpH1 = 1, kOpV0 = 2, kOpV1 = 3, kOpRecon = 4, kOpVol0 = 5, kOpVol1 = 6, kOpVol2 = 7, kOpReconTape = 8
+    kOpH0 = 0, kOpH1 = 1, kOpV0 = 2, kOpV1 = 3, kOpRecon = 4, kOpVol0 = 5, kOpVol1 = 6, kOpVol2 = 7,
+    kOpFlux = 8, kOpUpd0 = 9, kOpUpd1 = 10, kOpUpd2 = 11, kOpUpdEnd = 12
 };
 
 struct BPass {
@@ -82,14 +86,24 @@ struct BPlan {
     int* abort_flag;        // set when a wait gives up; later waits give up at once
 };
 
-// Cell rows an item of `op` reads (tile row ty of a scenario with ny rows).
+// Rows of its producer's output that an item of `op` reads (tile row ty of a
+// scenario with ny rows): cell rows; for a cell update edge rows, a tile row of
+// flux on either side for the limiter's partial sums.  Whatever an item
+// overwrites (edge planes and marks, slopes, the state) was last read two passes
+// before it by rows that its producer's rows have waited for.
 __device__ __forceinline__ void item_rows(int op, int ty, int ny, int& r0, int& r1) {
     if (op == kOpH0 || op == kOpH1) {
         const int y0 = op + 2 * kTileHY * ty;  // first edge row (parity op)
         r0 = y0 - 1; r1 = y0 + 2 * (kTileHY - 1);
     } else if (op == kOpV0 || op == kOpV1) {
         r0 = kTileVY * ty; r1 = r0 + kTileVY - 1;
-    } else if (op == kOpRecon || op == kOpReconTape) {
+    } else if (op == kOpFlux) {
+        r0 = kTileCY * ty - 1; r1 = kTileCY * ty + kTileCY - 1;
+    } else if (op >= kOpUpd0) {
+        r0 = max(kTileCY * (ty - 1), 0);
+        r1 = min(kTileCY * (ty + 2) - 1, ny);
+        return;
+    } else if (op == kOpRecon) {
         r0 = kTileCY * ty - 1; r1 = kTileCY * ty + kTileCY;
     } else {
         r0 = kTileCY * ty; r1 = r0 + kTileCY - 1;
@@ -101,7 +115,7 @@ __device__ __forceinline__ void item_rows(int op, int ty, int ny, int& r0, int& 
 // Tile rows of a pass of `kind` that write cell rows [r0, r1].
 __device__ __forceinline__ void producer_rows(int kind, int r0, int r1, int& t0, int& t1) {
     if (kind == kBV0 || kind == kBV1) { t0 = r0 / kTileVY; t1 = r1 / kTileVY; }
-    else if (kind == kBCell) { t0 = r0 / kTileCY; t1 = r1 / kTileCY; }
+    else if (kind >= kBCell) { t0 = r0 / kTileCY; t1 = r1 / kTileCY; }
     else {
         // horizontal edge row y = p + 2 t writes cell rows y - 1 and y
         const int p = kind;
@@ -155,7 +169,7 @@ __device__ __forceinline__ void queue_done(unsigned* c, unsigned n = 1u) {
 // One item's work: the single-grid kernels' per-thread bodies on one tile.
 // Returns the thread's dt-rate bits for the Euler stages that take the rate
 // maximum (kOpVol0, kOpVol1), kRateInitBits otherwise; the caller reduces them.
-template <int ORDER, int OP, class TAPE>
+template <int ORDER, int OP, bool KEEP>
 __device__ __forceinline__ unsigned long long item_work(const KArgs& a, int tx, int ty, double dt) {
     const int nx = a.c.nx, ny = a.c.ny, tid = threadIdx.x;
     if constexpr (OP == kOpH0 || OP == kOpH1) {
@@ -166,14 +180,23 @@ __device__ __forceinline__ unsigned long long item_work(const KArgs& a, int tx, 
         const int par = OP - kOpV0;
         const int x = par + 2 * (tx * kTileVX + tid % kTileVX), y = ty * kTileVY + tid / kTileVX;
         if (x <= nx && y < ny) lsh::do_edge<1, false, ORDER>(a, x, y, dt);
+    } else if constexpr (OP == kOpFlux) {
+        const int x = (tx >> 1) * kTileCX + tid % kTileCX, y = ty * kTileCY + tid / kTileCX, dir = tx & 1;
+        if (dir ? (x <= nx && y < ny) : (x < nx && y <= ny)) lsh::flux_edge<ORDER>(a, dir, x, y, dt);
     } else {
         const int i = tx * kTileCX + tid % kTileCX, j = ty * kTileCY + tid / kTileCX;
         const bool in = (i < nx && j < ny);
         if constexpr (OP == kOpRecon) {
-            if (in) lsh::recon_cell(a, j * nx + i);
-        } else if constexpr (OP == kOpReconTape) {
-            if constexpr (TAPE::kOn)
-                if (in) a.tape[j * nx + i] = TAPE::run(a, j * nx + i);
+            if (in) {
+                const unsigned t = lsh::recon_cell(a, j * nx + i);
+                if (a.tape) a.tape[j * nx + i] = t;
+            }
+        } else if constexpr (OP >= kOpUpd0) {
+            constexpr int MODE = (OP == kOpUpdEnd) ? -1 : OP - kOpUpd0;
+            unsigned long long bits = kRateInitBits;
+            bool busy = false;
+            if (in) bits = lsh::update_cell<MODE, KEEP>(a, i, j, dt, busy);
+            return (MODE == 0 || MODE == 1) ? bits : kRateInitBits;
         } else {
             constexpr int MODE = OP - kOpVol0;
             unsigned long long bits = kRateInitBits;
@@ -185,11 +208,11 @@ __device__ __forceinline__ unsigned long long item_work(const KArgs& a, int tx, 
 }
 
 // A run of tiles tx0 .. tx0 + run - 1 of one tile row; the largest rate bits.
-template <int ORDER, int OP, class TAPE>
+template <int ORDER, int OP, bool KEEP>
 __device__ __forceinline__ unsigned long long run_work(const KArgs& a, int tx0, int run, int ty, double dt) {
     unsigned long long bits = kRateInitBits;
     for (int j = 0; j < run; ++j) {
-        const unsigned long long b = item_work<ORDER, OP, TAPE>(a, tx0 + j, ty, dt);
+        const unsigned long long b = item_work<ORDER, OP, KEEP>(a, tx0 + j, ty, dt);
         bits = (b > bits) ? b : bits;
     }
     return bits;
@@ -205,8 +228,8 @@ __device__ __forceinline__ unsigned long long run_work(const KArgs& a, int tx0, 
 // Waits are bounded (~2 s of %globaltimer); one that runs out sets
 // LSH_ERR_TIMEOUT on its scenario and the batch's abort flag, and later
 // waits give up at once.
-template <int ORDER, class TAPE = NoTape>
-__global__ void __launch_bounds__(kBThreads, kBMaxCtas) k_batch_step(BPlan P, int fetch) {
+template <int ORDER, int KIND>
+__global__ void __launch_bounds__(kBThreads, KIND == kQColour ? kBMaxCtas : kBFluxCtas) k_batch_step(BPlan P, int fetch) {
     __shared__ __align__(16) unsigned long long sargs[(sizeof(KArgs) + 7) / 8];
     __shared__ int s_first, s_pass, s_scen, s_tile, s_ntx, s_copy, s_run;
     // the last decoded (pass, scenario): its items [s_lo, s_hi) of the queue,
@@ -282,23 +305,35 @@ __global__ void __launch_bounds__(kBThreads, kBMaxCtas) k_batch_step(BPlan P, in
             if (live) {
                 const double dt = a.tm->dt;
                 unsigned long long bits = kRateInitBits;
-                switch (ps.op) {
-                    case kOpH0: run_work<ORDER, kOpH0, TAPE>(a, tx, run, ty, dt); break;
-                    case kOpH1: run_work<ORDER, kOpH1, TAPE>(a, tx, run, ty, dt); break;
-                    case kOpV0: run_work<ORDER, kOpV0, TAPE>(a, tx, run, ty, dt); break;
-                    case kOpV1: run_work<ORDER, kOpV1, TAPE>(a, tx, run, ty, dt); break;
-                    default:
-                        if constexpr (ORDER == 1) {
-                            bits = run_work<ORDER, kOpVol0, TAPE>(a, tx, run, ty, dt);
-                        } else {
-                            if (ps.op == kOpRecon) run_work<ORDER, kOpRecon, TAPE>(a, tx, run, ty, dt);
-                            else if (TAPE::kOn && ps.op == kOpReconTape) run_work<ORDER, kOpReconTape, TAPE>(a, tx, run, ty, dt);
-                            else if (ps.op == kOpVol1) bits = run_work<ORDER, kOpVol1, TAPE>(a, tx, run, ty, dt);
-                            else run_work<ORDER, kOpVol2, TAPE>(a, tx, run, ty, dt);
-                        }
-                        break;
+                constexpr bool K = (KIND == kQFluxKeep);
+                if constexpr (KIND == kQColour) {
+                    switch (ps.op) {
+                        case kOpH0: run_work<ORDER, kOpH0, K>(a, tx, run, ty, dt); break;
+                        case kOpH1: run_work<ORDER, kOpH1, K>(a, tx, run, ty, dt); break;
+                        case kOpV0: run_work<ORDER, kOpV0, K>(a, tx, run, ty, dt); break;
+                        case kOpV1: run_work<ORDER, kOpV1, K>(a, tx, run, ty, dt); break;
+                        default:
+                            if constexpr (ORDER == 1) {
+                                bits = run_work<ORDER, kOpVol0, K>(a, tx, run, ty, dt);
+                            } else {
+                                if (ps.op == kOpRecon) run_work<ORDER, kOpRecon, K>(a, tx, run, ty, dt);
+                                else if (ps.op == kOpVol1) bits = run_work<ORDER, kOpVol1, K>(a, tx, run, ty, dt);
+                                else run_work<ORDER, kOpVol2, K>(a, tx, run, ty, dt);
+                            }
+                            break;
+                    }
+                } else {
+                    // stage 2 of a recomputation, and at order 1 its only stage, end at the accumulators
+                    constexpr int kLast = K ? kOpUpdEnd : (ORDER == 1 ? kOpUpd0 : kOpUpd2);
+                    if (ps.op == kOpFlux) run_work<ORDER, kOpFlux, K>(a, tx, run, ty, dt);
+                    else if (ps.op == kLast) bits = run_work<ORDER, kLast, K>(a, tx, run, ty, dt);
+                    else if constexpr (ORDER == 2) {
+                        if (ps.op == kOpRecon) run_work<ORDER, kOpRecon, K>(a, tx, run, ty, dt);
+                        else bits = run_work<ORDER, kOpUpd1, K>(a, tx, run, ty, dt);
+                    }
                 }
-                if (ps.op == kOpVol0 || ps.op == kOpVol1) lsh::block_max_bits<kBThreads>(bits, &a.tm->rmax_bits);
+                if (ps.op == kOpVol0 || ps.op == kOpVol1 || ps.op == kOpUpd0 || ps.op == kOpUpd1)
+                    lsh::block_max_bits<kBThreads>(bits, &a.tm->rmax_bits);
             }
             __syncthreads();  // the run's writes are done, and sargs may be refilled
             if (tid == 0) {
@@ -339,6 +374,9 @@ inline void queue_tiles(int nx, int ny, int kind, int& tx, int& ty) {
     } else if (kind == kBV0 || kind == kBV1) {
         tx = ((nx - (kind - kBV0)) / 2 + 1 + kTileVX - 1) / kTileVX;
         ty = (ny + kTileVY - 1) / kTileVY;
+    } else if (kind == kBFlux) {
+        tx = 2 * (nx / kTileCX + 1);  // both directions; edge places 0 .. nx, 0 .. ny
+        ty = ny / kTileCY + 1;
     } else {
         tx = (nx + kTileCX - 1) / kTileCX;
         ty = (ny + kTileCY - 1) / kTileCY;
@@ -348,6 +386,39 @@ inline void queue_tiles(int nx, int ny, int kind, int& tx, int& ty) {
 struct QPassSpec {
     int op, kind, var;
 };
+
+// A step's passes on the flux pass (`keep`: the recomputation's, arguments 0 and
+// 1 the stages') or on the colour passes.
+inline std::vector<QPassSpec> flux_queue_passes(int order, bool keep) {
+    std::vector<QPassSpec> v;
+    for (int st = 0; st < order; ++st) {
+        if (order == 2) v.push_back({kOpRecon, kBCell, st});
+        v.push_back({kOpFlux, kBFlux, st});
+        const int last = keep ? kOpUpdEnd : (order == 1 ? kOpUpd0 : kOpUpd2);
+        v.push_back({st + 1 < order ? int(kOpUpd1) : last, kBCell, st});
+    }
+    return v;
+}
+inline std::vector<QPassSpec> colour_queue_passes(int order) {
+    std::vector<QPassSpec> v;
+    for (int st = 0; st < order; ++st) {
+        if (order == 2) v.push_back({kOpRecon, kBCell, st});
+        v.push_back({kOpH0, kBH0, st});
+        v.push_back({kOpH1, kBH1, st});
+        v.push_back({kOpV0, kBV0, st});
+        v.push_back({kOpV1, kBV1, st});
+        v.push_back({(order == 1) ? kOpVol0 : (st == 0 ? kOpVol1 : kOpVol2), kBCell, st});
+    }
+    return v;
+}
+
+// The step's launch: CTAs beyond those the kernel is compiled for would only wait.
+template <int KIND>
+inline void launch_queue(const BPlan& p, int order, int sms, int ctas, int fetch, cudaStream_t s) {
+    const int grid = std::max(1, sms * std::min(std::max(ctas, 1), KIND == kQColour ? kBMaxCtas : kBFluxCtas));
+    if (order == 1) k_batch_step<1, KIND><<<grid, kBThreads, 0, s>>>(p, fetch);
+    else k_batch_step<2, KIND><<<grid, kBThreads, 0, s>>>(p, fetch);
+}
 
 // The plan of a chain of passes (each reading what the one before it wrote)
 // over scenarios of nx[s] x ny[s] cells: its items, counters and device

@@ -1,11 +1,12 @@
 // TEST INFRASTRUCTURE: the flux pass and cell update (flux_edge, update_cell)
 // against the colour passes (do_edge, volume_cell), both compiled for the
 // host: the same steps from the same state, every field and rate bit for bit.
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <vector>
 
-#include "../../landslidehysea_gb300/csrc/lsh_passes.cuh"
+#include "../../landslidehysea_gb300/csrc/lsh_adjoint.cuh"
 #include "../../landslidehysea_gb300/csrc/lsh_setup.h"
 
 using namespace lsh;
@@ -106,6 +107,47 @@ unsigned long long step(Grid& g, bool flux, double dt, long long* marked) {
 }  // namespace
 
 extern "C" {
+
+// One recomputed stage of step dt from W both ways (update_cell keeping its accumulators; the colour passes, copied
+// between): the number of accumulators, partial sums at cells with a wet edge, and branch tapes that differ.
+long long fluxc_keep(const lsh_params* p, const double* const* W, double dt) {
+    Grid a(*p, W), b(*p, W);
+    const int nx = p->nx, ny = p->ny, order = p->order;
+    const size_t N = a.N;
+    KArgs ka = a.args(0), kb = b.args(0);
+    ka.eb.depth[0] = ka.W[0]; ka.eb.depth[1] = ka.W[3];  // nothing is updated in place
+    ka.eb.depth_out[0] = ka.eb.depth_out[1] = nullptr;
+    long long bad = 0;
+    Vec sa[3][2], sb[3][2];
+    for (int c = 0; c < 3; ++c)
+        for (int l = 0; l < 2; ++l) { sa[c][l].assign(N, 7.0); sb[c][l].assign(N, 0.0); ka.part[c][l] = sa[c][l].data(); }
+    for (int k = 0; k < 7; ++k) std::fill(a.acc[k].begin(), a.acc[k].end(), 7.0);
+    if (order == 2)
+        for (size_t id = 0; id < N; ++id) {
+            bad += recon_cell(ka, int(id)) != recon_tape_cell(kb.W, nx, ny, int(id));
+            recon_cell(kb, int(id));
+        }
+    auto flux = [&](int dir, int x, int y) { order == 2 ? flux_edge<2>(ka, dir, x, y, dt) : flux_edge<1>(ka, dir, x, y, dt); };
+    for (int y = 0; y <= ny; ++y) for (int x = 0; x < nx; ++x) flux(0, x, y);
+    for (int y = 0; y < ny; ++y) for (int x = 0; x <= nx; ++x) flux(1, x, y);
+    for (int j = 0; j < ny; ++j) for (int i = 0; i < nx; ++i) { bool busy = false; update_cell<-1, true>(ka, i, j, dt, busy); }
+    auto copy = [&](int c) { for (int l = 0; l < 2; ++l) sb[c][l] = b.acc[3 * l]; };
+    for (int y = 0; y <= ny; y += 2) for (int x = 0; x < nx; ++x) order == 2 ? do_edge<0, true, 2>(kb, x, y, dt) : do_edge<0, true, 1>(kb, x, y, dt);
+    copy(0);
+    for (int y = 1; y <= ny; y += 2) for (int x = 0; x < nx; ++x) order == 2 ? do_edge<0, false, 2>(kb, x, y, dt) : do_edge<0, false, 1>(kb, x, y, dt);
+    copy(1);
+    for (int y = 0; y < ny; ++y) for (int x = 0; x <= nx; x += 2) order == 2 ? do_edge<1, false, 2>(kb, x, y, dt) : do_edge<1, false, 1>(kb, x, y, dt);
+    copy(2);
+    for (int y = 0; y < ny; ++y) for (int x = 1; x <= nx; x += 2) order == 2 ? do_edge<1, false, 2>(kb, x, y, dt) : do_edge<1, false, 1>(kb, x, y, dt);
+    for (size_t id = 0; id < N; ++id) {
+        const size_t j = id / nx;
+        const bool wet = a.kh[id] | a.kh[id + nx] | a.kv[id + j] | a.kv[id + j + 1];
+        for (int k = 0; k < 7; ++k) bad += lshm::bits_of(a.acc[k][id]) != lshm::bits_of(b.acc[k][id]);
+        for (int c = 0; c < 3 && wet; ++c)
+            for (int l = 0; l < 2; ++l) bad += lshm::bits_of(sa[c][l][id]) != lshm::bits_of(sb[c][l][id]);
+    }
+    return bad;
+}
 
 // Runs `nsteps` steps of size dt (the lagged CFL step when dt <= 0) both ways from W (7 arrays); returns the number of
 // values that differ in their bits; *marked: cells around which the limiter was evaluated.  A run ends with its first
