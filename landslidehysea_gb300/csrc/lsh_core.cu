@@ -4,18 +4,20 @@
 // Layout in HBM: FP64 structure-of-arrays, one array of nx*ny doubles per
 // variable (h1 q1x q1y h2 q2x q2y H), row-major (cell j*nx + i).  The step:
 //   order 1 (the reference scheme, ShallowWater.cu:391-442):
-//     4 colour passes over edges (hor-even, hor-odd, ver-even, ver-odd),
-//     accumulating into 7 SoA accumulators; the first pass writes instead of
-//     accumulating, which replaces the reference's two cudaMemset per step;
-//     then one volume kernel updates the state IN PLACE (each thread owns
-//     one cell), folds the per-cell dt into a block min and one 64-bit
-//     atomicMin on the bit pattern of the (positive) double, and a 1-thread
-//     kernel advances t and dt on the device.  No host sync per step, no
-//     texture copy-back (ShallowWater.cu:447-454), so a run of steps is one
-//     CUDA graph launch.
-//   order 2: minmod reconstruction kernel + the same 4 passes on face values
-//     + volume kernel, twice (Heun / TVD-RK2), the second volume kernel
-//     averaging with the step's initial state.
+//     a flux pass over all edges (one thread each) writes every edge's terms
+//     to planes; the cell update (one thread per cell) adds its four edges'
+//     terms in the reference's colour order, with the positivity limiter,
+//     updates the state IN PLACE, folds the cells' rates into one 64-bit
+//     atomicMax on the bit pattern of the (non-negative) double; a clock
+//     kernel advances t and dt on the device and lists the tiles that the
+//     next step has to visit.  No host sync per step, no texture copy-back
+//     (ShallowWater.cu:447-454), so a run of steps is one CUDA graph launch.
+//   order 2: minmod reconstruction kernel + the same two passes on face
+//     values, twice (Heun / TVD-RK2), the second update averaging with the
+//     step's initial state.
+//   Parameters that flux_fits refuses, and a device without room for the edge
+//   planes, take the reference's 4 colour passes (hor-even, hor-odd, ver-even,
+//   ver-odd) into 7 accumulators and a volume kernel, with the same bits.
 // The FP64 math lives in lsh_scheme.cuh.
 
 #include <cuda_runtime.h>

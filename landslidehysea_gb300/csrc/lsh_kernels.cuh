@@ -544,7 +544,11 @@ __global__ void __launch_bounds__(32 * kCellWarps, kSlopesBlocks[SMALL])
     int tx, ty, half, i, j;
     if (!tile_of(m, u0, kCellWarps, tx, ty)) return;
     tile_begin(d, m, a.tm, ty, 1);
-    if (tile_cell(a, tx, ty, u0, half, i, j)) lsh::recon_cell(a, j * a.c.nx + i);
+    if (tile_cell(a, tx, ty, u0, half, i, j)) {
+        const int id = j * a.c.nx + i;
+        if (SMALL) lsh::recon_cell_loaded(a, id);
+        else lsh::recon_cell(a, id);
+    }
     tile_end(d, ty);
 }
 

@@ -442,6 +442,24 @@ LSH_HD unsigned recon_cell(const KArgs& a, int id) {
     return recon_cell_from(a, id, i, j, [&](int k, int di, int dj) -> double { return a.W[k][id + di + dj * nx]; });
 }
 
+// The same with its 35 values loaded at once (a neighbour outside the grid is
+// the cell itself, and not read): for a small grid, whose warps cannot hide
+// loads that wait for the tests of others (64^2: 15.5 -> 10.5 us a launch, 156
+// -> 141 us a step; it needs 126 registers, so a large grid keeps the chain).
+LSH_HD unsigned recon_cell_loaded(const KArgs& a, int id) {
+    const int nx = a.c.nx, ny = a.c.ny;
+    const int j = id / nx, i = id - j * nx;
+    const int at[5] = {id, id - (i > 0), id + (i < nx - 1), id - (j > 0 ? nx : 0), id + (j < ny - 1 ? nx : 0)};
+    double v[7][5];
+#pragma unroll
+    for (int k = 0; k < 7; ++k)
+#pragma unroll
+        for (int n = 0; n < 5; ++n) v[k][n] = a.W[k][at[n]];
+    return recon_cell_from(a, id, i, j, [&](int k, int di, int dj) -> double {
+        return v[k][di < 0 ? 1 : di > 0 ? 2 : dj < 0 ? 3 : dj > 0 ? 4 : 0];
+    });
+}
+
 #if defined(__CUDACC__)
 // Block max of the per-cell rates (non-negative doubles order like their bit
 // patterns), then one 64-bit atomicMax per block.
@@ -956,6 +974,15 @@ LSH_HD unsigned long long update_cell(const KArgs& a, int i, int j, double dt, b
     for (int k = 0; k < 6; ++k) wo[k] = a.W[k][id];
 #pragma unroll
     for (int k = 3; k < 6; ++k) acc[k] = 0.0;
+    if (KEEP && !warp_any(any)) {
+        // nothing but dry edges: +0 all round (the recomputation visits every
+        // tile; in the listed ones of a step the test cost more than it saved,
+        // 104 against 108 us at 2048^2)
+#pragma unroll
+        for (int k = 0; k < 7; ++k) a.acc[k][id] = acc[k] = 0.0;
+        if constexpr (MODE < 0) return 0;
+        else return volume_finish<MODE, true>(a, id, j, dt, wo, acc, &busy);
+    }
     // an edge is limited only where one of its two cells is marked
     bool limit[2];
     const unsigned now = stage_mark(a);

@@ -125,7 +125,7 @@ long long fluxc_keep(const lsh_params* p, const double* const* W, double dt) {
     if (order == 2)
         for (size_t id = 0; id < N; ++id) {
             bad += recon_cell(ka, int(id)) != recon_tape_cell(kb.W, nx, ny, int(id));
-            recon_cell(kb, int(id));
+            bad += recon_cell_loaded(kb, int(id)) != recon_tape_cell(kb.W, nx, ny, int(id));
         }
     auto flux = [&](int dir, int x, int y) { order == 2 ? flux_edge<2>(ka, dir, x, y, dt) : flux_edge<1>(ka, dir, x, y, dt); };
     for (int y = 0; y <= ny; ++y) for (int x = 0; x < nx; ++x) flux(0, x, y);
