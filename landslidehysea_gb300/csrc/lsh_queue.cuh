@@ -38,7 +38,9 @@ constexpr int kBThreads = 64;    // threads per persistent CTA
 // What the queue's kernel runs.
 enum QueueKind : int { kQColour = 0, kQFlux = 1, kQFluxKeep = 2 };
 // CTAs per SM the step kernel is compiled for: the colour passes 20 (a register
-// budget of 48), the flux pass fewer, since its edges need more registers.
+// budget of 48), the flux pass fewer, since its edges need more registers (ms a
+// step of the 10 wet shelves of 128 to 512 squared: 1.096 at 10, 1.095 at 12,
+// 1.095 at 16).
 #ifndef LSH_BATCH_MAXCTAS
 #define LSH_BATCH_MAXCTAS 20
 #endif
@@ -80,6 +82,7 @@ struct BPlan {
     const int* tile_pre;    // [kind][n + 1]: first tile of each scenario (prefix sums)
     const int* row_pre;     // [kind][n + 1]: first tile row of each scenario
     const int* tiles_x;     // [kind][n]: tiles per tile row
+    const int* ny;          // [n]: cell rows of each scenario
     const KArgs* args;      // [var][n]: [n] stage 1, [n, 2n) stage 2, ...
     unsigned* ctr;          // completion counters: per pass, per scenario tile row
     unsigned* head;         // the step's queue head
@@ -124,14 +127,15 @@ __device__ __forceinline__ void producer_rows(int kind, int r0, int r1, int& t0,
     }
 }
 
-// Waits (one thread) until counters c[t0..t1] reach `target`.  Bounded:
+// Waits (one thread) until counters c[t0], c[t0 + step], ... up to t1 reach
+// `target`.  Bounded:
 // after ~2 s of %globaltimer from `start` (0: from the first miss) it sets
 // *abort_flag and gives up, as does every later wait that finds the flag
 // set.  Returns true when it gave up.
 __device__ __forceinline__ bool queue_wait(const unsigned* c, int t0, int t1, unsigned target, int* abort_flag,
-                                           unsigned long long& start) {
+                                           unsigned long long& start, int step = 1) {
     volatile int* abort_v = abort_flag;
-    for (int r = t0; r <= t1; ++r) {
+    for (int r = t0; r <= t1; r += step) {
         unsigned ns = 32;
         for (;;) {
             unsigned v;
@@ -149,7 +153,7 @@ __device__ __forceinline__ bool queue_wait(const unsigned* c, int t0, int t1, un
     return false;
 }
 
-// The producer rows a CTA's thread 0 last found complete: (pass, scenario,
+// The producer rows a CTA last found complete: (pass, scenario,
 // tile rows [t0, t1]).  Counters only grow within a launch, so an item whose
 // wait falls inside that range needs no new acquire: the earlier acquire,
 // followed by the block barrier, already orders its reads after the
@@ -231,22 +235,34 @@ __device__ __forceinline__ unsigned long long run_work(const KArgs& a, int tx0, 
 template <int ORDER, int KIND>
 __global__ void __launch_bounds__(kBThreads, KIND == kQColour ? kBMaxCtas : kBFluxCtas) k_batch_step(BPlan P, int fetch) {
     __shared__ __align__(16) unsigned long long sargs[(sizeof(KArgs) + 7) / 8];
-    __shared__ int s_first, s_pass, s_scen, s_tile, s_ntx, s_copy, s_run;
+    __shared__ unsigned s_first;
+    __shared__ int s_pass, s_scen, s_tile, s_ntx, s_copy, s_run, s_live;
+    __shared__ double s_dt;
     // the last decoded (pass, scenario): its items [s_lo, s_hi) of the queue,
     // and the arguments held in sargs (var * n + scenario, -1: none).
-    // Consecutive items of the queue share them, so most runs skip the
+    // Consecutive items of the queue share them, so runs of a fetch skip the
     // scenario search and the argument copy.
     __shared__ int s_lo, s_hi, s_args_key;
     const KArgs& a = *reinterpret_cast<const KArgs*>(sargs);
     const int tid = threadIdx.x;
-    WaitCache wc;  // thread 0's
-    if (tid == 0) { s_lo = 0; s_hi = 0; s_args_key = -1; }
+    WaitCache wc;  // the same in every thread
+    unsigned ahead = 0;  // thread 0: the next fetch
+    if (tid == 0) {
+        s_lo = 0;
+        s_hi = 0;
+        s_args_key = -1;
+        ahead = atomicAdd(P.head, (unsigned)fetch);
+    }
     for (;;) {
-        if (tid == 0) s_first = (int)atomicAdd(P.head, (unsigned)fetch);
+        if (tid == 0) s_first = ahead;
         __syncthreads();
-        const int first = s_first;
-        if (first >= P.total_items) break;
-        const int last = min(first + fetch, P.total_items);
+        const unsigned taken = s_first;
+        if (taken >= (unsigned)P.total_items) break;
+        // the fetch after this one: its round trip passes behind this one's work
+        // (a CTA finishes what it took in queue order, so the earliest
+        // unfinished item is still being worked on)
+        if (tid == 0) ahead = atomicAdd(P.head, (unsigned)fetch);
+        const int first = (int)taken, last = min(first + fetch, P.total_items);
         for (int it = first; it < last;) {
             if (tid == 0) {
                 if (it < s_lo || it >= s_hi) {
@@ -277,17 +293,24 @@ __global__ void __launch_bounds__(kBThreads, KIND == kQColour ? kBMaxCtas : kBFl
             __syncthreads();
             const int p = s_pass, s = s_scen, t = s_tile, ntx = s_ntx, run = s_run;
             const BPass ps = P.pass[p];
-            if (s_copy) {
-                const unsigned long long* src = reinterpret_cast<const unsigned long long*>(P.args + ps.var * P.n + s);
-                for (int k = tid; k < (int)((sizeof(KArgs) + 7) / 8); k += kBThreads) sargs[k] = src[k];
-                __syncthreads();
-            }
             const int ty = t / ntx, tx = t - ty * ntx;
-            const bool live = !a.tm->done;  // uniform: the clock changes between steps only
-            if (live && ps.prod >= 0 && tid == 0) {
+            // At once, each a round trip to L2: the arguments, the scenario's clock
+            // (which changes between steps only) and the producer's rows, one
+            // thread a row.
+            if (s_copy) {
+                const KArgs* from = P.args + ps.var * P.n + s;
+                const unsigned long long* src = reinterpret_cast<const unsigned long long*>(from);
+                for (int k = tid; k < (int)((sizeof(KArgs) + 7) / 8); k += kBThreads) sargs[k] = src[k];
+                if (tid == kBThreads - 1) {
+                    const lsh::TimeRec* tm = from->tm;
+                    s_live = !tm->done;
+                    s_dt = tm->dt;
+                }
+            }
+            if (ps.prod >= 0) {
                 const BPass pp = P.pass[ps.prod];
                 int r0, r1, t0, t1;
-                item_rows(ps.op, ty, a.c.ny, r0, r1);
+                item_rows(ps.op, ty, P.ny[s], r0, r1);
                 producer_rows(pp.kind, r0, r1, t0, t1);
                 const int rbase = P.row_pre[pp.kind * (P.n + 1) + s];
                 const int nrows = P.row_pre[pp.kind * (P.n + 1) + s + 1] - rbase;
@@ -295,15 +318,16 @@ __global__ void __launch_bounds__(kBThreads, KIND == kQColour ? kBMaxCtas : kBFl
                 t1 = min(t1, nrows - 1);
                 if (!wc.covers(ps.prod, s, t0, t1)) {
                     unsigned long long start = 0;
-                    const bool gave_up = queue_wait(P.ctr + pp.ctr_off + rbase, t0, t1,
-                                                    (unsigned)P.tiles_x[pp.kind * P.n + s], P.abort_flag, start);
-                    if (gave_up) atomicOr(&a.tm->err, 1 << LSH_ERR_TIMEOUT);
-                    else wc.set(ps.prod, s, t0, t1);
+                    if (queue_wait(P.ctr + pp.ctr_off + rbase, t0 + tid, t1, (unsigned)P.tiles_x[pp.kind * P.n + s],
+                                   P.abort_flag, start, kBThreads))
+                        atomicOr(&P.args[ps.var * P.n + s].tm->err, 1 << LSH_ERR_TIMEOUT);
+                    wc.set(ps.prod, s, t0, t1);
                 }
             }
             __syncthreads();
+            const bool live = s_live;  // uniform
             if (live) {
-                const double dt = a.tm->dt;
+                const double dt = s_dt;
                 unsigned long long bits = kRateInitBits;
                 constexpr bool K = (KIND == kQFluxKeep);
                 if constexpr (KIND == kQColour) {
@@ -429,6 +453,7 @@ inline int build_queue_plan(const std::vector<int>& nx, const std::vector<int>& 
     const int n = (int)nx.size();
     if ((int)passes.size() > kMaxPasses) { lsh::set_last_error("queue plan: too many passes"); return LSH_ERR_INVALID; }
     std::vector<int> tile_pre(size_t(kBKinds) * (n + 1)), row_pre(size_t(kBKinds) * (n + 1)), tiles_x(size_t(kBKinds) * n);
+    tiles_x.insert(tiles_x.end(), ny.begin(), ny.end());  // the rows table behind it
     long long kind_tiles[kBKinds], kind_rows[kBKinds];
     for (int k = 0; k < kBKinds; ++k) {
         long long tsum = 0, rsum = 0;
@@ -487,6 +512,7 @@ inline int build_queue_plan(const std::vector<int>& nx, const std::vector<int>& 
     P0.tile_pre = ti;
     P0.row_pre = ti + tile_pre.size();
     P0.tiles_x = ti + tile_pre.size() + row_pre.size();
+    P0.ny = P0.tiles_x + size_t(kBKinds) * n;
     char* rest = static_cast<char*>(*mem) + ((tbytes + 255) & ~size_t(255));
     P0.ctr = reinterpret_cast<unsigned*>(rest);
     P0.head = reinterpret_cast<unsigned*>(rest + size_t(ctrs) * sizeof(unsigned));
