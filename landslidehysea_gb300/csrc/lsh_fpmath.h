@@ -137,6 +137,17 @@ LSH_HD void rare() {
 #endif
 }
 
+// Keeps the loads of its arguments before it, and so at once: the compiler
+// would move each behind the tests that come before its use.
+#if defined(__CUDA_ARCH__)
+LSH_HD void pin(double& x) { asm volatile("" : "+d"(x)); }
+LSH_HD void pin(int& x) { asm volatile("" : "+r"(x)); }
+LSH_HD void pin(unsigned& x) { asm volatile("" : "+r"(x)); }
+template <class... T> LSH_HD void together(T&... x) { (pin(x), ...); }
+#else
+template <class... T> LSH_HD void together(T&...) {}
+#endif
+
 // c ? -x : x by flipping the sign bit (integer pipe): the bits of -x
 LSH_HD double neg_if(double x, bool c) {
     uint32_t lo, hi;

@@ -445,7 +445,7 @@ LSH_HD unsigned recon_cell(const KArgs& a, int id) {
 // The same with its 35 values loaded at once (a neighbour outside the grid is
 // the cell itself, and not read): for a small grid, whose warps cannot hide
 // loads that wait for the tests of others (64^2: 15.5 -> 10.5 us a launch, 156
-// -> 141 us a step; it needs 126 registers, so a large grid keeps the chain).
+// -> 141 us a step; it needs 84 registers, so a large grid keeps the chain).
 LSH_HD unsigned recon_cell_loaded(const KArgs& a, int id) {
     const int nx = a.c.nx, ny = a.c.ny;
     const int j = id / nx, i = id - j * nx;
@@ -893,13 +893,19 @@ LSH_HD double limited_mass(const KArgs& a, int i, int j, int layer, double dt, d
     const CellEdge e = cell_edge<P>(i, j);
     const size_t at = (size_t)e.y * (a.c.nx + DIR) + e.x, np = a.eb.plane[DIR];
     if (factor) *factor = 1.0;
-    if (a.eb.kind[DIR][at] <= layer) return 0.0;
-    const double m = a.eb.q[DIR][at + (layer ? 6 : 0) * np], p = a.eb.q[DIR][at + (layer ? 9 : 3) * np];
-    const double own = e.second ? p : m;
     const EdgeSides s = edge_sides<DIR>(a, e.x, e.y);
+    const int id1 = s.interior ? s.id1 : s.id0, row1 = s.interior ? s.row1 : s.row0;
     const unsigned now = stage_mark(a);
-    const unsigned* mark = a.eb.mark[layer];
-    if (!(mark[s.id0] == now || (s.interior && mark[s.id1] == now))) return own;
+    // all that the edge may need, at once (behind each other's tests: 1024^2
+    // fjord 357 against 350 us a step)
+    int kind = a.eb.kind[DIR][at];
+    double m = a.eb.q[DIR][at + (layer ? 6 : 0) * np], p = a.eb.q[DIR][at + (layer ? 9 : 3) * np];
+    unsigned mark0 = a.eb.mark[layer][s.id0], mark1 = a.eb.mark[layer][id1];
+    double h0 = a.eb.depth[layer][s.id0], h1 = a.eb.depth[layer][id1];
+    lshm::together(kind, m, p, mark0, mark1, h0, h1);
+    if (kind <= layer) return 0.0;
+    const double own = e.second ? p : m;
+    if (!(mark0 == now || mark1 == now)) return own;
     if (!gt0(m) && !(s.interior && gt0(p))) return own;
     // the limiter reads the partial sum of a cell that loses: mostly one of the two
     double other = 0.0;
@@ -907,10 +913,8 @@ LSH_HD double limited_mass(const KArgs& a, int i, int j, int layer, double dt, d
         const int io = e.second ? s.id0 - s.row0 * a.c.nx : s.id1 - s.row1 * a.c.nx;
         other = partial_mass<P>(a, io, e.second ? s.row0 : s.row1, layer, dt, nullptr);
     }
-    const int row1 = s.interior ? s.row1 : s.row0;
-    const double f = limiter(m, p, s.interior, a.eb.depth[layer][s.id0], e.second ? other : acc, a.geo.area[s.row0],
-                             a.geo.inv_area[s.row0], s.interior ? a.eb.depth[layer][s.id1] : 0.0,
-                             e.second ? acc : other, a.geo.area[row1], a.geo.inv_area[row1], dt, a.c);
+    const double f = limiter(m, p, s.interior, h0, e.second ? other : acc, a.geo.area[s.row0], a.geo.inv_area[s.row0],
+                             h1, e.second ? acc : other, a.geo.area[row1], a.geo.inv_area[row1], dt, a.c);
     if (factor) *factor = f;
     return (lshm::bits_of(f) != lshm::bits_of(1.0)) ? f * own : own;
 }
