@@ -3,8 +3,8 @@
 //
 // Every scenario keeps its own parameters, geometry, state and device clock
 // (t, dt), in one slab.  A step runs the same passes as the single-grid path
-// (reconstruction, 4 colour edge passes, Euler stage; twice at second
-// order), with the same device code (lsh_passes.cuh), but the whole step of
+// (reconstruction, flux pass, cell update; twice at second order), with the
+// same device code (lsh_passes.cuh), but the whole step of
 // every scenario is ONE persistent launch: CTAs of 64 threads pull work items
 // -- (pass, scenario, 2-D tile of the single-grid shapes) -- from a device
 // queue, in pass order.  An item waits only for the rows of its own scenario
@@ -204,12 +204,19 @@ int lsh_batch_create(const lsh_params* params, int n, int device, lsh_batch** ou
             edge_bytes += lsh::edge_layout(eb, nullptr, params[s].nx, params[s].ny);
             fits = fits && lsh::flux_fits(params[s]);
         }
-        if (fits && cudaMalloc(&b->edge_mem, edge_bytes) == cudaSuccess) {
-            cudaError_t e = cudaMemset(b->edge_mem, 0, edge_bytes);
-            if (e != cudaSuccess) return bail(bfail(e, "edge arrays"));
-        } else {
+        if (fits && cudaMalloc(&b->edge_mem, edge_bytes) != cudaSuccess) {
             b->edge_mem = nullptr;
             (void)cudaGetLastError();
+        }
+        // 256 MB stay free for the caller and for the plan
+        size_t room = 0, total = 0;
+        if (b->edge_mem && cudaMemGetInfo(&room, &total) == cudaSuccess && room < (size_t(256) << 20)) {
+            cudaFree(b->edge_mem);
+            b->edge_mem = nullptr;
+        }
+        if (b->edge_mem) {
+            cudaError_t e = cudaMemset(b->edge_mem, 0, edge_bytes);
+            if (e != cudaSuccess) return bail(bfail(e, "edge arrays"));
         }
     }
     { cudaError_t e = cudaMalloc(&b->d_tm, sizeof(lsh::TimeRec) * n); if (e != cudaSuccess) return bail(bfail(e, "cudaMalloc")); }

@@ -377,10 +377,16 @@ int lsh_create(const lsh_params* p, int device, lsh_ctx** out) {
     };
     // The flux pass and cell update where the parameters allow it and its edge
     // buffers fit the device beside the rest; the colour passes, which need 0.6
-    // of the memory, where they do not.
+    // of the memory, where they do not (256 MB stay free for the caller and for
+    // what the context allocates later).
     if (lsh::flux_fits(*p)) {
         cudaError_t e = cudaMalloc(&ctx->edge_mem, FluxMem{}.layout(nullptr, p->nx, p->ny));
         if (e == cudaSuccess) e = cudaMalloc(&ctx->slab, slab_bytes(true));
+        size_t room = 0, total = 0;
+        if (e == cudaSuccess && cudaMemGetInfo(&room, &total) == cudaSuccess && room < (size_t(256) << 20)) {
+            cudaFree(ctx->slab);
+            e = cudaErrorMemoryAllocation;
+        }
         if (e != cudaSuccess) {
             if (ctx->edge_mem) cudaFree(ctx->edge_mem);
             ctx->edge_mem = ctx->slab = nullptr;
