@@ -48,7 +48,7 @@ FJORD2048_FLOPS_PER_CELL_STEP = 804.0
 #   ncu --clock-control none --metrics sm__thread_inst_executed_pipe_fp64_pred_on.sum,\
 #       sm__pipe_fp64_cycles_active.sum,sm__cycles_elapsed.sum,\
 #       dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum \
-#       -k regex:"k_edges|k_volume|k_recon" -s 240 -c 12 \
+#       -k regex:"k_flux|k_update|k_slopes" -s 240 -c 12 \
 #       python bench.py --steps 2 --warmup 20 --no-cpu-baseline --no-e2e
 # They hold only for the kernel sources and the workload generator they were
 # captured on.  Those files are hashed (COUNTER_SOURCES); when the hash is not
@@ -59,18 +59,18 @@ COUNTER_SOURCES = ("landslidehysea_gb300/csrc/lsh_core.cu", "landslidehysea_gb30
                    "landslidehysea_gb300/csrc/lsh_fpmath.h", "landslidehysea_gb300/csrc/lsh_ieee.h",
                    "landslidehysea_gb300/csrc/lsh_setup.h",
                    "landslidehysea_gb300/build.py", "landslidehysea_gb300/scenarios.py")
-COUNTERS_SOURCE_HASH = "032c79f00d393a67"
-# FP64-pipe thread instructions per cell-update of one step (6.060e8 per step
+COUNTERS_SOURCE_HASH = "5f8bceb17935e7e3"
+# FP64-pipe thread instructions per cell-update of one step (2.240e8 per step
 # / 4,194,304 cells).  The FP64 pipe takes one such instruction per lane as
 # the measured peak's DFMA does, so the peak instruction rate is the measured
 # FP64 FLOP/s / 2.
-FJORD2048_FP64_INSTR_PER_CELL_STEP = 144.49
-# DRAM bytes (read + write) per launch of each step kernel; edge_h0 is the
-# first (accumulator-writing) horizontal pass.  A second-order step launches
-# recon and the four edge passes twice, each volume kernel once.
+FJORD2048_FP64_INSTR_PER_CELL_STEP = 53.40
+# DRAM bytes (read + write) per launch of each step kernel: recon is k_slopes,
+# edge_h0 ... edge_v1 the flux pass's four block ranges, volume1 and volume2 the
+# cell updates.  A second-order step launches the first five twice.
 FJORD2048_DRAM_BYTES_PER_LAUNCH = {
-    "recon": 139.65e6, "edge_h0": 356.35e6, "edge_h1": 170.95e6, "edge_v0": 170.5e6, "edge_v1": 167.4e6,
-    "volume1": 651.1e6, "volume2": 699.1e6,
+    "recon": 68.2e6, "edge_h0": 30.6e6, "edge_h1": 32.85e6, "edge_v0": 34.8e6, "edge_v1": 36.7e6,
+    "volume1": 158.7e6, "volume2": 190.0e6,
 }
 # Algorithmic HBM bytes per cell-step (FP64 state with perfect reuse): first
 # order 13 x 8 = 104 B (read 6 state + H, write 6 state); TVD-RK2 104 B for
@@ -500,7 +500,7 @@ def run_ours(args):
                 "algorithmic_bytes": algo, "algorithmic_bytes_per_cell_step": ALGO_BYTES_PER_CELL_STEP[order],
                 "peak_kind": f"{peak_kind} hbm_gbs",
                 "dominant_family": {
-                    "kernels": "k_edges_h / k_edges_v (4 colour passes per stage)",
+                    "kernels": "k_flux (four block ranges per stage)",
                     "launches_per_step": sum(1 for k in names_ms for _ in names_ms[k] if k.startswith("edge")),
                     "share_of_step": round(edge_ms / all_ms, 4), "ms_per_step": round(edge_ms, 4),
                     "dram_bytes_per_step": edge_traffic,
