@@ -868,7 +868,7 @@ LSH_RECURSE bool limit_near(const KArgs& a, int i, int j, int layer, double dt) 
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
         const int ci = i + (k == 1) - (k == 2), cj = j + (k == 3) - (k == 4);
-        if (ci < 0 || ci >= nx || cj < 0 || cj >= ny) continue;
+        if (near || ci < 0 || ci >= nx || cj < 0 || cj >= ny) continue;
         if (mk[(size_t)cj * nx + ci] == now && !holds_all(a, ci, cj, layer, dt)) near = true;
     }
     return near;
