@@ -509,10 +509,11 @@ LSH_HD void edge_raw2(const Face& A, const Face& B, double len, double dt, const
 // 1, h the cells' depths and acc the partial sums before this edge.  A side
 // limits when dt exceeds the time it takes to empty its layer, hp area /
 // (beta out + eps): tested as dt (beta out + eps) > hp area (the denominator
-// is positive), so the divisions run only on limited edges.
-LSH_HD double limiter(double m, double p, bool interior, double h0, double acc0, double area0, double inv_area0,
-                      double h1, double acc1, double area1, double inv_area1, double dt, const Consts& c) {
-    const bool oa = gt0(m), ob = interior && gt0(p);
+// is positive), so the divisions run only on limited edges.  oa, ob: whether
+// cell 0, 1 loses mass and may be emptied.
+LSH_HD double limiter_sides(bool oa, bool ob, double m, double p, double h0, double acc0, double area0,
+                            double inv_area0, double h1, double acc1, double area1, double inv_area1, double dt,
+                            const Consts& c) {
     double ha = 0.0, hb = 0.0, da = 1.0, db = 1.0;
     bool lim = false;
     if (oa) {
@@ -528,6 +529,10 @@ LSH_HD double limiter(double m, double p, bool interior, double h0, double acc0,
     if (!lim) return 1.0;
     const double dta = oa ? div(ha, da) : kBig, dtb = ob ? div(hb, db) : kBig;
     return div(tmin(dta, dtb), dt + kEps);
+}
+LSH_HD double limiter(double m, double p, bool interior, double h0, double acc0, double area0, double inv_area0,
+                      double h1, double acc1, double area1, double inv_area1, double dt, const Consts& c) {
+    return limiter_sides(gt0(m), interior && gt0(p), m, p, h0, acc0, area0, inv_area0, h1, acc1, area1, inv_area1, dt, c);
 }
 
 // Whether a loss `out` (> 0) is far from emptying a layer of depth h: both
