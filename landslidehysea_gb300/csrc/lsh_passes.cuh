@@ -411,8 +411,11 @@ LSH_HD unsigned recon_cell_from(const KArgs& a, int id, int i, int j, const Acc&
     // depth (by the exponents) no face of layer 1 falls below it.
     const double dh1x = sx[0] - sx[3], dh1y = sy[0] - sy[3];
     using lshm::okey;
-    const int64_t quarter = (int64_t)lshm::bits_of(h1) - ((int64_t)2 << 52);
-    const bool deep = quarter > ((int64_t)1 << 52) && (int64_t)lshm::bits_of(lshm::abs_bits(dh1x)) <= quarter &&
+    // (a depth of -0 or below fails the sign test: its pattern less two
+    // exponents would wrap round to a large one)
+    const int64_t quarter = (int64_t)(lshm::bits_of(h1) - ((uint64_t)2 << 52));
+    const bool deep = lsh::gt0(h1) && quarter > ((int64_t)1 << 52) &&
+                      (int64_t)lshm::bits_of(lshm::abs_bits(dh1x)) <= quarter &&
                       (int64_t)lshm::bits_of(lshm::abs_bits(dh1y)) <= quarter;
     if (!warp_all(deep)) {
         lshm::rare();
