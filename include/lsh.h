@@ -200,9 +200,13 @@ int lsh_step_noalloc(const lsh_params* p, double* const dev_state[LSH_NVARS], in
  * duration of the i-th kernel of the step (order 1: 6 kernels -- 4 edge
  * passes, volume, clock; order 2: 13 -- per stage reconstruction, 4 edge
  * passes, volume; then clock).  *n_kernels gets the count (<= cap written).
+ * lsh_probe_tiles: how many tiles of 16 x 4 cells the next step visits
+ * (*listed) of the grid's *total; both 0 where the step runs on the colour
+ * passes, which visit every cell.  Synchronous.
  * lsh_probe_fp64_peak: FP64 FMA throughput of this device, GFLOP/s
  * (2 flops per DFMA), from a dependent-chain microkernel timed with events. */
 int lsh_profile_step(lsh_ctx* ctx, float* ms_out, int cap, int* n_kernels);
+int lsh_probe_tiles(lsh_ctx* ctx, int* listed, int* total);
 int lsh_probe_fp64_peak(int device, double* gflops);
 
 /* Diagnostic: the bounded waits between passes give up instead of hanging.

@@ -1871,7 +1871,7 @@ int lsh_adjoint_create(const lsh_params* params, int device, int n_gauges, const
     // anew) nothing outside a reversed step's adjoint passes: one place for both,
     // so the adjoint needs no more memory.  Only a narrow grid's edges outgrow it.
     const size_t shared = size_t(6 + 21) * A->npad * sizeof(double);
-    const size_t flux_bytes = A->flux_on ? A->flux.layout(nullptr, params->nx, params->ny) : 0;
+    const size_t flux_bytes = A->flux_on ? A->flux.layout(nullptr, params->nx, params->ny, A->order) : 0;
     const size_t extra = (flux_bytes > shared) ? (flux_bytes - shared + 255) & ~size_t(255) : 0;
     const size_t bytes = (size_t(narr) * A->npad + ((geo_n + 31) & ~size_t(31))) * sizeof(double) + extra +
                          2 * A->npad * sizeof(unsigned) + 2 * A->npad + A->n_ctr * sizeof(unsigned);
@@ -1893,7 +1893,7 @@ int lsh_adjoint_create(const lsh_params* params, int device, int n_gauges, const
     for (int q = 0; q < 3; ++q) for (int v = 0; v < 2; ++v) { take(A->snap1[q][v]); take(A->snap2[q][v]); }
     for (int k = 0; k < 6; ++k) take(A->Xb[k]);
     for (int k = 0; k < 6; ++k) take(A->Xbn[k]);
-    if (A->flux_on) A->flux.layout(reinterpret_cast<unsigned char*>(cur), params->nx, params->ny);
+    if (A->flux_on) A->flux.layout(reinterpret_cast<unsigned char*>(cur), params->nx, params->ny, A->order);
     for (int k = 0; k < 6; ++k) take(A->Yb[k]);
     for (int k = 0; k < 7; ++k) { take(A->sxb[k]); take(A->syb[k]); take(A->accb[k]); }
     cur += extra / sizeof(double);

@@ -380,7 +380,7 @@ int lsh_create(const lsh_params* p, int device, lsh_ctx** out) {
     // of the memory, where they do not (256 MB stay free for the caller and for
     // what the context allocates later).
     if (lsh::flux_fits(*p)) {
-        cudaError_t e = cudaMalloc(&ctx->edge_mem, FluxMem{}.layout(nullptr, p->nx, p->ny));
+        cudaError_t e = cudaMalloc(&ctx->edge_mem, FluxMem{}.layout(nullptr, p->nx, p->ny, p->order));
         if (e == cudaSuccess) e = cudaMalloc(&ctx->slab, slab_bytes(true));
         size_t room = 0, total = 0;
         if (e == cudaSuccess && cudaMemGetInfo(&room, &total) == cudaSuccess && room < (size_t(256) << 20)) {
@@ -401,7 +401,7 @@ int lsh_create(const lsh_params* p, int device, lsh_ctx** out) {
         if (e != cudaSuccess) return bail(fail_cuda(e, "cudaMallocHost"));
     }
     if (ctx->edge_mem) {
-        ctx->flux.layout(static_cast<unsigned char*>(ctx->edge_mem), p->nx, p->ny);
+        ctx->flux.layout(static_cast<unsigned char*>(ctx->edge_mem), p->nx, p->ny, p->order);
         cudaError_t e = cudaMemsetAsync(ctx->flux.clear, 0, ctx->flux.clear_bytes, ctx->own);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->own);
         if (e != cudaSuccess) return bail(fail_cuda(e, "cudaMemset cell marks"));
@@ -660,6 +660,19 @@ int lsh_probe_fp64_peak(int device, double* gflops) {
     return LSH_OK;
 }
 
+int lsh_probe_tiles(lsh_ctx* ctx, int* listed, int* total) {
+    if (!ctx || !listed || !total) return LSH_ERR_INVALID;
+    *listed = *total = 0;
+    if (!ctx->edge_mem) return LSH_OK;
+    const TileMap& m = ctx->flux.map;
+    std::vector<int> rows(m.nty);
+    LSH_CUDA(cudaMemcpyAsync(rows.data(), m.count, rows.size() * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    LSH_CUDA(cudaStreamSynchronize(ctx->stream));
+    *total = m.ntx * m.nty;
+    for (int n : rows) *listed += n;
+    return LSH_OK;
+}
+
 int lsh_get_launch_count(lsh_ctx* ctx, long long* launches) {
     if (!ctx || !launches) return LSH_ERR_INVALID;
     *launches = ctx->launches;
@@ -776,11 +789,11 @@ extern "C" int lsh_step_noalloc(const lsh_params* p, double* const dev_state[LSH
         k_noalloc_take_dt<<<1, 1, 0, s>>>(tm, 2.0 * p->cfl);
     }
     FluxMem fm;
-    if (lsh::flux_fits(*p) && fm.layout(nullptr, nx, ny) <= kNaFluxBytes) {
+    if (lsh::flux_fits(*p) && fm.layout(nullptr, nx, ny, 1) <= kNaFluxBytes) {
         // every tile, with the passes overlapped; the counters are zero at load
         // and after each step
         unsigned char* mem = base + kNaHead + kNaAccBytes;
-        fm.layout(mem, nx, ny);
+        fm.layout(mem, nx, ny, 1);
         fm.map.count = nullptr;
         unsigned* ctr = reinterpret_cast<unsigned*>(mem + kNaFluxBytes);
         double* depth = reinterpret_cast<double*>(mem + kNaFluxBytes + ((kNaCtrBytes + 255) & ~size_t(255)));

@@ -380,8 +380,8 @@ __global__ void __launch_bounds__(kCellBlock) k_init_eta(KArgs a) {
 // before and after the step, its edges' kinds are dry, its slopes are zero and
 // flagged so (the reconstruction ran on it, and its neighbours, empty), and its
 // maximum of eta1 has seen the empty state.  On the 2048^2 fjord, 14% wet, the
-// blocks of dry tiles took 490 of the step's 1295 us; after a new state every
-// tile is busy.
+// blocks of dry tiles took 490 of the step's 1295 us (first order: 453 us with
+// every tile, 250 with the lists); after a new state every tile is busy.
 //
 // The flux pass is launched as four consecutive ranges of its blocks, the four
 // edge launches a step has always had (lsh_profile_step,
@@ -419,7 +419,8 @@ struct TileMap {
     int ntx, nty;
     int* list;               // per tile row: the listed tiles' columns, ascending
     int* count;              // per tile row: how many (null: every tile, and no busy flags)
-    // per stage and tile, one byte for each of its warps of the cell passes
+    // per stage (one plane serves for both at order 1) and tile, one byte for
+    // each of its warps of the cell passes
     unsigned short* busy[2];
 };
 
@@ -694,7 +695,7 @@ struct FluxMem {
     TileMap map{};
     unsigned char* clear = nullptr;
     size_t clear_bytes = 0;
-    size_t layout(unsigned char* mem, int nx, int ny) {
+    size_t layout(unsigned char* mem, int nx, int ny, int order) {
         const size_t tiles = size_t(tiles_x(nx)) * tiles_y(ny);
         size_t at = 0;
         auto take = [&](size_t bytes) { unsigned char* q = mem + at; at += (bytes + 255) & ~size_t(255); return q; };
@@ -704,7 +705,8 @@ struct FluxMem {
         map.count = reinterpret_cast<int*>(take(map.nty * sizeof(int)));
         at += lsh::edge_layout(eb, mem + at, nx, ny);
         clear = reinterpret_cast<unsigned char*>(eb.mark[0]);
-        for (int l = 0; l < 2; ++l) map.busy[l] = reinterpret_cast<unsigned short*>(take(tiles * sizeof(unsigned short)));
+        for (int l = 0; l < order; ++l) map.busy[l] = reinterpret_cast<unsigned short*>(take(tiles * sizeof(unsigned short)));
+        if (order == 1) map.busy[1] = map.busy[0];  // k_clock reads both
         clear_bytes = size_t(mem + at - clear);
         return at;
     }

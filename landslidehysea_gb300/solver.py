@@ -51,6 +51,7 @@ SIGNATURES = {
     "lsh_get_gauge_eta": (ctypes.c_int, [P, ctypes.c_int, P, P]),
     "lsh_get_launch_count": (ctypes.c_int, [P, ctypes.POINTER(ctypes.c_longlong)]),
     "lsh_profile_step": (ctypes.c_int, [P, ctypes.POINTER(ctypes.c_float), ctypes.c_int, ctypes.POINTER(ctypes.c_int)]),
+    "lsh_probe_tiles": (ctypes.c_int, [P, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]),
     "lsh_probe_fp64_peak": (ctypes.c_int, [ctypes.c_int, DP]),
     "lsh_probe_wait_bound": (ctypes.c_int, [ctypes.c_int, ctypes.POINTER(ctypes.c_int), DP]),
     "lsh_step_noalloc": (ctypes.c_int, [P, P, ctypes.c_int, DP, DP, P]),
@@ -247,6 +248,12 @@ class Solver:
         n = ctypes.c_longlong()
         _check(self.lib.lsh_get_launch_count(self._ctx, ctypes.byref(n)), "lsh_get_launch_count")
         return n.value
+
+    def listed_tiles(self):
+        """(tiles the next step visits, tiles of the grid); (0, 0) on the colour passes."""
+        n, total = ctypes.c_int(), ctypes.c_int()
+        _check(self.lib.lsh_probe_tiles(self._ctx, ctypes.byref(n), ctypes.byref(total)), "lsh_probe_tiles")
+        return n.value, total.value
 
     def profile_step(self):
         """Run one step with per-kernel CUDA events; returns a list of ms."""
