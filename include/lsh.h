@@ -230,7 +230,9 @@ int lsh_probe_wait_bound(int device, int* status_out, double* ms_out);
  * stays bit-identical to its single-grid run (lsh_create...). */
 typedef struct lsh_batch lsh_batch;
 typedef struct lsh_tune {
-    int32_t ctas_per_sm;        /* persistent CTAs of 64 threads per SM (1-20)  */
+    int32_t ctas_per_sm;        /* persistent CTAs of 64 threads per SM: 1-20;  */
+                                /* with peso = 1 and beta >= 1 at most 12 run,  */
+                                /* and lsh_batch_get_tune says 12 for more      */
     int32_t items_per_fetch;    /* work items a CTA takes from the queue at once */
     double ms_per_step;         /* measured by lsh_batch_autotune               */
 } lsh_tune;

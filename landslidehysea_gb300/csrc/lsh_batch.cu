@@ -277,7 +277,7 @@ int lsh_batch_create(const lsh_params* params, int n, int device, lsh_batch** ou
     std::vector<lsh::TimeRec> tms(n);
     for (int s = 0; s < n; ++s) { tms[s] = lsh::TimeRec{}; tms[s].t_end = INFINITY; tms[s].dt_min = params[s].dt_min; tms[s].done = 1; }
     { cudaError_t e = cudaMemcpy(b->d_tm, tms.data(), sizeof(lsh::TimeRec) * n, cudaMemcpyHostToDevice); if (e != cudaSuccess) return bail(bfail(e, "time")); }
-    b->tune = lsh_tune{16, 1, 0.0};
+    b->tune = lsh_tune{std::min(16, queue_max_ctas(b->edge_mem != nullptr)), 1, 0.0};
     if (int st = build_plan(b)) return bail(st);
     *out = b;
     return LSH_OK;
@@ -378,6 +378,7 @@ int lsh_batch_set_tune(lsh_batch* b, const lsh_tune* tune) {
         return LSH_ERR_INVALID;
     B_CUDA(cudaStreamSynchronize(b->stream));
     b->tune = *tune;
+    b->tune.ctas_per_sm = std::min(b->tune.ctas_per_sm, queue_max_ctas(b->edge_mem != nullptr));  // what runs
     if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
     return LSH_OK;
 }
@@ -401,7 +402,7 @@ int lsh_batch_autotune(lsh_batch* b, int trial_steps, lsh_tune* best_out) {
     lsh_tune best = b->tune;
     best.ms_per_step = INFINITY;
     for (int c : ctas) {
-        if (c > kBMaxCtas) continue;
+        if (c > queue_max_ctas(b->edge_mem != nullptr)) continue;
         for (int f : fetches) {
             lsh_tune t{c, f, 0.0};
             if (int s = lsh_batch_set_tune(b, &t)) { cudaEventDestroy(e0); cudaEventDestroy(e1); return s; }

@@ -48,6 +48,8 @@ enum QueueKind : int { kQColour = 0, kQFlux = 1, kQFluxKeep = 2 };
 #define LSH_BATCH_FLUX_CTAS 12
 #endif
 constexpr int kBMaxCtas = LSH_BATCH_MAXCTAS, kBFluxCtas = LSH_BATCH_FLUX_CTAS;
+// The most CTAs per SM that a queue runs; more would only wait.
+inline int queue_max_ctas(bool flux) { return flux ? kBFluxCtas : kBMaxCtas; }
 constexpr int kMaxPasses = 12;
 
 // Tilings of a scenario's passes, 64-thread tiles of the single-grid shapes:
@@ -436,10 +438,10 @@ inline std::vector<QPassSpec> colour_queue_passes(int order) {
     return v;
 }
 
-// The step's launch: CTAs beyond those the kernel is compiled for would only wait.
+// The step's launch.
 template <int KIND>
 inline void launch_queue(const BPlan& p, int order, int sms, int ctas, int fetch, cudaStream_t s) {
-    const int grid = std::max(1, sms * std::min(std::max(ctas, 1), KIND == kQColour ? kBMaxCtas : kBFluxCtas));
+    const int grid = std::max(1, sms * std::min(std::max(ctas, 1), queue_max_ctas(KIND != kQColour)));
     if (order == 1) k_batch_step<1, KIND><<<grid, kBThreads, 0, s>>>(p, fetch);
     else k_batch_step<2, KIND><<<grid, kBThreads, 0, s>>>(p, fetch);
 }
