@@ -36,6 +36,7 @@
 #include "../../include/lsh.h"
 #include "lsh_passes.cuh"
 #include "lsh_scheme.cuh"
+#include "lsh_run_until.h"
 #include "lsh_setup.h"
 #include "lsh_kernels.cuh"
 
@@ -282,6 +283,16 @@ int put_t_end(lsh_ctx* ctx, double t_end) {
     return LSH_OK;
 }
 
+// lsh_run_until's view of a context (lsh_run_until.h)
+struct CtxClock {
+    lsh_ctx* ctx;
+    TimeRec& rec() { return *ctx->tm_host; }
+    int read() { return read_time(ctx); }
+    int put(double t_end) { return put_t_end(ctx, t_end); }
+    int step(int n) { return lsh_step(ctx, n); }
+    int failed() { return err_bits_to_status(ctx->tm_host->err); }
+};
+
 }  // namespace
 
 extern "C" {
@@ -506,28 +517,8 @@ int lsh_synchronize(lsh_ctx* ctx) {
 int lsh_run_until(lsh_ctx* ctx, double t_end, long long max_steps, long long* steps_done) {
     if (!ctx) return LSH_ERR_INVALID;
     if (!ctx->has_state) { g_last_error = "lsh_set_state has not been called"; return LSH_ERR_INVALID; }
-    if (int s = read_time(ctx)) return s;
-    if (int s = put_t_end(ctx, t_end)) return s;
-    const long long start = ctx->tm_host->steps;
-    int status = LSH_OK;
-    while (!ctx->tm_host->done) {
-        long long left = (max_steps > 0) ? max_steps - (ctx->tm_host->steps - start) : (1LL << 40);
-        if (left <= 0) break;
-        // Steps past t_end find the record done and do nothing, but are launched
-        // all the same: as many as the next step's dt needs to get there (6
-        // readings 8 steps apart on a 512^2 fjord: 47 ms with batches of 128).
-        const double need = std::ceil((t_end - ctx->tm_host->t) / ctx->tm_host->dt);
-        int batch = (int)std::min<long long>(left, 8 * kGraphChunk);
-        if (need < batch) batch = std::max(1, (int)need);
-        if ((status = lsh_step(ctx, batch))) break;
-        if ((status = read_time(ctx))) break;
-    }
-    if (steps_done) *steps_done = ctx->tm_host->steps - start;
-    if (status == LSH_OK) status = err_bits_to_status(ctx->tm_host->err);
-    // step-count mode again for later lsh_step calls
-    int s2 = put_t_end(ctx, INFINITY);
-    if (status == LSH_OK) status = s2;
-    return status;
+    CtxClock c{ctx};
+    return lsh::run_until(c, t_end, max_steps, 8 * kGraphChunk, steps_done);
 }
 
 int lsh_get_state(lsh_ctx* ctx, double* const host_state[LSH_NVARS]) {
