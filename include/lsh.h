@@ -210,13 +210,13 @@ int lsh_probe_tiles(lsh_ctx* ctx, int* listed, int* total);
 int lsh_probe_fp64_peak(int device, double* gflops);
 
 /* Diagnostic: the bounded waits between passes give up instead of hanging.
- * One block runs the overlapped step's wait and the work queue's wait on
- * completion counters that nothing increments; each gives up after its bound
- * (about 2 s of device time) and records it.  *status_out = LSH_ERR_TIMEOUT
- * when both waits gave up and reported (the expected outcome), LSH_OK when
- * either did not; *ms_out (may be null) gets the kernel's duration.  The
- * device is used again afterwards, and the call returns LSH_OK if it
- * answers.  Takes about 4 s.  No reference counterpart. */
+ * A block each runs the waits of the overlapped steps and of the work queues
+ * on completion counters that nothing increments; each gives up after its
+ * bound (about 2 s of device time) and records it.  *status_out =
+ * LSH_ERR_TIMEOUT when all of them gave up and reported (the expected
+ * outcome), LSH_OK when one did not; *ms_out (may be null) gets the kernel's
+ * duration.  The device is used again afterwards, and the call returns LSH_OK
+ * if it answers.  Takes about 4 s.  No reference counterpart. */
 int lsh_probe_wait_bound(int device, int* status_out, double* ms_out);
 
 /* ---------------------------------------------------------------------------

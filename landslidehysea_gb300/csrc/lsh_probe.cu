@@ -1,12 +1,15 @@
 // lsh_probe.cu -- lsh_probe_wait_bound (include/lsh.h): shows on the device
 // that the passes' bounded waits give up and report instead of hanging.
 //
-// One block runs both waits the library uses between passes -- the
-// overlapped step's dep_begin (lsh_kernels.cuh) and the work queue's
-// queue_wait (lsh_queue.cuh) -- on completion counters that nothing
-// increments.  Each gives up after its bound (about 2 s of %globaltimer) and
-// records it: dep_begin in the time record's error word, queue_wait in its
-// abort flag.  The kernel then returns, and the context stays usable.
+// Blocks run the waits the library uses between passes on completion counters
+// that nothing increments: the first dep_begin (lsh_kernels.cuh: the colour
+// passes and the adjoint's) and then queue_wait by one thread (lsh_queue.cuh);
+// the others tile_begin (the flux pass's steps), over every tile of a row and
+// over the listed ones, and queue_wait by a block's threads, a row each (the
+// queues).  Each gives up after its bound (about 2 s of %globaltimer) and
+// records it: dep_begin and tile_begin in the time record's error word,
+// queue_wait in its abort flag.  The kernel then returns, and the context
+// stays usable.
 
 #include <cuda_runtime.h>
 
@@ -19,16 +22,47 @@
 
 namespace {
 
-// out[0]: the time record's timeout bit after dep_begin; out[1]: queue_wait
-// gave up; out[2]: the abort flag it left.
-__global__ void k_wait_probe(Dep d, TimeRec* tm, const unsigned* qctr, int* qabort, int* out) {
-    dep_begin(d, tm, 0, 0);
-    if (threadIdx.x == 0) {
+constexpr int kRows = 64;  // counters, all zero
+constexpr int kWaits = 5;
+
+struct WaitProbe {
+    TimeRec tm[3];
+    unsigned ctr[kRows];
+    int abort_flag[2];
+    int listed[3];  // tiles of the rows that block 2 waits for
+    int out[kWaits];  // 1 where a wait gave up and left its mark
+};
+
+__global__ void k_wait_probe(WaitProbe* w) {
+    if (blockIdx.x == 0) {
+        Dep d;
+        d.wait = w->ctr;  // the wait for 1 never ends by itself
+        d.target = 1;
+        d.kind = kDepCell;
+        d.ntiles = 1;
+        dep_begin(d, &w->tm[0], 0, 0);
+        if (threadIdx.x == 0) {
+            unsigned long long start = 0;
+            w->out[1] = queue_wait(w->ctr, 0, 0, 1u, &w->abort_flag[0], start) && w->abort_flag[0];
+            w->out[0] = (w->tm[0].err >> LSH_ERR_TIMEOUT) & 1;
+        }
+    } else if (blockIdx.x < 3) {
+        // tile row 1 of 3: waits for the rows 0 to 2
+        const int b = (int)blockIdx.x;
+        TileMap m{};
+        m.ntx = 1;
+        m.nty = 3;
+        m.count = (b == 2) ? w->listed : nullptr;
+        TileDep d;
+        d.wait = w->ctr;
+        d.per = 2;
+        tile_begin(d, m, &w->tm[b], 1, 1);
+        if (threadIdx.x == 0) w->out[1 + b] = (w->tm[b].err >> LSH_ERR_TIMEOUT) & 1;
+    } else {
         unsigned long long start = 0;
-        const bool gave_up = queue_wait(qctr, 0, 0, 1u, qabort, start);
-        out[0] = (tm->err >> LSH_ERR_TIMEOUT) & 1;
-        out[1] = gave_up ? 1 : 0;
-        out[2] = *qabort;
+        const bool gave_up = queue_wait(w->ctr, (int)threadIdx.x, kRows - 1, 1u, &w->abort_flag[1], start, (int)blockDim.x);
+        const int all = __syncthreads_and(gave_up);
+        if (threadIdx.x == 0) w->out[4] = all && w->abort_flag[1];
     }
 }
 
@@ -47,42 +81,36 @@ extern "C" int lsh_probe_wait_bound(int device, int* status_out, double* ms_out)
         cudaError_t e = cudaSetDevice(device);
         if (e != cudaSuccess) return probe_fail(e, "cudaSetDevice");
     }
-    // scratch: the time record, two counters, the abort flag, three results
-    void* mem = nullptr;
-    cudaError_t e = cudaMalloc(&mem, 256);
+    WaitProbe* w = nullptr;
+    cudaError_t e = cudaMalloc(&w, sizeof(WaitProbe));
     if (e != cudaSuccess) return probe_fail(e, "cudaMalloc");
-    e = cudaMemset(mem, 0, 256);
-    auto* tm = static_cast<TimeRec*>(mem);
-    unsigned* ctr = reinterpret_cast<unsigned*>(static_cast<char*>(mem) + 128);
-    int* qabort = reinterpret_cast<int*>(ctr + 2);
-    int* out = qabort + 1;
-    Dep d;
-    d.wait = ctr;  // ctr[0] stays 0: the wait for 1 never ends by itself
-    d.target = 1;
-    d.kind = kDepCell;
-    d.ntiles = 1;
+    WaitProbe init{};
+    for (int& n : init.listed) n = 1;
+    e = cudaMemcpy(w, &init, sizeof(init), cudaMemcpyHostToDevice);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (e == cudaSuccess) e = cudaEventCreate(&e0);
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     if (e == cudaSuccess) e = cudaEventRecord(e0);
     if (e == cudaSuccess) {
-        k_wait_probe<<<1, 32>>>(d, tm, ctr + 1, qabort, out);
+        k_wait_probe<<<4, 32>>>(w);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaEventRecord(e1);
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
     float ms = 0.f;
     if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-    int res[3] = {0, 0, 0};
-    if (e == cudaSuccess) e = cudaMemcpy(res, out, sizeof(res), cudaMemcpyDeviceToHost);
+    WaitProbe res{};
+    if (e == cudaSuccess) e = cudaMemcpy(&res, w, sizeof(res), cudaMemcpyDeviceToHost);
     // the device still answers after the waits gave up
-    if (e == cudaSuccess) e = cudaMemset(mem, 0, 256);
+    if (e == cudaSuccess) e = cudaMemset(w, 0, sizeof(WaitProbe));
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    cudaFree(mem);
+    cudaFree(w);
     if (e != cudaSuccess) return probe_fail(e, "lsh_probe_wait_bound");
     if (ms_out) *ms_out = ms;
-    *status_out = (res[0] && res[1] && res[2]) ? LSH_ERR_TIMEOUT : LSH_OK;
+    *status_out = LSH_ERR_TIMEOUT;
+    for (int k = 0; k < kWaits; ++k)
+        if (!res.out[k]) *status_out = LSH_OK;
     return LSH_OK;
 }
