@@ -46,6 +46,22 @@ struct EdgeBuf {
     double* depth_out[2];     // where the flux pass leaves them (null: they stay in W)
 };
 
+// An EdgeBuf's arrays placed in `mem` (256-byte aligned; null: the size alone),
+// the marks last; the bytes they take.
+inline size_t edge_layout(EdgeBuf& eb, unsigned char* mem, int nx, int ny) {
+    const size_t N = size_t(nx) * ny;
+    size_t at = 0;
+    auto take = [&](size_t bytes) { unsigned char* q = mem + at; at += (bytes + 255) & ~size_t(255); return q; };
+    const size_t n[2] = {(N + nx + 31) & ~size_t(31), (N + ny + 31) & ~size_t(31)};
+    for (int d = 0; d < 2; ++d) {
+        eb.plane[d] = n[d];
+        eb.q[d] = reinterpret_cast<double*>(take(kEdgePlanes * n[d] * sizeof(double)));
+        eb.kind[d] = take(n[d]);
+    }
+    for (int l = 0; l < 2; ++l) eb.mark[l] = reinterpret_cast<unsigned*>(take(N * sizeof(unsigned)));
+    return at;
+}
+
 struct KArgs {
     Consts c;
     Geo geo;
@@ -634,25 +650,8 @@ LSH_HD unsigned long long volume_cell(const KArgs& a, int id, double dt) {
 // That an unmarked cell is never limited needs its partial sums not to fall
 // below what its own edges take, so the limiter's factors must not be
 // negative: a limited edge takes at most peso / beta of a cell's content, and
-// Its arrays placed in `mem` (256-byte aligned; null: the size alone), the marks
-// last; the bytes they take.
-inline size_t edge_layout(EdgeBuf& eb, unsigned char* mem, int nx, int ny) {
-    const size_t N = size_t(nx) * ny;
-    size_t at = 0;
-    auto take = [&](size_t bytes) { unsigned char* q = mem + at; at += (bytes + 255) & ~size_t(255); return q; };
-    const size_t n[2] = {(N + nx + 31) & ~size_t(31), (N + ny + 31) & ~size_t(31)};
-    for (int d = 0; d < 2; ++d) {
-        eb.plane[d] = n[d];
-        eb.q[d] = reinterpret_cast<double*>(take(kEdgePlanes * n[d] * sizeof(double)));
-        eb.kind[d] = take(n[d]);
-    }
-    for (int l = 0; l < 2; ++l) eb.mark[l] = reinterpret_cast<unsigned*>(take(N * sizeof(unsigned)));
-    return at;
-}
-
 // flux_fits asks for peso = 1 and beta >= 1 (the reference's values, both 1).
 // The colour passes take the other parameters.
-
 inline bool flux_fits(const lsh_params& p) { return p.peso == 1.0 && p.beta >= 1.0; }
 
 LSH_HD unsigned stage_mark(const KArgs& a) { return 2u * (unsigned)a.tm->steps + a.eb.stage + 1u; }
