@@ -263,8 +263,9 @@ LSH_HD double friction_mu(double h1, double u1, double h2, double u2, const Cons
 }
 
 LSH_HD double fsc_of(double h1, const Consts& c) {
-    // above 4 eps_h the exponent's argument is beyond 746 (40^2) and
-    // exp_neg gives 0, so this is 1 - r (1 - 0) = 1 - r
+    // logarithms 3 apart (each low by at most 0.0861) put h1 above 7.5 eps_h: the
+    // exponent is beyond 75^2, exp_neg gives 0 from 746 on, so this is
+    // 1 - r (1 - 0) = 1 - r
     if (log2_low(h1) - log2_low(c.eps_h) > 3 * kLog2One && gt0(h1)) return 1.0 - c.r;
     const double a = (10.0 * h1) * c.inv_eps;
     return 1.0 - c.r * (1.0 - exp_neg(a * a));
