@@ -15,7 +15,7 @@ namespace lsh {
 constexpr unsigned long long kRateInitBits = 0ULL;  // +0.0
 constexpr int kEdgeBlock = 128;
 constexpr int kCellBlock = 256;
-constexpr double kReconThin = 0.5;  // second order: least face depth / cell depth (half() of the depth)
+constexpr double kReconThin = 0.5;  // second order: least face depth / cell depth
 
 // Sticky error bit: an atomic OR on the device, a plain OR in host code.
 LSH_HD void err_or(int* word, int bit) {
@@ -435,7 +435,8 @@ LSH_HD unsigned recon_cell_from(const KArgs& a, int id, int i, int j, const Acc&
                       (int64_t)lshm::bits_of(lshm::abs_bits(dh1y)) <= quarter;
     if (!warp_all(deep)) {
         lshm::rare();
-        const int64_t k1 = okey(lsh::half(h1));  // kReconThin h1
+        static_assert(kReconThin == 0.5, "half() below gives kReconThin h");
+        const int64_t k1 = okey(lsh::half(h1));
         bad = okey(h1 + dh1x) < k1 || okey(h1 - dh1x) < k1 || okey(h1 + dh1y) < k1 || okey(h1 - dh1y) < k1;
     }
     if (!fast) {
