@@ -679,7 +679,7 @@ LSH_HD void load_side(const KArgs& a, int id, CellSide<ORDER>& c) {
 
 // The face of a cell toward its +slope side (`neg`: the other one) in the edge
 // frame (face_depths, face_rest).  BARE: layer 1 alone, zeros for layer 2.
-template <int DIR, int ORDER, bool BARE>
+template <int ORDER>
 LSH_HD double side_depth(const CellSide<ORDER>& c, bool neg, int layer) {
     double h = c.w[3 * layer];
     if constexpr (ORDER == 2) h = h + lshm::neg_if(layer ? c.s[3] + c.s[6] : c.s[0] - c.s[3], neg);
@@ -735,9 +735,9 @@ LSH_HD EdgeKind flux_faces(const KArgs& a, const EdgeSides& s, Face& A, Face& B)
     const bool na = !(s.side0 & 1);
     const bool bare = bare_side<ORDER>(ca) & bare_side<ORDER>(cb);
     if (warp_all(bare)) {
-        A.h1 = side_depth<DIR, ORDER, true>(ca, na, 0);
+        A.h1 = side_depth<ORDER>(ca, na, 0);
         B.h1 = A.h1;
-        if (s.interior) { lshm::rare(); B.h1 = side_depth<DIR, ORDER, true>(cb, true, 0); }
+        if (s.interior) { lshm::rare(); B.h1 = side_depth<ORDER>(cb, true, 0); }
         if (lshm::lt_pos(half(A.h1 + B.h1), kEps)) return kEdgeDry;
         side_rest<DIR, ORDER, true>(ca, na, s.pos_normal, A);
         if (s.interior) {
@@ -750,10 +750,10 @@ LSH_HD EdgeKind flux_faces(const KArgs& a, const EdgeSides& s, Face& A, Face& B)
         }
         return kEdgeSingle;
     }
-    A.h1 = side_depth<DIR, ORDER, false>(ca, na, 0);
-    A.h2 = side_depth<DIR, ORDER, false>(ca, na, 1);
-    B.h1 = s.interior ? side_depth<DIR, ORDER, false>(cb, true, 0) : A.h1;
-    B.h2 = s.interior ? side_depth<DIR, ORDER, false>(cb, true, 1) : A.h2;
+    A.h1 = side_depth<ORDER>(ca, na, 0);
+    A.h2 = side_depth<ORDER>(ca, na, 1);
+    B.h1 = s.interior ? side_depth<ORDER>(cb, true, 0) : A.h1;
+    B.h2 = s.interior ? side_depth<ORDER>(cb, true, 1) : A.h2;
     // dry edge (Arista_kernel.cu:397)
     if (lshm::lt_pos(half(A.h1 + B.h1), kEps) && lshm::lt_pos(half(A.h2 + B.h2), kEps)) return kEdgeDry;
     side_rest<DIR, ORDER, false>(ca, na, s.pos_normal, A);
