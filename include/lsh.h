@@ -104,7 +104,13 @@ int lsh_params_default(lsh_params* p);
 int lsh_check_device(void);
 
 /* Create a context on `device` (-1: current device).  Allocates the FP64 SoA
- * state (ping-pong), accumulators and the device-resident time/dt record.
+ * state (ping-pong), edge fluxes or accumulators and the device-resident
+ * time/dt record.  Where peso = 1 and beta >= 1 (the flux pass) that is about
+ * 310 bytes a cell at order 1 and 430 at order 2, if the device has them with
+ * 256 MB to spare; otherwise the context takes the colour passes, with the
+ * same results at about 180 and 290 bytes and a lower speed (lsh_probe_tiles
+ * tells which).  Of several contexts that share a device the first ones take
+ * the larger share.
  * Replaces inicializarDatosCuda (ShallowWater.cu:14-110). */
 int lsh_create(const lsh_params* p, int device, lsh_ctx** out);
 int lsh_destroy(lsh_ctx* ctx);
