@@ -386,7 +386,10 @@ __global__ void __launch_bounds__(kCellBlock) k_init_eta(KArgs a) {
 // The flux pass is launched as four consecutive ranges of its blocks, the four
 // edge launches a step has always had (lsh_profile_step,
 // lsh_get_launch_count); nothing orders them, so a small grid's run side by
-// side and a large one's follow each other as one grid's blocks would.
+// side and a large one's follow each other as one grid's blocks would.  One
+// range instead takes a step of 24 x 17 cells from 42.5 to 39.7 us, of a 64^2
+// fjord at first order from 19.9 to 16.4, at second from 131.5 to 128.9, and
+// makes no difference from 200^2 up.
 // Overlap as above (programmatic dependent launches), by tile rows: a block
 // adds 1 to its tile row's counter, and waits for its producer's listed tiles
 // in the rows around its own: the flux pass for the row itself and the one
