@@ -59,7 +59,7 @@ COUNTER_SOURCES = ("landslidehysea_gb300/csrc/lsh_core.cu", "landslidehysea_gb30
                    "landslidehysea_gb300/csrc/lsh_fpmath.h", "landslidehysea_gb300/csrc/lsh_ieee.h",
                    "landslidehysea_gb300/csrc/lsh_setup.h",
                    "landslidehysea_gb300/build.py", "landslidehysea_gb300/scenarios.py")
-COUNTERS_SOURCE_HASH = "e472b3a9f1ed5e14"
+COUNTERS_SOURCE_HASH = "4c3eedfbad4c8c04"
 # FP64-pipe thread instructions per cell-update of one step (2.239e8 per step
 # / 4,194,304 cells).  The FP64 pipe takes one such instruction per lane as
 # the measured peak's DFMA does, so the peak instruction rate is the measured
@@ -69,8 +69,8 @@ FJORD2048_FP64_INSTR_PER_CELL_STEP = 53.39
 # edge_h0 ... edge_v1 the flux pass's four block ranges, volume1 and volume2 the
 # cell updates.  A second-order step launches the first five twice.
 FJORD2048_DRAM_BYTES_PER_LAUNCH = {
-    "recon": 67.6e6, "edge_h0": 30.6e6, "edge_h1": 32.85e6, "edge_v0": 34.8e6, "edge_v1": 36.7e6,
-    "volume1": 157.7e6, "volume2": 189.5e6,
+    "recon": 67.9e6, "edge_h0": 30.6e6, "edge_h1": 32.85e6, "edge_v0": 34.8e6, "edge_v1": 36.7e6,
+    "volume1": 157.6e6, "volume2": 189.5e6,
 }
 # Algorithmic HBM bytes per cell-step (FP64 state with perfect reuse): first
 # order 13 x 8 = 104 B (read 6 state + H, write 6 state); TVD-RK2 104 B for
